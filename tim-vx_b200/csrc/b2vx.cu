@@ -481,21 +481,89 @@ struct PackedContraction {
   std::vector<int32_t> tapc;       // [taps][Ocp]
   bool need_s = false;
   int rows = 0, Kp = 0;
-  // largest |accumulator * acc_scale| any output channel can reach, the accumulator being the true
-  // sum((x - zx)*(w - zw)) + bias with every product at the end of the input type's range that makes it largest
-  double real_max = 0.0;
 };
+
+// Whether every weight minus its zero point fits an int8: such a kernel is packed with the zero point subtracted, and
+// the contraction needs no sum of the inputs (S) beside the products.  True for any int8 kernel with zero point 0, for
+// uint8 with zero point 128, and for most trained uint8 kernels, whose values spread about their zero point.
+bool weights_fit_s8(const TensorRec& w, int Oc) {
+  const size_t per_oc = w.elems() / Oc;
+  const bool u8 = w.d.dtype == B2VX_DT_UINT8, per_ch = w.d.quant_type == B2VX_QUANT_SYMMETRIC_PER_CHANNEL;
+  for (int oc = 0; oc < Oc; ++oc) {
+    const int zw = per_ch ? (w.zps.empty() ? 0 : w.zps[oc]) : w.zp();
+    if (zw == (u8 ? 128 : 0)) continue;
+    const uint8_t* row = w.host.data() + static_cast<size_t>(oc) * per_oc;
+    int lo = 255, hi = -128;
+    if (u8) for (size_t i = 0; i < per_oc; ++i) { lo = std::min<int>(lo, row[i]); hi = std::max<int>(hi, row[i]); }
+    else for (size_t i = 0; i < per_oc; ++i) { const int v = static_cast<int8_t>(row[i]); lo = std::min(lo, v); hi = std::max(hi, v); }
+    if (lo - zw < -128 || hi - zw > 127) return false;
+  }
+  return true;
+}
+
+// Per-channel constants of the tensor-core epilogue's fixed-point requantization (requant_fixed4).  acc_max bounds the
+// accumulators; blocks of blk_w channels, counted from the start of each tile of tile_data, share a window.  Returns false
+// when a channel does not allow it (every element then takes the exact sequence).
+bool fixed_point_columns(const PackedContraction& pk, const OutQuant& out, double acc_max, int tile_data, int blk_w, std::vector<FixedColumn>* cols,
+                         int* shl) {
+  const size_t n = pk.acc_scale.size();
+  const double two32 = 4294967296.0;
+  std::vector<double> r(n);   // acc_scale / out scale in units of 2^-32
+  double r_max = 0.0;
+  for (size_t c = 0; c < n; ++c) {
+    r[c] = static_cast<double>(pk.acc_scale[c]) / static_cast<double>(out.scale) * two32;
+    if (!(r[c] >= 0.0 && std::fabs(static_cast<double>(pk.bias_full[c])) * r[c] < 1e18)) return false;
+    r_max = std::max(r_max, r[c]);
+  }
+  int k = 0;
+  while (k < 20 && r_max / (1 << k) >= 2147483000.0) ++k;
+  if (!(r_max / (1 << k) < 2147483000.0) || acc_max * (1 << k) >= 2147483647.0) return false;
+  *shl = k;
+  // |real / scale| of an output that does not saturate, and the middle of its range
+  const double top = std::max(out.hi - out.zp, out.zp - out.lo) + 1.0, half = 0.5 * (out.hi - out.lo) + 1.0, mid = 0.5 * (out.hi + out.lo) - out.zp;
+  cols->resize(n);
+  for (size_t tile = 0; tile < n; tile += tile_data) {
+    const size_t tile_end = std::min(n, tile + tile_data);
+    for (size_t c0 = tile; c0 < tile_end; c0 += blk_w) {
+      const size_t c1 = std::min(tile_end, c0 + blk_w);
+      double w = 0.0;
+      for (size_t c = c0; c < c1; ++c) {
+        const double mul = std::nearbyint(r[c] / (1 << k));
+        (*cols)[c].mul = static_cast<int32_t>(mul);
+        if (r[c] == 0.0) continue;
+        // what the rounding of the multiplier costs over the range, once its value at the middle has gone into the addend;
+        // and what the reference rounds: product and quotient (half an ulp each), an accumulator beyond 2^24 when it
+        // becomes a float.  (The addition in its floor(|x| + 0.5f) moves no result across an integer except just below
+        // x = 0.5, by less than 2^-24.)
+        const double err = std::fabs(r[c] - mul * (1 << k)) / r[c] * half;
+        const double ref = top * (top * two32 < r[c] * 16777216.0 ? 2.02 : 3.03) / 16777216.0 + 1.0 / 8388608.0;
+        w = std::max(w, err + ref);
+      }
+      if (!(w < 0.25)) return false;
+      const int64_t half_window = static_cast<int64_t>(w * two32) + 4;
+      for (size_t c = c0; c < c1; ++c) {
+        FixedColumn& f = (*cols)[c];
+        const double centre = r[c] > 0.0 ? (r[c] - static_cast<double>(f.mul) * (1 << k)) / r[c] * mid * two32 : 0.0;
+        f.add = (static_cast<int64_t>(pk.bias_full[c]) << k) * f.mul + (static_cast<int64_t>(out.zp - out.lo) << 32) + (int64_t(1) << 31) +
+                half_window + std::llround(centre);
+        f.window = static_cast<uint32_t>(2 * half_window);
+      }
+    }
+  }
+  return true;
+}
 
 // Weight element (kx,ky,ic,oc) of a WHIcOc kernel as a signed value together
 // with the zero point that still has to be subtracted from it: u8 weights are
 // shifted by 128 into int8 (dz = zw-128), s8 weights are kept (dz = zw).
 // K index by k_order: 0 tap*Cs + ic; 1 ic*taps + tap (the kernel tensor's own order, used with the
-// WHCN im2col); 2 / 3 (ky*C + ic)*8 + kx / (ky*C + ic)*4 + kx (filter rows padded to 8 / 4 taps, used with the row-of-8 / row-of-4 im2col).  Rows come in n_tiles tiles of tile_rows rows: output channel oc is row
-// (oc / tile_data) * tile_rows + oc % tile_data; when some dz != 0 and tile_rows > tile_data, row
+// WHCN im2col); 2 / 3 (ky*C + ic)*8 + kx / (ky*C + ic)*4 + kx (filter rows padded to 8 / 4 taps, used with the row-of-8 / row-of-4 im2col).  Rows come in the tiles of `tiling`, each tile's channels in gemm_tc_row_of_channel's
+// order (blk_w == 0: in plain order); when some dz != 0 and tile_rows > tile_data, row
 // tile_data of every tile is the all-ones row (its dot product with an input row is S).
+// centred: the zero point is subtracted here (weights_fit_s8), dz is 0.
 void pack_contraction(const TensorRec& x, const TensorRec& w, const TensorRec* bias, int kw, int kh, int C, int Cs,
-                      int Kp, int Oc, int Ocp, int n_tiles, int tile_data, int tile_rows, int k_order,
-                      PackedContraction* out) {
+                      int Kp, int Oc, int Ocp, const GemmTcTiling& tiling, int k_order, bool centred, PackedContraction* out) {
+  const int n_tiles = tiling.n_tiles, tile_data = tiling.data, tile_rows = tiling.rows;
   const int rows = n_tiles * tile_rows;
   const int taps = kw * kh;
   const bool w_u8 = w.d.dtype == B2VX_DT_UINT8;
@@ -516,12 +584,10 @@ void pack_contraction(const TensorRec& x, const TensorRec& w, const TensorRec* b
   const float sx = x.scale();
   std::vector<int64_t> tapsum(taps);
   const int32_t* b = bias ? reinterpret_cast<const int32_t*>(bias->host.data()) : nullptr;
-  const int x_lo = (x.d.dtype == B2VX_DT_INT8 ? -128 : 0) - zx, x_hi = (x.d.dtype == B2VX_DT_INT8 ? 127 : 255) - zx;
-  out->real_max = 0.0;
   for (int oc = 0; oc < Oc; ++oc) {
     const int zw = per_ch ? (w.zps.empty() ? 0 : w.zps[oc]) : w.zp();
     const float sw = per_ch ? w.scales[oc] : w.scale();
-    const int dz = w_u8 ? zw - 128 : zw;
+    const int dz = centred ? 0 : (w_u8 ? zw - 128 : zw);
     out->dz[oc] = dz;
     if (dz != 0) out->need_s = true;
     out->acc_scale[oc] = sx * sw;
@@ -529,22 +595,16 @@ void pack_contraction(const TensorRec& x, const TensorRec& w, const TensorRec* b
   out->w8.assign(static_cast<size_t>(rows) * Kp, 0);
   for (int oc = 0; oc < Oc; ++oc) {
     std::fill(tapsum.begin(), tapsum.end(), 0);
-    int64_t pos = 0, neg = 0;
-    int8_t* row = out->w8.data() + (static_cast<size_t>(oc / tile_data) * tile_rows + oc % tile_data) * Kp;
+    const int shift = centred ? (per_ch ? (w.zps.empty() ? 0 : w.zps[oc]) : w.zp()) : (w_u8 ? 128 : 0);
+    int8_t* row = out->w8.data() + (static_cast<size_t>(oc / tile_data) * tile_rows + (tiling.blk_w ? gemm_tc_row_of_channel(tiling, oc % tile_data) : oc % tile_data)) * Kp;
     for (int ic = 0; ic < C; ++ic) {
       for (int t = 0; t < taps; ++t) {
         const size_t src = (static_cast<size_t>(oc) * C + ic) * taps + t;   // WHIcOc, W fastest: tap = ky*kw + kx
-        const int v = w_u8 ? static_cast<int>(w.host[src]) - 128 : static_cast<int>(reinterpret_cast<const int8_t*>(w.host.data())[src]);
+        const int v = (w_u8 ? static_cast<int>(w.host[src]) : static_cast<int>(static_cast<int8_t>(w.host[src]))) - shift;
         row[kidx(t, ic)] = static_cast<int8_t>(v);
         tapsum[t] += v;
-        const int64_t wr = v - out->dz[oc];   // the real weight minus its zero point
-        const int64_t p0 = wr * x_lo, p1 = wr * x_hi;
-        pos += p0 > p1 ? p0 : p1;
-        neg += p0 < p1 ? p0 : p1;
       }
     }
-    const double hi = static_cast<double>(pos + (b ? b[oc] : 0)), lo = static_cast<double>(neg + (b ? b[oc] : 0));
-    out->real_max = std::max(out->real_max, std::max(std::fabs(hi), std::fabs(lo)) * std::fabs(static_cast<double>(out->acc_scale[oc])));
     int64_t all = 0;
     for (int t = 0; t < taps; ++t) {
       // contribution of one fully in-bounds tap beyond the raw products:
@@ -704,6 +764,8 @@ b2vx_status plan_contraction(b2vx_graph* g, uint32_t node_index, const char* lab
   // padding, or when the window covers the whole (unpadded) input.
   const bool identity_1x1 = kw == 1 && kh == 1 && geo.sx == 1 && geo.sy == 1 && !has_pad;
   const bool identity_full = kw == x.W && kh == x.H && !has_pad && y.W == 1 && y.H == 1 && geo.dx == 1 && geo.dy == 1;
+  const bool centred = g->use_tc && any_dz && weights_fit_s8(w, y.C);
+  if (centred) any_dz = false;
   const bool tc_ok = g->use_tc && (!any_dz || dz_is_uniform);   // one leftover weight zero point: the S column handles it
 
   ContractEpilogue ep;
@@ -777,7 +839,7 @@ b2vx_status plan_contraction(b2vx_graph* g, uint32_t node_index, const char* lab
     // Measured at N = K = 4096: faster than the 128-row tile up to 8 rows (1.8x at one row); at 16 rows the
     // dp4a rate bounds it and the tensor-core kernel is level or better.
     if (g->fc_small_m && mode == IDENTITY && M <= 16 && (!any_dz || x.C == x.Cp)) {
-      pack_contraction(x, w, bias, kw, kh, x.C, Cs, Kp, y.C, y.Cp, 1, y.Cp, y.Cp, 0, &pk);
+      pack_contraction(x, w, bias, kw, kh, x.C, Cs, Kp, y.C, y.Cp, GemmTcTiling{1, y.Cp, y.Cp, 0}, 0, centred, &pk);
       int8_t* dw8s = nullptr; int32_t* dbias_s = nullptr; float* dscale_s = nullptr;
       b2vx_status sts = upload(g, pk.w8, &dw8s);
       if (sts == B2VX_OK) sts = upload(g, pk.bias_full, &dbias_s);
@@ -799,7 +861,7 @@ b2vx_status plan_contraction(b2vx_graph* g, uint32_t node_index, const char* lab
     }
     const GemmTcTiling tiling = gemm_tc_choose_tiling(M, y.Cp, Kp, any_dz ? 1 : 0);
     const int Np = tiling.n_tiles * tiling.rows;
-    pack_contraction(x, w, bias, kw, kh, x.C, Cs, Kp, y.C, y.Cp, tiling.n_tiles, tiling.data, tiling.rows, mode == WHCN ? 1 : (mode == WHCN8 ? (padk == 8 ? 2 : 3) : 0), &pk);
+    pack_contraction(x, w, bias, kw, kh, x.C, Cs, Kp, y.C, y.Cp, tiling, mode == WHCN ? 1 : (mode == WHCN8 ? (padk == 8 ? 2 : 3) : 0), centred, &pk);
     ep.dz_uniform = any_dz ? dz_value : 0;
     if (mode == IMPLICIT && need_border) {
       // correction of class (r, c) = minus the folded contribution of every tap that is out of bounds there
@@ -832,12 +894,14 @@ b2vx_status plan_contraction(b2vx_graph* g, uint32_t node_index, const char* lab
     ep.bias_full = dbias;
     ep.acc_scale = dscale;
     {
-      // largest |acc * acc_scale / out scale| any input can produce: decides whether the epilogue may
-      // use its fast rounding (valid below 2^21)
-      // (bounded per output channel from the weights themselves; the integer the epilogue converts is that true
-      // accumulator: the S term of a weight zero point and the border corrections are already in it)
-      const double tmax = pk.real_max / std::fabs(static_cast<double>(ep.out.scale));
-      ep.exact_only = !(tmax < 2097152.0);
+      std::vector<FixedColumn> fix;
+      FixedColumn* dfix = nullptr;
+      // raw accumulators, the S term and the border corrections each stay below taps * channels * 255 * 128 * 2
+      if (fixed_point_columns(pk, ep.out, 4.0 * taps * x.C * 255 * 128, tiling.data, tiling.blk_w, &fix, &ep.fix_shl)) {
+        st = upload(g, fix, &dfix);
+        if (st != B2VX_OK) return st;
+        ep.fix = dfix;
+      }
     }
     void* fused_out = nullptr;
     if (g->fuse_request >= 0) {
@@ -953,7 +1017,7 @@ b2vx_status plan_contraction(b2vx_graph* g, uint32_t node_index, const char* lab
 
   // CUDA-core path: K = tap*Cp + c, out-of-bounds taps are skipped and corrected per tap.
   const int Kp = taps * x.Cp;
-  pack_contraction(x, w, bias, kw, kh, x.C, x.Cp, Kp, y.C, y.Cp, 1, y.Cp, y.Cp + 1, 0, &pk);
+  pack_contraction(x, w, bias, kw, kh, x.C, x.Cp, Kp, y.C, y.Cp, GemmTcTiling{1, y.Cp, y.Cp + 1, 0}, 0, centred, &pk);
   int8_t* dw8 = nullptr; int32_t *dbias = nullptr, *ddz = nullptr, *dtapc = nullptr; float* dscale = nullptr;
   b2vx_status st = upload(g, pk.w8, &dw8);
   if (st == B2VX_OK) st = upload(g, pk.bias_full, &dbias);

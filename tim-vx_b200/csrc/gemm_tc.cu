@@ -26,18 +26,23 @@
 //                            after each stage, accumulator-ready after a tile.
 //   warps 4-19  epilogue     16 warps (four per SM scheduler, to hide latency).
 //                            A warp owns the 32 TMEM lanes (tile rows) its id
-//                            maps to and every fourth 16-column chunk:
-//                            tcgen05.ld (the next chunk's load in flight),
-//                            folded bias, requantize two floats per
-//                            instruction, saturating pack, and a 16-byte store
-//                            per thread straight to the output.  No barrier
-//                            joins the warps, so they drift apart and work on
-//                            neighbouring tiles; two accumulator buffers
-//                            overlap tile i's epilogue with tile i+1's MMAs.
-//                            (B2VX_TC_STORE=tma: write the bytes swizzled into
-//                            a staging tile instead and store it with TMA.)
-//                            Tiles of at most 64 columns: four teams of four
-//                            warps, each team on its own tile with all chunks.
+//                            maps to and one of four runs of column blocks.
+//                            tcgen05.ld in the 16 x 256-bit shape: a thread
+//                            gets four columns of four rows per 16 columns, so
+//                            that the per-column constants it reads from shared
+//                            memory serve four rows (one row per thread made
+//                            that traffic, 12 bytes per output, the bound of
+//                            every short-K layer: 128 bytes per clock).  The
+//                            packed weight rows are permuted so that these
+//                            columns are neighbouring channels: a thread ends
+//                            up with 16 (8, 4) consecutive bytes of four rows
+//                            and four threads store 64 (32, 16) consecutive
+//                            bytes of a row.  Requantization: requant_fixed4.
+//                            No barrier joins the warps, so they drift apart
+//                            and work on neighbouring tiles; two accumulator
+//                            buffers overlap tile i's epilogue with tile i+1's
+//                            MMAs.  Tiles of at most 64 columns: four teams of
+//                            four warps, each team on its own tile.
 //   warp 3      residual producer of a fused Add (template FUSE): the Add's
 //                            64 KB table by four bulk copies first, then the
 //                            Add's other operand, tile by tile, into the
@@ -155,15 +160,13 @@ struct GemmParams {
   // (about 56 bytes per clock) could not feed.  The price: both accumulators are in use, so a pair's epilogue does
   // not overlap the next pair's main loop; chosen only where the main loop is many times longer.
   int pair;
-  // output through shared memory + TMA store: the tile is staged as BN/store_span column blocks of
-  // [128 rows][store_span bytes], 16-byte chunks XOR-swizzled the way the store's tensor map expects.
-  // store_span == 0: BN is not a multiple of 32, threads store their 16-byte pieces directly.
-  int store_span;
-  // FUSE: the residual tile comes into the same staging memory by TMA (tensor map in the output map's
-  // slot, column blocks of res_span bytes); 0: BN is not a multiple of 32, threads load their pieces.
-  int res_span;
+  // Columns are dealt to the epilogue warps in blocks of blk_w (64, 32 or 16), blk_per_group consecutive blocks to a
+  // warp group (all of them in team mode).  plain_order: the weight rows are not permuted (blk_w is 16 then).
+  int blk_w, blk_per_group, plain_order;
+  // FUSE: the residual tile comes by TMA into buffers (two, in team mode four: 1 << res_shift) of
+  // [blocks][128 rows][blk_w] bytes, 16-byte pieces XOR-swizzled; 0: threads load their residual bytes themselves.
+  int res_tma, res_shift;
   int dz;                  // weight zero point left after the shift into int8; != 0: column BNd of the accumulator is S
-  int exact_only;          // requantize with the exact sequence only (the fast form's range check failed)
   long long wait_limit;    // cycles after which a barrier wait gives up (kWaitLimitCycles)
   uint32_t tx_extra;       // test aid: bytes added to what the A producer announces, so that its barrier never completes
 #ifdef B2VX_TC_TRACE
@@ -252,25 +255,6 @@ __device__ __forceinline__ void bulk_load(uint32_t dst, const void* src, uint32_
                ::"r"(dst), "l"(reinterpret_cast<uint64_t>(src)), "r"(bytes), "r"(bar)
                : "memory");
 }
-__device__ __forceinline__ void tma_store_2d(const CUtensorMap* map, uint32_t src, int c0, int c1) {
-  asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%2, %3}], [%1];"
-               ::"l"(reinterpret_cast<uint64_t>(map)), "r"(src), "r"(c0), "r"(c1)
-               : "memory");
-}
-__device__ __forceinline__ void tma_store_4d(const CUtensorMap* map, uint32_t src, int c0, int c1, int c2, int c3) {
-  asm volatile("cp.async.bulk.tensor.4d.global.shared::cta.bulk_group [%0, {%2, %3, %4, %5}], [%1];"
-               ::"l"(reinterpret_cast<uint64_t>(map)), "r"(src), "r"(c0), "r"(c1), "r"(c2), "r"(c3)
-               : "memory");
-}
-__device__ __forceinline__ void tma_store_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
-// Waits until at most N of this thread's store groups still have to read their shared-memory source.
-template <int N>
-__device__ __forceinline__ void tma_store_wait_read() {
-  asm volatile("cp.async.bulk.wait_group.read %0;" ::"n"(N) : "memory");
-}
-__device__ __forceinline__ void tma_store_wait_all() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
-// Makes this thread's shared-memory writes visible to the TMA engine (async proxy).
-__device__ __forceinline__ void fence_smem_to_async() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 // Barrier among the epilogue warps only.
 __device__ __forceinline__ void epilogue_barrier() { asm volatile("bar.sync 1, %0;" ::"n"(kEpilogueThreads) : "memory"); }
 
@@ -316,14 +300,13 @@ __device__ __forceinline__ void tc_mma_i8_halves(uint32_t tmem_d, uint32_t a_lo,
       : "memory");
 }
 
-__device__ __forceinline__ void tc_ld_32x16(uint32_t taddr, int (&r)[16]) {
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
-      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
-      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
-        "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-      : "r"(taddr)
-      : "memory");
+// 16 lanes x 16 columns: thread t gets, of the 8-column halves h = 0, 1, columns 2 * (t % 4) + {0, 1} of row t / 4 in
+// r[4 h], r[4 h + 1] and of row t / 4 + 8 in r[4 h + 2], r[4 h + 3].
+__device__ __forceinline__ void tc_ld_16x16(uint32_t taddr, int* r) {
+  asm volatile("tcgen05.ld.sync.aligned.16x256b.x2.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+               : "r"(taddr)
+               : "memory");
 }
 __device__ __forceinline__ void tc_ld_32x1(uint32_t taddr, int& r) {
   asm volatile("tcgen05.ld.sync.aligned.32x32b.x1.b32 {%0}, [%1];" : "=r"(r) : "r"(taddr) : "memory");
@@ -359,28 +342,30 @@ struct SmemHeader {
   unsigned long long tmem_empty[kMaxAccBuffers];
   unsigned long long b_full;         // resident weights landed
   unsigned long long tab_full;       // FUSE: the Add's table landed
-  unsigned long long res_full[2];    // FUSE: residual tile landed / read by all epilogue warps
-  unsigned long long res_empty[2];
+  unsigned long long res_full[kGroups];    // FUSE: residual tile landed / read by the epilogue warps
+  unsigned long long res_empty[kGroups];
   uint32_t tmem_base;
   int abort_flag;
-  // this CTA's N tile: folded bias and accumulator scale per column; read as 128-bit vectors
-  alignas(16) int bias[256];
-  alignas(16) float scale[256];
+  FixedColumns cols;                 // this CTA's N tile
 };
 
 // EXTRA: rows carry a weight-zero-point term (p.dz, S column) and/or border corrections
-// (p.ep.border_corr); the plain form contains no code for either.
+// (p.ep.border_corr), or the fixed-point multipliers had to be halved (p.ep.fix_shl); the plain form contains no code
+// for any of these.
 // FUSE: a residual Add follows the convolution and is done here: the 64 KB table of that Add sits in
-// shared memory behind the operand ring, the epilogue loads the residual's 16 bytes beside its own
-// and stores the table's answers instead (direct stores only).
-template <bool EXTRA, bool FUSE>
+// shared memory behind the operand ring, the epilogue loads the residual's bytes beside its own
+// and stores the table's answers instead.
+// STEPS: column blocks of 16 * STEPS (1, 2 or 4) columns.  A template parameter because small layers are bound by
+// instruction fetch (a launch executes every line of the kernel about once per warp): code for the other widths in the
+// same kernel costs them.
+template <bool EXTRA, bool FUSE, int STEPS>
 __global__ void __launch_bounds__(kThreadsTc, 1)
 gemm_i8_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
-                  const __grid_constant__ CUtensorMap map_d, const GemmParams p) {
+                  const __grid_constant__ CUtensorMap map_r, const GemmParams p) {
   extern __shared__ uint8_t smem_raw[];
   TC_MARK(0);
   pdl_trigger();   // the next kernel of the stream may begin its own prologue
-  // [ring of stages | two staging tiles | header], the first two 1024-byte aligned (128-byte swizzle)
+  // [ring of stages | resident weights | residual tiles | Add table | header], 1024-byte aligned up to the table
   const uint32_t raw_addr = smem_u32(smem_raw);
   const uint32_t tiles_addr = (raw_addr + 1023u) & ~1023u;
   uint8_t* tiles = smem_raw + (tiles_addr - raw_addr);
@@ -392,9 +377,9 @@ gemm_i8_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
   const uint32_t ring_bytes = (p.stages * stage_bytes + 1023u) & ~1023u;
   const uint32_t bres_bytes = p.b_resident ? ((static_cast<uint32_t>(p.num_kb_b) * b_bytes + 1023u) & ~1023u) : 0u;
   const uint32_t bres_addr = tiles_addr + ring_bytes;                    // resident weights: k-block after k-block
-  const uint32_t staging_bytes = (p.store_span || p.res_span) ? static_cast<uint32_t>(kBlockM) * p.BNd : 0u;   // per buffer, multiple of 4096
-  uint8_t* staging = tiles + ring_bytes + bres_bytes;
-  uint8_t* add_tab = staging + 2 * staging_bytes;                 // 64 KB when FUSE
+  const uint32_t res_bytes = static_cast<uint32_t>(kBlockM) * p.BNd;   // one residual tile
+  uint8_t* res_tiles = tiles + ring_bytes + bres_bytes;
+  uint8_t* add_tab = res_tiles + (p.res_tma ? res_bytes << p.res_shift : 0u);    // 64 KB when FUSE
   SmemHeader* hdr = reinterpret_cast<SmemHeader*>(add_tab + (FUSE ? 65536 : 0));
   volatile int* abort_flag = &hdr->abort_flag;
 
@@ -406,7 +391,7 @@ gemm_i8_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
     // descriptor fetches overlap the rest of the prologue instead of delaying the first loads
     asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&map_a)) : "memory");
     asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&map_b)) : "memory");
-    if (p.store_span || p.res_span) asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&map_d)) : "memory");
+    if (p.res_tma) asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&map_r)) : "memory");
   }
   if (threadIdx.x == 0) {
     for (int s = 0; s < p.stages; ++s) {
@@ -419,9 +404,9 @@ gemm_i8_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
     }
     mbar_init(smem_u32(&hdr->b_full), 1);
     mbar_init(smem_u32(&hdr->tab_full), 1);
-    for (int b = 0; b < 2; ++b) {
+    for (int b = 0; b < kGroups; ++b) {
       mbar_init(smem_u32(&hdr->res_full[b]), 1);
-      mbar_init(smem_u32(&hdr->res_empty[b]), kEpilogueWarps);
+      mbar_init(smem_u32(&hdr->res_empty[b]), p.teams ? 4 : kEpilogueWarps);
     }
     hdr->abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -465,11 +450,11 @@ gemm_i8_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
     // stage's k-blocks.
     const bool is_a = warp == 0;
     uint32_t it = 0, s = 0, ph = 0;   // stage index and ring phase, advanced without divisions
-    // Everything above touched only constants and this CTA's own shared/tensor memory.  The operand
-    // loads are the first access to what earlier kernels of the stream produced (and every later
-    // access of this kernel, the output stores included, depends on them through the barriers).
-    pdl_wait();
-    bool ok = true;
+    // Everything above touched only constants and this CTA's own shared/tensor memory.  The A operand's loads are the
+    // first access to what earlier kernels of the stream produced (and every later access of this kernel, the output
+    // stores included, depends on them through the barriers); weights are constants, their loads run ahead.  The wait
+    // comes after the first slot is armed, so that only the load itself follows it.
+    bool ok = true, waited = !is_a;
     int m_tile = m_tile0;
     const int tstep = p.pair ? 2 : 1;   // pair mode: tiles j and j + 1 of this CTA go through the ring together
     for (int tile = blockIdx.x; ok && tile < num_tiles; tile += tstep * gridDim.x, m_tile += tstep * m_step) {
@@ -493,6 +478,12 @@ gemm_i8_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
         if (is_a) TC_TRACE(0, it, 0);
         if (elect_one()) {
           mbar_arrive_expect_tx(full, static_cast<uint32_t>(cnt) * (is_a ? p.a_tx_bytes * (two ? 2u : 1u) : b_bytes) + (is_a ? p.tx_extra : 0u));
+        }
+        if (!waited) {
+          waited = true;
+          pdl_wait();
+        }
+        if (elect_one()) {
           uint32_t dst = tiles_addr + s * stage_bytes;
           int t_tap = tap, t_cb = cb, t_ky = ky, t_kx = kx;
           for (int gi = 0; gi < cnt; ++gi, dst += sub_bytes) {
@@ -532,6 +523,9 @@ gemm_i8_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
     bool ok = true;
     int j = 0;
     const int ksteps = p.BK >> 5;
+    // Descriptors: the high halves never change (except halo mode's A), the low ones are addresses.
+    const uint64_t desc0 = make_smem_desc(0, p.sbo, p.layout_type);
+    const uint32_t d_hi = static_cast<uint32_t>(desc0 >> 32), d_lo = static_cast<uint32_t>(desc0);
     if (p.b_resident && static_cast<int>(blockIdx.x) < num_tiles) {
       ok = mbar_wait(smem_u32(&hdr->b_full), 0, abort_flag, p.status, 8, p.wait_limit);
       ok = __all_sync(0xffffffffu, ok);
@@ -549,21 +543,21 @@ gemm_i8_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
       const uint32_t tmem_d = tmem_base + a * p.acc_stride;
       uint32_t accumulate = 0;
       for (int kb0 = 0; kb0 < p.num_kb; kb0 += p.group, ++it) {
+        const uint32_t a_lo0 = d_lo + ((tiles_addr + s * stage_bytes) >> 4);
+        const uint32_t b_lo0 = p.b_resident ? d_lo + ((bres_addr + static_cast<uint32_t>(kb0) * b_bytes) >> 4) : a_lo0 + (b_off >> 4);
+        const int cnt = min(p.group, p.num_kb - kb0);
         ok = mbar_wait(smem_u32(&hdr->full[s]), ph, abort_flag, p.status, 3, p.wait_limit);
         ok = __all_sync(0xffffffffu, ok);
         if (!ok) break;
         TC_TRACE(1, it, 0);
         tc_fence_after();
-        const int cnt = min(p.group, p.num_kb - kb0);
         if (p.halo) {
           // one stage = the input patch of channel block kb0: every tap is a shifted view of it.  The issuing thread
           // shares its scheduler with four epilogue warps, so every instruction here costs several cycles: descriptors
           // are built once per stage and advanced by additions to their address field (16-byte units).
           if (elect_one()) {
-            const uint64_t da0 = make_smem_desc(tiles_addr + s * stage_bytes, static_cast<uint32_t>(p.halo_w) * p.BK, p.layout_type);
-            const uint64_t db0 = make_smem_desc(bres_addr + static_cast<uint32_t>(kb0) * b_bytes, p.sbo, p.layout_type);
-            const uint32_t a_hi = static_cast<uint32_t>(da0 >> 32), b_hi = static_cast<uint32_t>(db0 >> 32);
-            uint32_t b_lo = static_cast<uint32_t>(db0);
+            const uint32_t a_hi = static_cast<uint32_t>(make_smem_desc(0, static_cast<uint32_t>(p.halo_w) * p.BK, p.layout_type) >> 32), b_hi = d_hi;
+            uint32_t b_lo = b_lo0;
             const uint32_t db_step = (static_cast<uint32_t>(p.cblocks) * b_bytes) >> 4;
             const uint32_t px16 = static_cast<uint32_t>(p.BK) >> 4;           // one pixel of the patch, in 16-byte units
             const int taps_h = p.halo_kh;
@@ -571,7 +565,7 @@ gemm_i8_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
             if (p.kw == 3 && taps_h == 3) {
               // The 3x3 window written out (halo mode always has 64-byte channel blocks: a pixel is four 16-byte units,
               // two k steps): eighteen instructions whose descriptors differ by constants, no loop control between them.
-              uint32_t a_row = static_cast<uint32_t>(da0);
+              uint32_t a_row = a_lo0;
               const uint32_t row16 = static_cast<uint32_t>(p.halo_w) * 4u;
 #pragma unroll
               for (int ky = 0; ky < 3; ++ky, a_row += row16) {
@@ -585,7 +579,7 @@ gemm_i8_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
               }
             } else {
               for (int ky = 0; ky < taps_h; ++ky) {
-                uint32_t a_lo = static_cast<uint32_t>(da0) + static_cast<uint32_t>(ky * p.halo_w) * px16;
+                uint32_t a_lo = a_lo0 + static_cast<uint32_t>(ky * p.halo_w) * px16;
                 for (int kx = 0; kx < p.kw; ++kx, a_lo += px16, b_lo += db_step) {
                   if (first) {
                     tc_mma_i8_halves<0>(tmem_d, a_lo, a_hi, b_lo, b_hi, p.idesc);
@@ -600,11 +594,8 @@ gemm_i8_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
             tc_commit(smem_u32(&hdr->empty[s]));
           }
         } else if (elect_one()) {
-          const uint64_t da0 = make_smem_desc(tiles_addr + s * stage_bytes, p.sbo, p.layout_type);
-          const uint64_t db0 = make_smem_desc(p.b_resident ? bres_addr + static_cast<uint32_t>(kb0) * b_bytes : tiles_addr + s * stage_bytes + b_off,
-                                              p.sbo, p.layout_type);
-          const uint32_t a_hi = static_cast<uint32_t>(da0 >> 32), b_hi = static_cast<uint32_t>(db0 >> 32);
-          uint32_t a_lo = static_cast<uint32_t>(da0), b_lo = static_cast<uint32_t>(db0);
+          const uint32_t a_hi = d_hi, b_hi = d_hi;
+          uint32_t a_lo = a_lo0, b_lo = b_lo0;
           const uint32_t da_step = sub_bytes >> 4, db_step = (p.b_resident ? b_bytes : sub_bytes) >> 4;
           const uint32_t a2 = a_bytes >> 4;            // pair mode: the second tile's A block follows the first's
           const uint32_t tmem_d2 = tmem_d + p.acc_stride;
@@ -652,7 +643,7 @@ gemm_i8_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
   } else if (FUSE && warp == 3) {
     // ------------------------------------------------------------ residual producer (FUSE)
     // The residual tile of the Add (same rows and columns as the output tile) is brought into the
-    // staging memory by TMA, two tiles deep, so that the epilogue reads it from shared memory.
+    // residual buffers by TMA, two tiles deep, so that the epilogue reads it from shared memory.
     // First of all the Add's 64 KB table (a constant of the graph, so no waiting for earlier kernels): four bulk copies
     // that land while the first tiles are loaded and multiplied; the epilogue warps wait for them before their first
     // look-up.  (Copied by the epilogue threads themselves with ordinary loads, the table kept them from their first
@@ -663,9 +654,9 @@ gemm_i8_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
       for (int q = 0; q < 4; ++q) bulk_load(smem_u32(add_tab) + q * 16384u, p.ep.add_table + q * 16384, 16384u, full);
     }
     __syncwarp();
-    if (p.res_span) {
+    if (p.res_tma) {
       pdl_wait();   // the residual is an earlier kernel's output
-      const int span = p.res_span;
+      const int span = p.blk_w;
       int nload = 0;
       for (int blk = 0; blk * span < p.BNd; ++blk)
         if (n_tile * p.BNd + blk * span < p.Ocp) ++nload;
@@ -673,21 +664,21 @@ gemm_i8_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
       bool ok = true;
       int m_tile = m_tile0, j = 0;
       for (int tile = blockIdx.x; ok && tile < num_tiles; tile += gridDim.x, m_tile += m_step, ++j) {
-        const uint32_t b = j & 1, ph = (j >> 1) & 1;
+        const uint32_t b = j & ((1 << p.res_shift) - 1), ph = (j >> p.res_shift) & 1;
         ok = mbar_wait(smem_u32(&hdr->res_empty[b]), ph ^ 1, abort_flag, p.status, 6, p.wait_limit);
         ok = __all_sync(0xffffffffu, ok);
         if (!ok) break;
         if (elect_one()) {
           const uint32_t full = smem_u32(&hdr->res_full[b]);
           mbar_arrive_expect_tx(full, static_cast<uint32_t>(nload) * box_bytes);
-          uint32_t dst = smem_u32(staging + b * staging_bytes);
+          uint32_t dst = smem_u32(res_tiles + b * res_bytes);
           for (int blk = 0; blk < nload; ++blk, dst += static_cast<uint32_t>(kBlockM) * span) {
             const int col = n_tile * p.BNd + blk * span;
             if (p.conv) {
               const int rest = m_tile / p.tiles_w;
-              tma_load_4d(dst, &map_d, col, (m_tile % p.tiles_w) * p.TW, (rest % p.tiles_h) * p.TH, (rest / p.tiles_h) * p.TN, full);
+              tma_load_4d(dst, &map_r, col, (m_tile % p.tiles_w) * p.TW, (rest % p.tiles_h) * p.TH, (rest / p.tiles_h) * p.TN, full);
             } else {
-              tma_load_2d(dst, &map_d, col, m_tile * kBlockM, full);
+              tma_load_2d(dst, &map_r, col, m_tile * kBlockM, full);
             }
           }
         }
@@ -696,78 +687,80 @@ gemm_i8_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
     }
   } else if (warp >= kFirstEpilogueWarp) {
     // ------------------------------------------------------------ epilogue
-    // The epilogue's constants (this N tile's folded bias and scales) are staged by the epilogue warps themselves,
-    // behind a barrier of their own: the producers and the MMA warp are already at work on the first tile meanwhile.
+    // The epilogue's constants (this N tile's columns) are staged by the epilogue warps themselves, behind a barrier of
+    // their own: the producers and the MMA warp are already at work on the first tile meanwhile.
+    constexpr int w = 16 * STEPS;
     for (int i = threadIdx.x - kFirstEpilogueWarp * 32; i < p.BNd; i += kEpilogueThreads) {
-      const int oc = n_tile * p.BNd + i;
-      hdr->bias[i] = oc < p.Ocp ? p.ep.bias_full[oc] : 0;
-      hdr->scale[i] = oc < p.Ocp ? p.ep.acc_scale[oc] : 0.0f;
+      // entry i: 16-column step (i % w) / 16 of block i / w, thread quad position (i / 4) % 4, its column i % 4
+      const int in_blk = i % w, quad = (in_blk >> 2) & 3;
+      const int ch = p.plain_order ? i - in_blk + (((i >> 1) & 1) << 3) + 2 * quad + (i & 1) : i - in_blk + quad * (w >> 2) + ((in_blk >> 4) << 2) + (i & 3);
+      const int oc = n_tile * p.BNd + ch;
+      FixedColumn f = {0, 0, oc < p.Ocp ? 0xFFFFFFFFu : 0u};   // without fixed-point constants: always redo
+      if (oc < p.Ocp && p.ep.fix) *reinterpret_cast<uint4*>(&f) = __ldg(reinterpret_cast<const uint4*>(p.ep.fix + oc));
+      hdr->cols.bias[i] = oc < p.Ocp ? p.ep.bias_full[oc] : 0;
+      hdr->cols.scale[i] = oc < p.Ocp ? p.ep.acc_scale[oc] : 0.0f;
+      hdr->cols.mul[i] = f.mul;
+      hdr->cols.add[i] = f.add;
+      if (i % 16 == 0) hdr->cols.window[i >> 4] = f.window;
     }
     epilogue_barrier();
     const int ew = warp - kFirstEpilogueWarp;     // 0..15
     const int quarter = warp & 3;                 // TMEM lanes [32*quarter, +32) belong to this warp
-    const int col_group = ew >> 2;                // this warp takes 16-column chunks col_group, col_group+4, ...
+    const int col_group = ew >> 2;                // run of column blocks (or team) of this warp
     const int row_in_tile = quarter * 32 + lane;
-    const bool store_issuer = threadIdx.x == kFirstEpilogueWarp * 32;
+    const int g = lane >> 2, q = lane & 3;        // this thread's rows are g + 8 k of the warp's 32, its columns the q-th quarter of a block
     const OutQuant oq = p.ep.out;
-    const RequantConsts rc = make_requant_consts(oq, p.exact_only);
-    // position of this thread's 16-byte chunks inside a staging column block
-    const int span_b = p.store_span;
-    const int span_r = FUSE ? p.res_span : 0;        // never both: a fused Add stores directly
-    const int span_s = span_b ? span_b : span_r;     // layout of the staging memory either way
-    const int span_shift = span_s == 128 ? 7 : (span_s == 64 ? 6 : 5);
-    const int swz = span_s == 128 ? (row_in_tile & 7) : span_s == 64 ? ((row_in_tile >> 1) & 3) : ((row_in_tile >> 2) & 1);
-    int j = 0;
-    // Once a wait has given up (alive == false) a thread does no more work, but it keeps running the
-    // loop and both barriers of every tile, so the other epilogue threads never wait for it.
-    // Output row of this thread in M tile m_tile (-1 outside the tensor) and, for a border pixel of a padded
-    // convolution, the row of corrections of its class.
-    auto locate = [&](int m_tile, long long& row, const int32_t*& corr_row) {
+    const uint32_t out_flip = oq.lo < 0 ? 0x80808080u : 0u;
+    const int shl = EXTRA ? p.ep.fix_shl : 0;
+    const int nblk = p.BNd / w;
+    const int blk0 = p.teams ? 0 : col_group * p.blk_per_group, blk1 = p.teams ? nblk : min(nblk, blk0 + p.blk_per_group);
+    // Once a wait has given up (alive == false) a thread does no more work, but it keeps running the loop.
+    // Output row of this lane (-1 outside the tensor) in M tile m_tile of a convolution and its border class.
+    auto locate = [&](int m_tile, int& row, int& cls) {
       row = -1;
-      corr_row = nullptr;
-      if (p.conv) {
-        if (!span_b || FUSE || (EXTRA && p.ep.border_corr)) {
-          const int tw = m_tile % p.tiles_w, rest = m_tile / p.tiles_w;
-          const int th = rest % p.tiles_h, tn = rest / p.tiles_h;
-          const int i = row_in_tile % p.TW, r2 = row_in_tile / p.TW;
-          const int jh = r2 % p.TH, l = r2 / p.TH;
-          const int wo = tw * p.TW + i, ho = th * p.TH + jh, n = tn * p.TN + l;
-          if (l < p.TN && wo < p.Wo && ho < p.Ho && n < p.Nimg) {
-            row = (static_cast<long long>(n) * p.Ho + ho) * p.Wo + wo;
-            if (EXTRA && p.ep.border_corr) {
-              const int cls = __ldg(p.ep.row_class + ho) * p.ep.n_col_classes + __ldg(p.ep.col_class + wo);
-              if (cls) corr_row = p.ep.border_corr + static_cast<size_t>(cls) * p.Ocp + n_tile * p.BNd;
-            }
-          }
-        }
-      } else if (!span_b || FUSE) {
-        row = static_cast<long long>(m_tile) * kBlockM + row_in_tile;
-        if (row >= p.M) row = -1;
+      cls = 0;
+      const int tw = m_tile % p.tiles_w, rest = m_tile / p.tiles_w;
+      const int th = rest % p.tiles_h, tn = rest / p.tiles_h;
+      const int i = row_in_tile % p.TW, r2 = row_in_tile / p.TW;
+      const int jh = r2 % p.TH, l = r2 / p.TH;
+      const int wo = tw * p.TW + i, ho = th * p.TH + jh, n = tn * p.TN + l;
+      if (l < p.TN && wo < p.Wo && ho < p.Ho && n < p.Nimg) {
+        row = (n * p.Ho + ho) * p.Wo + wo;
+        if (EXTRA && p.ep.border_corr) cls = __ldg(p.ep.row_class + ho) * p.ep.n_col_classes + __ldg(p.ep.col_class + wo);
       }
     };
     bool alive = true;
     bool table_ready = !FUSE;
     const int j_step = p.teams ? kGroups : 1;               // team mode: warp group col_group takes tiles j = col_group (mod kGroups)
-    const int c_first = p.teams ? 0 : col_group * 16;       // and all of their chunks
-    const int c_step = p.teams ? 16 : kGroups * 16;
-    j = p.teams ? col_group : 0;
+    int j = p.teams ? col_group : 0;
     for (int tile = blockIdx.x + j * static_cast<int>(gridDim.x); tile < num_tiles; tile += j_step * static_cast<int>(gridDim.x), j += j_step) {
       const int m_tile = m_tile0 + j * m_step;
       const uint32_t a = j & ((1 << p.acc_shift) - 1), aph = (j >> p.acc_shift) & 1;
-      uint8_t* stage_out = staging + (j & 1) * staging_bytes;
-      long long row;                 // direct-store path: output row (pixel index into D), -1 outside the tensor
-      const int32_t* corr_row;       // border pixels of a padded convolution: their correction, this N tile
-      locate(m_tile, row, corr_row);
+      const int rb = j & ((1 << p.res_shift) - 1);   // residual buffer
+      int row[4], cls[4];            // output rows (pixel indexes into D) of this thread, -1 outside the tensor; border classes
+      if (p.conv) {
+        int my_row, my_cls;
+        locate(m_tile, my_row, my_cls);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          row[k] = __shfl_sync(0xffffffffu, my_row, g + 8 * k);
+          cls[k] = EXTRA ? __shfl_sync(0xffffffffu, my_cls, g + 8 * k) : 0;
+        }
+      } else {
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          row[k] = m_tile * kBlockM + quarter * 32 + g + 8 * k;
+          if (row[k] >= p.M) row[k] = -1;
+          cls[k] = 0;
+        }
+      }
       TC_EPI(j, 0);
       if (alive) alive = mbar_wait(smem_u32(&hdr->tmem_full[a]), aph, abort_flag, p.status, 4, p.wait_limit);
       alive = __all_sync(0xffffffffu, alive);   // the TMEM loads below are warp-wide
-      if (!alive) {
-        if (span_b) epilogue_barrier();
-        continue;
-      }
+      if (!alive) continue;
       TC_EPI(j, 1);
-      if (span_r) {
-        alive = mbar_wait(smem_u32(&hdr->res_full[j & 1]), (j >> 1) & 1, abort_flag, p.status, 7, p.wait_limit);
+      if (p.res_tma) {
+        alive = mbar_wait(smem_u32(&hdr->res_full[rb]), (j >> p.res_shift) & 1, abort_flag, p.status, 7, p.wait_limit);
         alive = __all_sync(0xffffffffu, alive);
         if (!alive) continue;
       }
@@ -781,105 +774,128 @@ gemm_i8_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
       if (warp == kFirstEpilogueWarp && lane == 0) TC_TRACE(2, j, 0);
       tc_fence_after();
       const uint32_t taddr = tmem_base + a * p.acc_stride + (static_cast<uint32_t>(quarter * 32) << 16);
-      // Chunks col_group, col_group + 4, ... of 16 columns; the TMEM load of the next chunk is in flight
-      // while the current one is requantized.
-      int sub = 0;
+      int sub[4] = {0, 0, 0, 0};
       if (EXTRA && p.dz != 0) {
-        // S = sum of this row's inputs: the accumulator column of the all-ones weight row
+        // S = sum of a row's inputs: the accumulator column of the all-ones weight row
         int s_val;
         tc_ld_32x1(taddr + p.BNd, s_val);
         tc_ld_wait1(s_val);
-        sub = p.dz * s_val;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) sub[k] = p.dz * __shfl_sync(0xffffffffu, s_val, g + 8 * k);
       }
-      auto emit = [&](const int (&acc)[16], int c0) {
-        const int cbase = n_tile * p.BNd + c0;
-        if (!span_b && (row < 0 || cbase + 16 > p.Ocp)) return;
-        uint4 res16 = make_uint4(0, 0, 0, 0);
-        if (FUSE) {
-          if (span_r) {
-            const int blk = c0 >> span_shift, chunk = (c0 & (span_r - 1)) >> 4;
-            res16 = *reinterpret_cast<const uint4*>(staging + (j & 1) * staging_bytes + static_cast<size_t>(blk) * kBlockM * span_r +
-                                                    row_in_tile * span_r + ((chunk ^ swz) << 4));
-          } else if (row >= 0 && cbase + 16 <= p.Ocp) {
-            res16 = __ldg(reinterpret_cast<const uint4*>(p.ep.add_residual + row * p.ldd + cbase));
+      // One block of 16 * STEPS columns: the thread's 4 * STEPS bytes of each of its four rows.
+      auto block = [&](int cb) {
+        uint32_t out[4][STEPS];
+#pragma unroll
+        for (int s = 0; s < STEPS; ++s) {
+          int acc[16];
+          tc_ld_16x16(taddr + cb + 16 * s, acc);
+          tc_ld_16x16(taddr + cb + 16 * s + (16u << 16), acc + 8);
+          const int c = cb + 16 * s + 4 * q;     // this thread's entries of the column constants
+          const int4 m = *reinterpret_cast<const int4*>(&hdr->cols.mul[c]);
+          const longlong2 a01 = *reinterpret_cast<const longlong2*>(&hdr->cols.add[c]), a23 = *reinterpret_cast<const longlong2*>(&hdr->cols.add[c + 2]);
+          const uint32_t window = hdr->cols.window[(cb >> 4) + s];
+          tc_ld_wait(acc);
+          int x[4][4];
+          uint32_t low[4];
+#pragma unroll
+          for (int k = 0; k < 4; ++k) {
+            const int b0 = (k >> 1) * 8 + (k & 1) * 2;
+            x[k][0] = acc[b0]; x[k][1] = acc[b0 + 1]; x[k][2] = acc[b0 + 4]; x[k][3] = acc[b0 + 5];
+            if (EXTRA) {
+              x[k][0] -= sub[k]; x[k][1] -= sub[k]; x[k][2] -= sub[k]; x[k][3] -= sub[k];
+              const int oc = n_tile * p.BNd + cb + q * 4 * STEPS + 4 * s;
+              if (cls[k] && oc < p.Ocp) {
+                const int4 c4 = __ldg(reinterpret_cast<const int4*>(p.ep.border_corr + static_cast<size_t>(cls[k]) * p.Ocp + oc));
+                x[k][0] += c4.x; x[k][1] += c4.y; x[k][2] += c4.z; x[k][3] += c4.w;
+              }
+            }
+#ifdef B2VX_ABL_NOREQ
+            out[k][s] = x[k][0] ^ x[k][1] ^ x[k][2] ^ x[k][3] ^ m.x;
+            low[k] = 0xFFFFFFFFu;
+#else
+            out[k][s] = requant_fixed4(x[k], m, a01, a23, shl, low[k]);
+#endif
+          }
+          if (min(__vimin3_u32(low[0], low[1], low[2]), low[3]) < window) {
+#pragma unroll
+            for (int k = 0; k < 4; ++k)
+              if (low[k] < window) out[k][s] = requant_redo4(out[k][s], x[k][0], x[k][1], x[k][2], x[k][3], &hdr->cols, c, window, shl, oq);
+          }
+#pragma unroll
+          for (int k = 0; k < 4; ++k) out[k][s] ^= out_flip;
+        }
+        const int col = n_tile * p.BNd + cb + q * 4 * STEPS;
+        const bool col_ok = col + 4 * STEPS <= p.Ocp;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          const size_t at = static_cast<size_t>(row[k]) * p.ldd + col;
+          const bool ok = row[k] >= 0 && col_ok;
+          if (FUSE) {
+            uint32_t res[STEPS];
+            if (p.res_tma) {
+              // 16-byte pieces are swizzled by the row: by row bits 1-2 in 64-byte rows, by bit 2 in 32-byte rows
+              const int r = quarter * 32 + g + 8 * k;
+              const uint8_t* base = res_tiles + rb * res_bytes + cb * kBlockM + r * 16 * STEPS;
+              if constexpr (STEPS == 4) {
+                const uint4 v = *reinterpret_cast<const uint4*>(base + ((q ^ ((r >> 1) & 3)) << 4));
+                res[0] = v.x; res[1] = v.y; res[2] = v.z; res[3] = v.w;
+              } else if constexpr (STEPS == 2) {
+                const uint2 v = *reinterpret_cast<const uint2*>(base + (((q >> 1) ^ ((r >> 2) & 1)) << 4) + ((q & 1) << 3));
+                res[0] = v.x; res[1] = v.y;
+              } else {
+                res[0] = *reinterpret_cast<const uint32_t*>(base + q * 4);
+              }
+            } else {
+#pragma unroll
+              for (int s = 0; s < STEPS; ++s) res[s] = 0;
+              if (ok) {
+                if constexpr (STEPS == 4) {
+                  const uint4 v = __ldg(reinterpret_cast<const uint4*>(p.ep.add_residual + at));
+                  res[0] = v.x; res[1] = v.y; res[2] = v.z; res[3] = v.w;
+                } else if constexpr (STEPS == 2) {
+                  const uint2 v = __ldg(reinterpret_cast<const uint2*>(p.ep.add_residual + at));
+                  res[0] = v.x; res[1] = v.y;
+                } else {
+                  res[0] = __ldg(reinterpret_cast<const uint32_t*>(p.ep.add_residual + at));
+                }
+              }
+            }
+#pragma unroll
+            for (int s = 0; s < STEPS; ++s) {
+#ifdef B2VX_ABL_NOLUT
+              out[k][s] ^= res[s];
+#else
+              out[k][s] = add_lut_word(out[k][s], res[s], add_tab);
+#endif
+            }
+          }
+          if (!ok) continue;
+          if constexpr (STEPS == 4) {
+            *reinterpret_cast<uint4*>(p.D + at) = make_uint4(out[k][0], out[k][1], out[k][2], out[k][3]);
+          } else if constexpr (STEPS == 2) {
+            *reinterpret_cast<uint2*>(p.D + at) = make_uint2(out[k][0], out[k][1]);
+          } else if (!p.plain_order) {
+            *reinterpret_cast<uint32_t*>(p.D + at) = out[k][0];
+          } else {   // columns 2 q, 2 q + 1 and 8 + 2 q, 9 + 2 q of the 16
+            uint8_t* d = p.D + at - 4 * q + 2 * q;
+            *reinterpret_cast<uint16_t*>(d) = static_cast<uint16_t>(out[k][0]);
+            *reinterpret_cast<uint16_t*>(d + 8) = static_cast<uint16_t>(out[k][0] >> 16);
           }
         }
-#ifdef B2VX_ABL_NOREQ
-        uint4 out16 = make_uint4(acc[0] ^ acc[4] ^ acc[8] ^ acc[12], acc[1] ^ acc[5] ^ acc[9] ^ acc[13], acc[2] ^ acc[6] ^ acc[10] ^ acc[14],
-                                 acc[3] ^ acc[7] ^ acc[11] ^ acc[15]);
-#else
-        uint4 out16 = requant_chunk16<EXTRA>(acc, &hdr->bias[c0], &hdr->scale[c0], rc, sub,
-                                             (corr_row && cbase + 16 <= p.Ocp) ? corr_row + c0 : nullptr);
-#endif
-#ifdef B2VX_ABL_NOLUT
-        if (FUSE) { out16.x ^= res16.x; out16.y ^= res16.y; out16.z ^= res16.z; out16.w ^= res16.w; }
-        else
-#endif
-        if (FUSE) {
-          out16.x = add_lut_word(out16.x, res16.x, add_tab);
-          out16.y = add_lut_word(out16.y, res16.y, add_tab);
-          out16.z = add_lut_word(out16.z, res16.z, add_tab);
-          out16.w = add_lut_word(out16.w, res16.w, add_tab);
-        }
-        if (span_b) {
-          const int blk = c0 >> span_shift, chunk = (c0 & (span_b - 1)) >> 4;   // span_b is 32, 64 or 128
-          *reinterpret_cast<uint4*>(stage_out + static_cast<size_t>(blk) * kBlockM * span_b + row_in_tile * span_b +
-                                    ((chunk ^ swz) << 4)) = out16;
-        } else {
-          *reinterpret_cast<uint4*>(p.D + row * p.ldd + cbase) = out16;
-        }
       };
-      {
-        int acc_a[16], acc_b[16];
-        int c0 = c_first;
-        if (c0 < p.BNd) tc_ld_32x16(taddr + c0, acc_a);
-        while (c0 < p.BNd) {
-          tc_ld_wait(acc_a);
-          if (c0 + c_step < p.BNd) tc_ld_32x16(taddr + c0 + c_step, acc_b);
-          emit(acc_a, c0);
-          c0 += c_step;
-          if (c0 >= p.BNd) break;
-          tc_ld_wait(acc_b);
-          if (c0 + c_step < p.BNd) tc_ld_32x16(taddr + c0 + c_step, acc_a);
-          emit(acc_b, c0);
-          c0 += c_step;
-        }
-      }
+#pragma unroll 1
+      for (int blk = blk0; blk < blk1; ++blk) block(blk * w);
       TC_EPI(j, 3);
       // accumulator buffer (and residual buffer) free again
       tc_fence_before();
       __syncwarp();
       if (lane == 0) {
         mbar_arrive(smem_u32(&hdr->tmem_empty[a]));
-        if (span_r) mbar_arrive(smem_u32(&hdr->res_empty[j & 1]));
-      }
-      if (span_b) {
-        // One barrier per tile.  Before it, the issuer makes sure the previous tile's store has read
-        // its staging buffer (it was issued a whole tile ago): after the barrier every thread may
-        // write that buffer for the next tile, and the issuer stores the tile just written.
-        fence_smem_to_async();
-        if (store_issuer) tma_store_wait_read<0>();
-        epilogue_barrier();
-        if (store_issuer) {
-          const int nblk = p.BNd / span_b;
-          for (int blk = 0; blk < nblk; ++blk) {
-            const int col = n_tile * p.BNd + blk * span_b;
-            if (col >= p.Ocp) break;
-            const uint32_t src = smem_u32(stage_out + static_cast<size_t>(blk) * kBlockM * span_b);
-            if (p.conv) {
-              const int rest = m_tile / p.tiles_w;
-              tma_store_4d(&map_d, src, col, (m_tile % p.tiles_w) * p.TW, (rest % p.tiles_h) * p.TH, (rest / p.tiles_h) * p.TN);
-            }
-            else tma_store_2d(&map_d, src, col, m_tile * kBlockM);
-          }
-          tma_store_commit();
-        }
+        if (p.res_tma) mbar_arrive(smem_u32(&hdr->res_empty[rb]));
       }
       if (warp == kFirstEpilogueWarp && lane == 0) TC_TRACE(2, j, 1);
     }
-    // The staging buffers only have to stay intact until the last store has read them; the writes
-    // themselves are complete, like any other store, when the grid is.
-    if (store_issuer) tma_store_wait_read<0>();
   }
 
   // ---------------------------------------------------------------- common exit
@@ -1004,7 +1020,7 @@ bool encode_u8(CUtensorMap* map, const void* base, int rank, const uint64_t* dim
 struct GemmTcPlan {
   CUtensorMap map_a;
   CUtensorMap map_b;
-  CUtensorMap map_d;
+  CUtensorMap map_r;   // residual tile of a fused Add
   GemmParams params;
   int grid;
   size_t smem;
@@ -1020,8 +1036,19 @@ int gemm_tc_available(void) {
 
 namespace {
 
+typedef void (*GemmKernel)(CUtensorMap, CUtensorMap, CUtensorMap, GemmParams);
+
+template <bool EXTRA, bool FUSE>
+GemmKernel kernel_of_width(int blk_w) {
+  return blk_w == 64 ? gemm_i8_tc_kernel<EXTRA, FUSE, 4> : blk_w == 32 ? gemm_i8_tc_kernel<EXTRA, FUSE, 2> : gemm_i8_tc_kernel<EXTRA, FUSE, 1>;
+}
+GemmKernel kernel_variant(bool extra, bool fuse, int blk_w) {
+  return extra ? (fuse ? kernel_of_width<true, true>(blk_w) : kernel_of_width<true, false>(blk_w))
+               : (fuse ? kernel_of_width<false, true>(blk_w) : kernel_of_width<false, false>(blk_w));
+}
+
 // Everything of a plan that does not depend on how A is addressed: N tiling, K block / swizzle mode,
-// output staging, stage count, TMEM columns, instruction descriptor, the B tensor map.
+// column blocks, stage count, TMEM columns, instruction descriptor, the B tensor map.
 // Kspan is the K extent one tap (or the whole GEMM) covers, used to pick BK.
 // halo_w, halo_h: extent in pixels of the input patch (tile + halo) the caller would load per channel block if the plan
 // turns out to allow the halo mode of the implicit convolution (0: not asked for).
@@ -1035,11 +1062,15 @@ bool finish_plan(GemmTcPlan* plan, const int8_t* B, int a_signed, int Np, int Kp
     p.n_tiles = tiling->n_tiles;
     p.BN = tiling->rows;
     p.BNd = tiling->data;
+    p.blk_w = tiling->blk_w;
+    if (p.blk_w < 16 || p.BNd % p.blk_w) { *why = "gemm_tc: bad column blocks"; return false; }
     if (p.BN > 256 || (p.BN & 15) || (p.BNd & 15) || p.BNd < 16 || p.BNd > p.BN) { *why = "gemm_tc: bad N tiling"; return false; }
   } else {
     p.n_tiles = (Np + 255) / 256;
     p.BN = (((Np + p.n_tiles - 1) / p.n_tiles) + 15) & ~15;
     p.BNd = p.BN;
+    p.blk_w = 16;
+    p.plain_order = 1;
   }
   if (p.n_tiles * p.BN != Np) { *why = "gemm_tc: weight rows must be packed to n_tiles*BN"; return false; }
   p.dz = e.dz_uniform;
@@ -1054,35 +1085,28 @@ bool finish_plan(GemmTcPlan* plan, const int8_t* B, int a_signed, int Np, int Kp
   p.BK = best_bk;
   p.layout_type = p.BK == 128 ? 2u : (p.BK == 64 ? 4u : 6u);
   p.sbo = 8u * p.BK;
-  // Output staging for the TMA store: column blocks as wide as the widest swizzle span dividing BN.
-  p.store_span = p.BNd % 128 == 0 ? 128 : (p.BNd % 64 == 0 ? 64 : (p.BNd % 32 == 0 ? 32 : 0));
-  // Measured over the ResNet-50 layer shapes, threads storing their 16-byte pieces themselves beat the
-  // staged TMA store (no CTA-wide barrier per tile, epilogue warps drift apart and overlap tiles, and
-  // the staging memory goes to the operand ring instead), so that is the default;
-  // B2VX_TC_STORE=tma selects the staged store.
-  static const bool tma_store = [] { const char* e = std::getenv("B2VX_TC_STORE"); return e && std::strcmp(e, "tma") == 0; }();
-  p.res_span = e.add_residual != nullptr ? p.store_span : 0;
-  if (!tma_store || e.add_residual != nullptr) p.store_span = 0;
   const size_t add_table_bytes = e.add_residual != nullptr ? 65536 : 0;
   static const bool no_teams = [] { const char* e2 = std::getenv("B2VX_TC_TEAMS"); return e2 && std::strcmp(e2, "0") == 0; }();
   // (wide_teams: the caller found the launch bound by its epilogue, short K and many tiles per CTA, so tiles of up to 128
   // columns also go one per warp group: four tiles in flight instead of four passes over every tile)
-  p.teams = ((p.BNd <= 64 || (wide_teams && p.BN <= 128)) && p.store_span == 0 && !no_teams) ? kGroups : 0;
-  if (p.teams) p.res_span = 0;   // four tiles in flight do not fit the two residual buffers: threads load their pieces
-  if (p.res_span) {
-    // The Add's table and two residual tiles leave less for the operand ring: three stages must remain,
+  p.teams = ((p.BNd <= 64 || (wide_teams && p.BN <= 128)) && !no_teams) ? kGroups : 0;
+  p.blk_per_group = (p.BNd / p.blk_w + kGroups - 1) / kGroups;
+  p.res_tma = e.add_residual != nullptr && !p.plain_order ? 1 : 0;
+  p.res_shift = p.teams ? 2 : 1;
+  if (p.res_tma) {
+    // The Add's table and the residual tiles leave less for the operand ring: three stages must remain,
     // with 64-byte K blocks if 128-byte ones do not fit (these layers are bound by their epilogue, not by
     // the main loop); failing that the epilogue threads load their residual pieces themselves.
-    const size_t left = kSmemBudget - 2048 - sizeof(SmemHeader) - add_table_bytes - 2 * static_cast<size_t>(kBlockM) * p.BNd;
+    const size_t left = kSmemBudget - 2048 - sizeof(SmemHeader) - add_table_bytes - (static_cast<size_t>(kBlockM) * p.BNd << p.res_shift);
     if (left < 3 * static_cast<size_t>(kBlockM + p.BN) * p.BK && p.BK == 128) {
       p.BK = 64;
       p.layout_type = 4u;
       p.sbo = 8u * p.BK;
     }
-    if (left < 3 * static_cast<size_t>(kBlockM + p.BN) * p.BK) p.res_span = 0;
+    if (left < 3 * static_cast<size_t>(kBlockM + p.BN) * p.BK) p.res_tma = 0;
   }
   const int kblocks_per_tile = taps * ((Kspan + p.BK - 1) / p.BK);
-  const size_t staging = (p.store_span || p.res_span) ? 2 * static_cast<size_t>(kBlockM) * p.BNd : 0;
+  const size_t staging = p.res_tma ? static_cast<size_t>(kBlockM) * p.BNd << p.res_shift : 0;
   // A and B tiles are whole swizzle atoms (8 rows x BK bytes; BN and 128 are multiples of 8), so every
   // tile start keeps the alignment its swizzle pattern repeats on (8*BK bytes) relative to the 1024-byte
   // aligned start of the ring.  Several k-blocks share a stage (one barrier round trip) when they are
@@ -1133,7 +1157,6 @@ bool finish_plan(GemmTcPlan* plan, const int8_t* B, int a_signed, int Np, int Kp
   p.idesc = (2u << 4) | (static_cast<uint32_t>(a_signed ? 1 : 0) << 7) | (1u << 10) |
             (static_cast<uint32_t>(p.BN >> 3) << 17) | (static_cast<uint32_t>(kBlockM >> 4) << 24);
   p.ep = e;
-  p.exact_only = e.exact_only;
   p.wait_limit = kWaitLimitCycles;
   p.tx_extra = 0;
   p.D = static_cast<uint8_t*>(D);
@@ -1152,16 +1175,21 @@ bool finish_plan(GemmTcPlan* plan, const int8_t* B, int a_signed, int Np, int Kp
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev < 0 || dev >= 64 || !attr_set[dev]) {
-    if (cudaFuncSetAttribute(gemm_i8_tc_kernel<false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024) != cudaSuccess ||
-        cudaFuncSetAttribute(gemm_i8_tc_kernel<true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024) != cudaSuccess ||
-        cudaFuncSetAttribute(gemm_i8_tc_kernel<false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024) != cudaSuccess ||
-        cudaFuncSetAttribute(gemm_i8_tc_kernel<true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024) != cudaSuccess) {
+    bool raised = true;
+    for (int v = 0; v < 12; ++v)
+      raised = raised && cudaFuncSetAttribute(kernel_variant(v & 1, v & 2, 16 << (v >> 2)), cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024) == cudaSuccess;
+    if (!raised) {
       *why = "gemm_tc: cannot raise the dynamic shared memory limit";
       return false;
     }
     if (dev >= 0 && dev < 64) attr_set[dev] = true;
   }
   return true;
+}
+
+// Swizzle of a [rows][w] column block of the residual tile.
+CUtensorMapSwizzle block_swizzle(int w) {
+  return w == 64 ? CU_TENSOR_MAP_SWIZZLE_64B : (w == 32 ? CU_TENSOR_MAP_SWIZZLE_32B : CU_TENSOR_MAP_SWIZZLE_NONE);
 }
 
 void set_grid(GemmTcPlan* plan) {
@@ -1196,7 +1224,7 @@ GemmTcPlan* gemm_tc_plan_create(const void* A, int a_signed, const int8_t* B, in
   GemmTcPlan* plan = new GemmTcPlan();
   GemmParams& p = plan->params;
   std::memset(&p, 0, sizeof(p));
-  std::memset(&plan->map_d, 0, sizeof(plan->map_d));
+  std::memset(&plan->map_r, 0, sizeof(plan->map_r));
   const char* why = "";
   // pair mode where the main loop dwarfs the epilogue (K of 4096 or more) and there are at least two tiles per SM
   int sms = 148;
@@ -1219,12 +1247,10 @@ GemmTcPlan* gemm_tc_plan_create(const void* A, int a_signed, const int8_t* B, in
   const uint64_t adims[2] = {static_cast<uint64_t>(Kp), static_cast<uint64_t>(M)};
   const uint32_t abox[2] = {static_cast<uint32_t>(p.BK), kBlockM};
   bool ok = encode_u8(&plan->map_a, A, 2, adims, abox, nullptr, swizzle_of(p.BK));
-  if (ok && (p.store_span || p.res_span)) {
-    // the output tile for the staged store, or (fused Add) the residual tile of the same geometry
-    const int span = p.store_span ? p.store_span : p.res_span;
-    const uint64_t ddims[2] = {static_cast<uint64_t>(ldd), static_cast<uint64_t>(M)};
-    const uint32_t dbox[2] = {static_cast<uint32_t>(span), kBlockM};
-    ok = encode_u8(&plan->map_d, p.store_span ? D : static_cast<const void*>(e.add_residual), 2, ddims, dbox, nullptr, swizzle_of(span));
+  if (ok && p.res_tma) {
+    const uint64_t rdims[2] = {static_cast<uint64_t>(ldd), static_cast<uint64_t>(M)};
+    const uint32_t rbox[2] = {static_cast<uint32_t>(p.blk_w), kBlockM};
+    ok = encode_u8(&plan->map_r, e.add_residual, 2, rdims, rbox, nullptr, block_swizzle(p.blk_w));
   }
   if (!ok) {
     delete plan;
@@ -1249,7 +1275,7 @@ GemmTcPlan* gemm_tc_conv_plan_create(const void* X, int x_signed, const int8_t* 
   GemmTcPlan* plan = new GemmTcPlan();
   GemmParams& p = plan->params;
   std::memset(&p, 0, sizeof(p));
-  std::memset(&plan->map_d, 0, sizeof(plan->map_d));
+  std::memset(&plan->map_r, 0, sizeof(plan->map_r));
   const char* why = "";
   const int Kp = g.kh * g.kw * g.Cp;
   // Halo mode (see GemmParams): a tile is 8 x 16 output pixels of one image.  Asked for when the convolution has more
@@ -1299,11 +1325,10 @@ GemmTcPlan* gemm_tc_conv_plan_create(const void* X, int x_signed, const int8_t* 
                            static_cast<uint32_t>(p.halo ? halo_h : (bh - 1) * g.sy + 1), static_cast<uint32_t>(bn)};
   const uint32_t estr[4] = {1, static_cast<uint32_t>(g.sx), static_cast<uint32_t>(g.sy), 1};
   bool ok = encode_u8(&plan->map_a, X, 4, dims, box, estr, swizzle_of(p.BK));
-  if (ok && (p.store_span || p.res_span)) {
-    const int span = p.store_span ? p.store_span : p.res_span;
-    const uint64_t ddims[4] = {static_cast<uint64_t>(g.Ocp), static_cast<uint64_t>(g.Wo), static_cast<uint64_t>(g.Ho), static_cast<uint64_t>(g.N)};
-    const uint32_t dbox[4] = {static_cast<uint32_t>(span), static_cast<uint32_t>(bw), static_cast<uint32_t>(bh), static_cast<uint32_t>(bn)};
-    ok = encode_u8(&plan->map_d, p.store_span ? D : static_cast<const void*>(e.add_residual), 4, ddims, dbox, nullptr, swizzle_of(span));
+  if (ok && p.res_tma) {
+    const uint64_t rdims[4] = {static_cast<uint64_t>(g.Ocp), static_cast<uint64_t>(g.Wo), static_cast<uint64_t>(g.Ho), static_cast<uint64_t>(g.N)};
+    const uint32_t rbox[4] = {static_cast<uint32_t>(p.blk_w), static_cast<uint32_t>(bw), static_cast<uint32_t>(bh), static_cast<uint32_t>(bn)};
+    ok = encode_u8(&plan->map_r, e.add_residual, 4, rdims, rbox, nullptr, block_swizzle(p.blk_w));
   }
   if (!ok) {
     delete plan;
@@ -1313,6 +1338,22 @@ GemmTcPlan* gemm_tc_conv_plan_create(const void* X, int x_signed, const int8_t* 
   return plan;
 }
 
+namespace {
+
+// Column block width of a tile of `data` columns.  A team works on whole tiles, so there the widest block counts;
+// otherwise the width that leaves the busiest of the four warp groups the fewest columns, the widest among equals.
+int column_block(int data, bool teams) {
+  int best_w = 16, best_cols = 1 << 30;
+  for (int w : {64, 32, 16}) {
+    if (data % w) continue;
+    const int cols = teams ? data : (data / w + kGroups - 1) / kGroups * w;
+    if (cols < best_cols) { best_cols = cols; best_w = w; }
+  }
+  return best_w;
+}
+
+}  // namespace
+
 GemmTcTiling gemm_tc_choose_tiling(long long M, int Ocp, int Kp, int with_s) {
   int dev = 0, sms = 148;
   cudaGetDevice(&dev);
@@ -1321,7 +1362,7 @@ GemmTcTiling gemm_tc_choose_tiling(long long M, int Ocp, int Kp, int with_s) {
   const int max_data = 256 - extra;
   const long long m_tiles = (M + kBlockM - 1) / kBlockM;
   const double rows = static_cast<double>(M < kBlockM ? M : kBlockM);
-  GemmTcTiling best = {0, 0, 0};
+  GemmTcTiling best = {0, 0, 0, 0};
   double best_time = 0.0;
   const bool l2_resident = (static_cast<double>(M) + Ocp) * Kp < 48.0e6;
   // B2VX_TC_BN=<width>: force the tile width (a tuning aid; ignored when it does not fit)
@@ -1333,6 +1374,7 @@ GemmTcTiling gemm_tc_choose_tiling(long long M, int Ocp, int Kp, int with_s) {
       best.n_tiles = nt;
       best.data = data;
       best.rows = data + extra;
+      best.blk_w = column_block(data, data <= 64);
       return best;
     }
   }
@@ -1378,7 +1420,14 @@ GemmTcTiling gemm_tc_choose_tiling(long long M, int Ocp, int Kp, int with_s) {
     best.data = (((Ocp + best.n_tiles - 1) / best.n_tiles) + 15) & ~15;
     best.rows = best.data + extra;
   }
+  // (the same test as wide_teams in gemm_tc_plan_create; block widths are free to choose, a mismatch costs only time)
+  best.blk_w = column_block(best.data, best.data <= 64 || (best.rows <= 128 && Kp <= 128 && m_tiles >= 8LL * sms));
   return best;
+}
+
+int gemm_tc_row_of_channel(const GemmTcTiling& t, int c) {
+  const int w = t.blk_w, in_blk = c % w, quad = in_blk / (w / 4), rem = in_blk % (w / 4);
+  return c - in_blk + 16 * (rem / 4) + 8 * ((rem & 3) >> 1) + 2 * quad + (rem & 1);
 }
 
 // Dense int8 tensor-pipe rate of the current device in TOP/s (2 * MAC): best of `reps` launches of the
@@ -1442,12 +1491,10 @@ GemmTcPlan* gemm_tc_plan_build_in(void* storage, size_t storage_bytes, const voi
   const uint64_t adims[2] = {static_cast<uint64_t>(Kp), static_cast<uint64_t>(M)};
   const uint32_t abox[2] = {static_cast<uint32_t>(p.BK), kBlockM};
   bool ok = encode_u8(&plan->map_a, A, 2, adims, abox, nullptr, swizzle_of(p.BK));
-  if (ok && (p.store_span || p.res_span)) {
-    // the output tile for the staged store, or (fused Add) the residual tile of the same geometry
-    const int span = p.store_span ? p.store_span : p.res_span;
-    const uint64_t ddims[2] = {static_cast<uint64_t>(ldd), static_cast<uint64_t>(M)};
-    const uint32_t dbox[2] = {static_cast<uint32_t>(span), kBlockM};
-    ok = encode_u8(&plan->map_d, p.store_span ? D : static_cast<const void*>(e.add_residual), 2, ddims, dbox, nullptr, swizzle_of(span));
+  if (ok && p.res_tma) {
+    const uint64_t rdims[2] = {static_cast<uint64_t>(ldd), static_cast<uint64_t>(M)};
+    const uint32_t rbox[2] = {static_cast<uint32_t>(p.blk_w), kBlockM};
+    ok = encode_u8(&plan->map_r, e.add_residual, 2, rdims, rbox, nullptr, block_swizzle(p.blk_w));
   }
   if (!ok) return fail("gemm_tc: cuTensorMapEncodeTiled failed");
   set_grid(plan);
@@ -1478,14 +1525,10 @@ cudaError_t gemm_tc_launch(const GemmTcPlan* plan, cudaStream_t s) {
     stalled.params.tx_extra = 16;
     plan = &stalled;
   }
-  cudaError_t launched;
-  const bool extra = plan->params.dz != 0 || plan->params.ep.border_corr != nullptr;
+  const bool extra = plan->params.dz != 0 || plan->params.ep.border_corr != nullptr || plan->params.ep.fix_shl != 0;
   const bool fuse = plan->params.ep.add_residual != nullptr;
-#define B2VX_GEMM_LAUNCH(E_, F_) launch_pdl(gemm_i8_tc_kernel<E_, F_>, dim3(plan->grid), dim3(kThreadsTc), plan->smem, s, plan->map_a, \
-                                            plan->map_b, plan->map_d, plan->params)
-  if (fuse) launched = extra ? B2VX_GEMM_LAUNCH(true, true) : B2VX_GEMM_LAUNCH(false, true);
-  else launched = extra ? B2VX_GEMM_LAUNCH(true, false) : B2VX_GEMM_LAUNCH(false, false);
-#undef B2VX_GEMM_LAUNCH
+  const cudaError_t launched = launch_pdl(kernel_variant(extra, fuse, plan->params.blk_w), dim3(plan->grid), dim3(kThreadsTc), plan->smem, s, plan->map_a, plan->map_b,
+                        plan->map_r, plan->params);
   if (launched != cudaSuccess) return launched;
 #ifdef B2VX_TC_TRACE
   {
@@ -1497,7 +1540,7 @@ cudaError_t gemm_tc_launch(const GemmTcPlan* plan, cudaStream_t s) {
       const long long t0 = h[0];
       const GemmParams& p = plan->params;
       std::fprintf(stderr, "trace: BN %d BK %d group %d stages %d num_kb %d m_tiles %d n_tiles %d grid %d conv %d span %d\n", p.BN, p.BK,
-                   p.group, p.stages, p.num_kb, p.m_tiles, p.n_tiles, plan->grid, p.conv, p.store_span);
+                   p.group, p.stages, p.num_kb, p.m_tiles, p.n_tiles, plan->grid, p.conv, p.blk_w);
       std::fprintf(stderr, "marks: entry %lld  prologue done %lld  all roles done %lld (cycles from first producer wait)\n", h[384] - t0, h[385] - t0, h[386] - t0);
       for (int i = 0; i < 20; ++i)
         std::fprintf(stderr, "it %2d  prodA slot-free %7lld issued %7lld | mma data-in %7lld committed %7lld | epi acc-ready %7lld done %7lld\n",

@@ -29,6 +29,15 @@ struct OutQuant {
   int32_t hi;
 };
 
+// Constants of one output channel for requant_fixed4: the multiplier acc_scale / out.scale in units of 2^(fix_shl - 32);
+// bias, zero point, rounding half and half the window folded into one addend; the window of the column block the channel
+// lies in (results with a smaller fraction are redone exactly).
+struct alignas(16) FixedColumn {
+  long long add;
+  int32_t mul;
+  uint32_t window;
+};
+
 // Geometry of one convolution / pooling window sweep over channels-last data.
 struct ConvGeom {
   int N, H, W, C, Cp;        // input
@@ -49,10 +58,9 @@ struct ContractEpilogue {
   const int32_t* tapc;       // null when the input zero point is 0 or there is no padding
   OutQuant out;
   int out_is_float;          // write float(acc)*acc_scale instead of quantizing
-  // Tensor-core epilogue only: 1 = requantize with the exact sequence only.  The fast form needs
-  // |acc * acc_scale / out.scale| < 2^21 for every possible accumulator, which the planner checks
-  // from K, the bias and the scales.
-  int exact_only;
+  // Tensor-core epilogue, fixed-point requantization (requant_fixed4).  Null: every element takes the exact sequence.
+  const struct FixedColumn* fix;   // [Ocp]
+  int fix_shl;
   // Tensor-core path, weights with one zero point left over (dz_uniform = zw - 128 for uint8 weights):
   // the packed weights carry an all-ones row per N tile, whose accumulator column is S.
   int dz_uniform;
@@ -209,13 +217,17 @@ struct GemmTcPlan;   // opaque: tensor maps + launch geometry, built once at com
 // N tiling of a GEMM: n_tiles tiles of `data` output channels each.  The packed weight matrix has
 // n_tiles * rows rows; inside a tile, rows [0, data) are output channels, and when rows > data row
 // `data` is the all-ones row (S column) and the rest is zero.
+// A tile's channels lie in its data rows in the order gemm_tc_row_of_channel gives: column blocks of blk_w (64, 32 or 16)
+// channels, within a block permuted so that an epilogue thread's accumulator columns are neighbouring channels.
 struct GemmTcTiling {
-  int n_tiles, data, rows;
+  int n_tiles, data, rows, blk_w;
 };
+// Packed row, within its tile, of the tile's channel c.
+int gemm_tc_row_of_channel(const GemmTcTiling& t, int c);
 // Picks the tiling for M x Ocp x Kp from a small cost model (waves of tiles over the SMs, operand
 // bytes per tile, epilogue work per tile).  with_s: reserve 16 rows per tile for the ones row.
 GemmTcTiling gemm_tc_choose_tiling(long long M, int Ocp, int Kp, int with_s);
-// tiling == null: ceil(Np / 256) equal tiles of Np / n_tiles rows, no ones row.
+// tiling == null: ceil(Np / 256) equal tiles of Np / n_tiles rows in channel order, no ones row.
 GemmTcPlan* gemm_tc_plan_create(const void* A, int a_signed, const int8_t* B, int M, int Np, int Kp, int Oc,
                                 void* D, int ldd, int d_signed, const ContractEpilogue& e, int* status,
                                 char* err, size_t err_len, const GemmTcTiling* tiling = nullptr);

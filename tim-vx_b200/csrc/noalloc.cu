@@ -122,9 +122,8 @@ extern "C" b2vx_status b2vx_conv2d_first_layer_noalloc(const b2vx_conv2d_noalloc
   ep.out.zp = d->out_zero_point;
   ep.out.lo = 0;
   ep.out.hi = 255;
-  // The scales are device memory, which this call may not read back to bound |accumulator * scale / out_scale| the
-  // way the graph's planner does; the exact requantization is right for any scales.
-  ep.exact_only = 1;
+  // The scales are device memory, which this call may not read back to derive the fixed-point multipliers of the graph's
+  // planner: the exact requantization runs for every element.
   alignas(64) unsigned char plan_storage[1024];
   if (gemm_tc_plan_bytes() > sizeof(plan_storage)) return fail(err, err_len, B2VX_BAD_STATE, "plan storage too small");
   char why[160] = {0};

@@ -247,6 +247,58 @@ __device__ __forceinline__ uint4 requant_chunk16(const int (&acc)[16], const int
   return make_uint4(wh[0] ^ rc.out_flip, wh[1] ^ rc.out_flip, wh[2] ^ rc.out_flip, wh[3] ^ rc.out_flip);
 }
 
+// Requantization in 64-bit fixed point, the epilogue of the tensor-core kernel.  Per column the host folds accumulator
+// scale / output scale into a multiplier M (units of 2^-32) and bias, zero point and rounding half into an addend, so that
+//     P = acc * M + A          high word = floor(acc * r + bias * r + zp - lo + 1/2 + W),  low word = its fraction,
+// costs one multiply-add per element; the high words go straight into the saturating pack.  W bounds how far P and the
+// reference's float quotient (two or three roundings) can lie apart wherever the output does not saturate.  A fraction
+// of 2 W (the window of the 16 columns) or more says that no half-integer lies between the two: the high word is then
+// the reference's answer, its tie rule included.  The few elements below (2 W is about 1e-4) are redone exactly.
+// Per element: one multiply-add (2.65 cycles of an SM scheduler measured, 2 for most other integer instructions), half a
+// pack, half a three-input minimum.  The form with two packed float products that it replaced took an addition, an
+// int-to-float conversion, 1.5 packed float operations, two subtractions and a whole pack.
+struct FixedColumns {                // one N tile, in the order the epilogue threads read it
+  alignas(16) int mul[256];
+  alignas(16) long long add[256];
+  alignas(16) int bias[256];         // for the exact sequence: folded bias and accumulator scale
+  alignas(16) float scale[256];
+  uint32_t window[16];               // per 16 columns
+};
+
+// The exact sequence for those of four columns whose fraction lies in the window.  Not inlined: it is rare,
+// and sixteen copies of it cost the common path registers and instruction cache.
+static __device__ __noinline__ uint32_t requant_redo4(uint32_t word, int a0, int a1, int a2, int a3, const FixedColumns* cols, int c, uint32_t window,
+                                               int shl, OutQuant oq) {
+  const int acc[4] = {a0, a1, a2, a3};
+  const int4 m = *reinterpret_cast<const int4*>(&cols->mul[c]), b = *reinterpret_cast<const int4*>(&cols->bias[c]);
+  const float4 sc = *reinterpret_cast<const float4*>(&cols->scale[c]);
+  const longlong2 a01 = *reinterpret_cast<const longlong2*>(&cols->add[c]), a23 = *reinterpret_cast<const longlong2*>(&cols->add[c + 2]);
+  const int mul[4] = {m.x, m.y, m.z, m.w}, bias[4] = {b.x, b.y, b.z, b.w};
+  const float scale[4] = {sc.x, sc.y, sc.z, sc.w};
+  const long long add[4] = {a01.x, a01.y, a23.x, a23.y};
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    const uint32_t f = (static_cast<uint32_t>(acc[k]) << shl) * static_cast<uint32_t>(mul[k]) + static_cast<uint32_t>(add[k]);
+    if (f >= window) continue;
+    const float real = __fmul_rn(__int2float_rn(acc[k] + bias[k]), scale[k]);
+    const uint32_t q = static_cast<uint32_t>(requant(real, oq) - oq.lo) & 0xFFu;
+    word = (word & ~(0xFFu << (8 * k))) | (q << (8 * k));
+  }
+  return word;
+}
+
+// Four neighbouring columns of one row (x[0..3] with columns c .. c + 3; m, a01, a23: their constants, loaded once for
+// several rows) to four bytes q - lo; `low` receives the smallest fraction.  The caller tests it, once for several rows:
+// a branch after every four elements kept the scheduler from overlapping their multiply-adds.
+__device__ __forceinline__ uint32_t requant_fixed4(const int (&x)[4], const int4& m, const longlong2& a01, const longlong2& a23, int shl,
+                                                   uint32_t& low) {
+  const long long p0 = static_cast<long long>(x[0] << shl) * m.x + a01.x, p1 = static_cast<long long>(x[1] << shl) * m.y + a01.y;
+  const long long p2 = static_cast<long long>(x[2] << shl) * m.z + a23.x, p3 = static_cast<long long>(x[3] << shl) * m.w + a23.y;
+  low = min(__vimin3_u32(static_cast<uint32_t>(p0), static_cast<uint32_t>(p1), static_cast<uint32_t>(p2)), static_cast<uint32_t>(p3));
+  return pack_sat_u8(static_cast<int>(p1 >> 32), static_cast<int>(p0 >> 32),
+                     pack_sat_u8(static_cast<int>(p3 >> 32), static_cast<int>(p2 >> 32), 0u));
+}
+
 // Quantized Add of four byte pairs through the 64 KB table (entry (a, b) at a*256 + (b ^ ((a & 31) << 2)),
 // which spreads pairs that share b over the shared-memory banks): build the indices, four byte loads, pack.
 __device__ __forceinline__ uint32_t add_lut_word(uint32_t aw, uint32_t bw, const uint8_t* tab) {
