@@ -1,0 +1,44 @@
+"""Inputs and outputs on both sides of the sizes at which they go through the graph's page-locked memory, written and read
+in every order a caller may use."""
+import numpy as np
+import pytest
+
+import pyb2vx as B
+
+pytestmark = pytest.mark.gpu
+
+
+def relu(lib, dims):
+    g = B.Graph(lib, 0)
+    x = g.tensor(B.DT_UINT8, dims, B.ATTR_INPUT, scale=0.1, zero_point=10)
+    y = g.tensor(B.DT_UINT8, dims, B.ATTR_OUTPUT, scale=0.1, zero_point=10)
+    g.relu(x, y)
+    g.compile()
+    return g, x, y
+
+
+# [W, H, C, N]: layouts that coincide and that do not; rows without pixels; tiny, small and large
+SHAPES = [(1, 1, 5, 1), (1, 1, 16, 3), (1, 1, 1000, 7), (1, 1, 1001, 64), (1, 1, 1008, 64), (3, 3, 10, 2), (56, 56, 3, 1), (64, 64, 64, 1), (65, 64, 64, 1),
+          (1, 1, 1000, 262), (1, 1, 1000, 263)]
+
+
+@pytest.mark.parametrize("dims", SHAPES)
+def test_round_trip(product_lib, dims):
+    rng = np.random.default_rng(3)
+    g, x, y = relu(product_lib, list(dims))
+    a, b = (rng.integers(0, 256, size=dims[::-1]).astype(np.uint8) for _ in range(2))
+    want = lambda v: np.maximum(v, 10)
+    g.write(x, a)
+    g.run()
+    np.testing.assert_array_equal(g.read(y), want(a))
+    np.testing.assert_array_equal(g.read(x), a)
+    g.write(x, b)
+    np.testing.assert_array_equal(g.read(y), want(a))   # not run yet
+    g.run_async()
+    g.write(x, a)                                       # waits for the run that reads b
+    np.testing.assert_array_equal(g.read(y), want(b))
+    g.run_async()
+    np.testing.assert_array_equal(g.read(y), want(a))
+    g.profile(2)
+    np.testing.assert_array_equal(g.read(y), want(a))
+    g.close()

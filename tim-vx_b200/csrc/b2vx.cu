@@ -62,6 +62,10 @@ struct TensorRec {
   size_t cl_bytes = 0, io_bytes = 0;
   bool is_activation = false;
   bool cl_used = false;        // some kernel reads the channels-last copy (decides whether a graph input is converted)
+  // Small inputs and outputs go through page-locked memory of the graph (see kStagedBytes): the caller's bytes of an
+  // input, or the result of an output as of the last run.  d_io may point here too.
+  uint8_t* h_in = nullptr;
+  uint8_t* h_out = nullptr;
   bool io_direct = false;      // a graph output whose producer writes the WHCN copy itself (no conversion at the end)
 
   size_t elems() const {
@@ -114,13 +118,16 @@ struct b2vx_graph {
   std::vector<NodeRec> nodes;
   std::vector<uint32_t> order;
   std::vector<Step> steps;
+  // transfers of small inputs and outputs before and after the steps of a run (kStagedBytes)
+  std::vector<std::function<cudaError_t(cudaStream_t)>> copies_in, copies_out;
   std::vector<void*> allocs;
   std::vector<GemmTcPlan*> gemm_plans;
   std::vector<std::function<b2vx_status()>> finalizers;   // run once device scratch exists
   void* scratch = nullptr;
   size_t scratch_bytes = 0;
-  int* d_status = nullptr;
-  int* h_status = nullptr;
+  int* status = nullptr;       // page-locked: kernels that gave up on a barrier store a code here
+  uint8_t* h_staging = nullptr;
+  bool idle = true;            // nothing queued since the stream was last waited for
   bool compiled = false;
   bool use_tc = false;
   bool fuse_add = true;      // residual Add into the preceding convolution's epilogue (B2VX_FUSE_ADD=0 disables)
@@ -197,6 +204,22 @@ b2vx_status upload(b2vx_graph* g, const std::vector<T>& v, T** out) {
   if (!v.empty()) CUDA_TRY(g, cudaMemcpy(p, v.data(), v.size() * sizeof(T), cudaMemcpyHostToDevice));
   *out = static_cast<T*>(p);
   return B2VX_OK;
+}
+
+// Inputs and outputs of up to this many bytes are not copied by the copy engine: a write is a memcpy into page-locked
+// memory, which a copy kernel at the head of the run reads over the bus, and the last kernel of a run leaves the output in
+// page-locked memory, where a read finds it (in 16-byte pieces: 64 x 1000 results as single bytes took 117 us).  A copy call of its own costs 8 - 13 us from call to
+// return whatever its size; at 50 GB/s over the bus and about 15 GB/s for the memcpy, 256 KB costs about as much.
+constexpr size_t kStagedBytes = 256 * 1024;
+// Inputs this small are read over the bus by the kernels themselves, without a copy on the device.
+constexpr size_t kTinyBytes = 4096;
+
+// Waits for everything of this graph that is queued on its stream.
+cudaError_t wait_idle(b2vx_graph* g) {
+  if (g->idle) return cudaSuccess;
+  const cudaError_t e = cudaStreamSynchronize(g->stream);
+  if (e == cudaSuccess) g->idle = true;
+  return e;
 }
 
 // ---------------------------------------------------------------- shapes
@@ -979,10 +1002,10 @@ b2vx_status plan_contraction(b2vx_graph* g, uint32_t node_index, const char* lab
       char err[160] = {0};
       GemmTcPlan* pl;
       if (implicit) {
-        pl = gemm_tc_conv_plan_create(A, x_signed, dw8, geo, Np, ycl, ep, g->d_status, err, sizeof(err), &tiling);
+        pl = gemm_tc_conv_plan_create(A, x_signed, dw8, geo, Np, ycl, ep, g->status, err, sizeof(err), &tiling);
       } else {
         const void* Aptr = need_im2col ? g->scratch : A;
-        pl = gemm_tc_plan_create(Aptr, x_signed, dw8, M, Np, Kp, Oc, ycl, ldd, y_signed, ep, g->d_status, err, sizeof(err), &tiling);
+        pl = gemm_tc_plan_create(Aptr, x_signed, dw8, M, Np, Kp, Oc, ycl, ldd, y_signed, ep, g->status, err, sizeof(err), &tiling);
       }
       if (!pl) return fail(g, B2VX_UNSUPPORTED, lbl + ": " + err);
       g->gemm_plans.push_back(pl);
@@ -1605,14 +1628,12 @@ b2vx_status b2vx_graph_create(b2vx_context* ctx, int32_t device_id, b2vx_graph**
   g->device = device_id;
   DeviceGuard guard(device_id);
   if (cudaStreamCreateWithFlags(&g->own_stream, cudaStreamNonBlocking) != cudaSuccess ||
-      cudaMalloc(reinterpret_cast<void**>(&g->d_status), sizeof(int)) != cudaSuccess ||
-      cudaMemset(g->d_status, 0, sizeof(int)) != cudaSuccess ||
-      cudaHostAlloc(reinterpret_cast<void**>(&g->h_status), sizeof(int), cudaHostAllocDefault) != cudaSuccess) {
+      cudaHostAlloc(reinterpret_cast<void**>(&g->status), sizeof(int), cudaHostAllocDefault) != cudaSuccess) {
     ctx->err = std::string("graph_create: ") + cudaGetErrorString(cudaGetLastError());
     delete g;
     return B2VX_CUDA_ERROR;
   }
-  *g->h_status = 0;
+  *g->status = 0;
   g->stream = g->own_stream;
   const char* k = std::getenv("B2VX_CONV_KERNEL");
   g->use_tc = gemm_tc_available() && !(k && std::strcmp(k, "simt") == 0);
@@ -1635,8 +1656,8 @@ void b2vx_graph_destroy(b2vx_graph* g) {
   if (g->exec) cudaGraphExecDestroy(g->exec);
   for (GemmTcPlan* p : g->gemm_plans) gemm_tc_plan_destroy(p);
   for (void* p : g->allocs) cudaFree(p);
-  if (g->d_status) cudaFree(g->d_status);
-  if (g->h_status) cudaFreeHost(g->h_status);
+  if (g->status) cudaFreeHost(g->status);
+  if (g->h_staging) cudaFreeHost(g->h_staging);
   if (g->own_stream) cudaStreamDestroy(g->own_stream);
   delete g;
 }
@@ -1697,9 +1718,18 @@ b2vx_status b2vx_tensor_write(b2vx_graph* g, uint32_t id, const void* src, size_
   }
   if (t.d.attr & B2VX_ATTR_CONSTANT) return fail(g, B2VX_BAD_STATE, "tensor_write: constants are frozen at compile");
   if (!t.d_io) return fail(g, B2VX_BAD_STATE, "tensor_write: tensor has no device storage");
+  if (t.h_in) {
+    if (!g->idle) {   // a queued run may still read the previous bytes
+      DeviceGuard guard(g->device);
+      CUDA_TRY(g, wait_idle(g));
+    }
+    std::memcpy(t.h_in, src, bytes);
+    return B2VX_OK;
+  }
   DeviceGuard guard(g->device);
+  g->idle = false;
   CUDA_TRY(g, cudaMemcpyAsync(t.d_io, src, bytes, cudaMemcpyHostToDevice, g->stream));
-  CUDA_TRY(g, cudaStreamSynchronize(g->stream));
+  CUDA_TRY(g, wait_idle(g));
   return B2VX_OK;
 }
 
@@ -1717,10 +1747,19 @@ b2vx_status b2vx_tensor_read(b2vx_graph* g, uint32_t id, void* dst, size_t bytes
     std::memcpy(dst, t.host.data(), bytes);
     return B2VX_OK;
   }
+  if (t.h_in || t.h_out) {
+    if (!g->idle) {
+      DeviceGuard guard(g->device);
+      CUDA_TRY(g, wait_idle(g));
+    }
+    std::memcpy(dst, t.h_in ? t.h_in : t.h_out, bytes);
+    return B2VX_OK;
+  }
   DeviceGuard guard(g->device);
   if (t.d_io) {
+    g->idle = false;
     CUDA_TRY(g, cudaMemcpyAsync(dst, t.d_io, bytes, cudaMemcpyDeviceToHost, g->stream));
-    CUDA_TRY(g, cudaStreamSynchronize(g->stream));
+    CUDA_TRY(g, wait_idle(g));
     return B2VX_OK;
   }
   // intermediate tensor: convert on the fly (debugging / per-layer checks)
@@ -1728,7 +1767,8 @@ b2vx_status b2vx_tensor_read(b2vx_graph* g, uint32_t id, void* dst, size_t bytes
   CUDA_TRY(g, cudaMalloc(&tmp, bytes));
   launch_cl_to_whcn(t.d_cl, tmp, t.N, t.C, t.H, t.W, t.Cp, static_cast<int>(dtype_size(t.d.dtype)), g->stream);
   cudaError_t e = cudaMemcpyAsync(dst, tmp, bytes, cudaMemcpyDeviceToHost, g->stream);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(g->stream);
+  g->idle = false;
+  if (e == cudaSuccess) e = wait_idle(g);
   cudaFree(tmp);
   if (e != cudaSuccess) return fail(g, B2VX_CUDA_ERROR, std::string("tensor_read: ") + cudaGetErrorString(e));
   return B2VX_OK;
@@ -1973,10 +2013,20 @@ b2vx_status b2vx_graph_compile(b2vx_graph* g) {
              (g->tensors[n.in[0]].d.dtype == B2VX_DT_INT32 || g->tensors[n.out].d.dtype == B2VX_DT_INT32))
       return fail(g, B2VX_UNSUPPORTED, "int32 activations are supported by Add, Reshape, Transpose and Concat only");
   }
-  for (TensorRec& t : g->tensors) {
+  std::vector<char> written(g->tensors.size(), 0);
+  for (const NodeRec& n : g->nodes)
+    if (!n.removed) written[n.out] = 1;
+  size_t staging = 0;   // page-locked bytes of the small inputs and outputs
+  auto stage_slot = [&](const TensorRec& t) { const size_t at = staging; staging += (t.io_bytes + 255) & ~static_cast<size_t>(255); return at; };
+  std::vector<std::pair<size_t, size_t>> staged;   // tensor, offset
+  for (size_t ti = 0; ti < g->tensors.size(); ++ti) {
+    TensorRec& t = g->tensors[ti];
     if (!t.is_activation) continue;
     if (!t.has_shape) return fail(g, B2VX_SHAPE_MISMATCH, "an activation tensor has no shape");
     map_dims(t);
+    const int kind = t.d.attr & (B2VX_ATTR_INPUT | B2VX_ATTR_OUTPUT | B2VX_ATTR_VARIABLE | B2VX_ATTR_CONSTANT);
+    if (t.io_bytes <= kStagedBytes && ((kind == B2VX_ATTR_INPUT && !written[ti]) || (kind == B2VX_ATTR_OUTPUT && written[ti])))
+      staged.emplace_back(ti, stage_slot(t));
     b2vx_status st = dev_alloc(g, &t.d_cl, t.cl_bytes);
     if (st != B2VX_OK) return st;
     CUDA_TRY(g, cudaMemsetAsync(t.d_cl, 0, t.cl_bytes, g->stream));
@@ -1987,6 +2037,17 @@ b2vx_status b2vx_graph_compile(b2vx_graph* g) {
         st = dev_alloc(g, &t.d_io, t.io_bytes);
         if (st != B2VX_OK) return st;
       }
+    }
+  }
+
+  if (staging) {
+    CUDA_TRY(g, cudaHostAlloc(reinterpret_cast<void**>(&g->h_staging), staging, cudaHostAllocDefault));
+    std::memset(g->h_staging, 0, staging);
+    for (const auto& s : staged) {
+      TensorRec& t = g->tensors[s.first];
+      (t.d.attr & B2VX_ATTR_INPUT ? t.h_in : t.h_out) = g->h_staging + s.second;
+      // tiny ones are read and written over the bus by the graph's own kernels
+      if (t.d_io != t.d_cl && t.io_bytes <= kTinyBytes) t.d_io = g->h_staging + s.second;
     }
   }
 
@@ -2025,6 +2086,12 @@ b2vx_status b2vx_graph_compile(b2vx_graph* g) {
     std::vector<Step> head;
     for (size_t i = 0; i < g->tensors.size(); ++i) {
       TensorRec& t = g->tensors[i];
+      if (t.is_activation && t.h_in && t.d_io != t.h_in) {
+        const void* from = t.h_in;
+        void* to = t.d_io;
+        const size_t n16 = (t.io_bytes + 15) / 16;
+        g->copies_in.push_back([=](cudaStream_t st2) { launch_copy16(from, to, n16, st2); return cudaGetLastError(); });
+      }
       if (!t.is_activation || !t.cl_used || !(t.d.attr & (B2VX_ATTR_INPUT | B2VX_ATTR_VARIABLE))) continue;
       if (t.d_io == t.d_cl) continue;
       const void* src = t.d_io;
@@ -2040,14 +2107,25 @@ b2vx_status b2vx_graph_compile(b2vx_graph* g) {
   for (size_t i = 0; i < g->tensors.size(); ++i) {
     TensorRec& t = g->tensors[i];
     if (!t.is_activation || !(t.d.attr & B2VX_ATTR_OUTPUT)) continue;
-    if (t.d_io == t.d_cl || t.io_direct) continue;
-    const void* src = t.d_cl;
-    void* dst = t.d_io;
-    const int N = t.N, C = t.C, H = t.H, W = t.W, Cp = t.Cp, el = static_cast<int>(dtype_size(t.d.dtype));
-    Step s;
-    s.info = make_info("cl_to_whcn", B2VX_NO_TENSOR, 0, t.io_bytes + t.cl_bytes);
-    s.fn = [=](cudaStream_t st2) { launch_cl_to_whcn(src, dst, N, C, H, W, Cp, el, st2); return cudaGetLastError(); };
-    g->steps.push_back(std::move(s));
+    if (t.d_io != t.d_cl && !t.io_direct) {
+      const void* src = t.d_cl;
+      // one pixel per image: the rows lose their padding on the way to the host
+      const bool rows = t.h_out != nullptr && t.H * t.W == 1;
+      void* dst = rows ? t.h_out : t.d_io;
+      const int N = t.N, C = t.C, H = t.H, W = t.W, Cp = t.Cp, el = static_cast<int>(dtype_size(t.d.dtype));
+      Step s;
+      s.info = make_info("cl_to_whcn", B2VX_NO_TENSOR, 0, t.io_bytes + t.cl_bytes);
+      if (rows) s.fn = [=](cudaStream_t st2) { launch_pack_rows16(src, dst, N, C * el, Cp * el, st2); return cudaGetLastError(); };
+      else s.fn = [=](cudaStream_t st2) { launch_cl_to_whcn(src, dst, N, C, H, W, Cp, el, st2); return cudaGetLastError(); };
+      g->steps.push_back(std::move(s));
+      if (rows) continue;
+    }
+    if (t.h_out && t.d_io != t.h_out) {
+      const void* from = t.d_io;
+      void* to = t.h_out;
+      const size_t n16 = (t.io_bytes + 15) / 16;
+      g->copies_out.push_back([=](cudaStream_t st2) { launch_copy16(from, to, n16, st2); return cudaGetLastError(); });
+    }
   }
   if (g->scratch_bytes) {
     b2vx_status st = dev_alloc(g, &g->scratch, g->scratch_bytes);
@@ -2062,6 +2140,10 @@ b2vx_status b2vx_graph_compile(b2vx_graph* g) {
   // 4. data that was supplied before compile: inputs written early, constant activations
   for (TensorRec& t : g->tensors) {
     if (!t.is_activation || !t.host_valid || !t.d_io) continue;
+    if (t.h_in) {
+      std::memcpy(t.h_in, t.host.data(), t.io_bytes);
+      continue;
+    }
     CUDA_TRY(g, cudaMemcpyAsync(t.d_io, t.host.data(), t.io_bytes, cudaMemcpyHostToDevice, g->stream));
     if ((t.d.attr & B2VX_ATTR_CONSTANT) && t.d_io != t.d_cl)
       launch_whcn_to_cl(t.d_io, t.d_cl, t.N, t.C, t.H, t.W, t.Cp, static_cast<int>(dtype_size(t.d.dtype)), g->stream);
@@ -2077,12 +2159,15 @@ b2vx_status b2vx_graph_run_async(b2vx_graph* g) {
   b2vx_status st = b2vx_graph_compile(g);
   if (st != B2VX_OK) return st;
   DeviceGuard guard(g->device);
+  g->idle = false;
   if (g->use_cuda_graph && !g->exec && !g->capture_failed && !g->steps.empty()) {
     // Record the plan once; on any failure fall back to launching kernel by kernel.
     cudaGraph_t graph = nullptr;
     bool ok = cudaStreamBeginCapture(g->stream, cudaStreamCaptureModeThreadLocal) == cudaSuccess;
     if (ok) {
+      for (auto& copy : g->copies_in) ok = ok && copy(g->stream) == cudaSuccess;
       for (Step& s : g->steps) ok = ok && s.fn(g->stream) == cudaSuccess;
+      for (auto& copy : g->copies_out) ok = ok && copy(g->stream) == cudaSuccess;
       ok = (cudaStreamEndCapture(g->stream, &graph) == cudaSuccess) && ok && graph != nullptr;
     }
     if (ok) ok = cudaGraphInstantiate(&g->exec, graph, 0) == cudaSuccess;
@@ -2098,23 +2183,25 @@ b2vx_status b2vx_graph_run_async(b2vx_graph* g) {
     if (e != cudaSuccess) return fail(g, B2VX_CUDA_ERROR, std::string("cudaGraphLaunch: ") + cudaGetErrorString(e));
     return B2VX_OK;
   }
+  for (auto& copy : g->copies_in) CUDA_TRY(g, copy(g->stream));
   for (Step& s : g->steps) {
     cudaError_t e = s.fn(g->stream);
     if (e != cudaSuccess) {
       return fail(g, B2VX_CUDA_ERROR, std::string(s.info.name) + ": " + cudaGetErrorString(e));
     }
   }
+  for (auto& copy : g->copies_out) CUDA_TRY(g, copy(g->stream));
   return B2VX_OK;
 }
 
 b2vx_status b2vx_graph_sync(b2vx_graph* g) {
   if (!g) return B2VX_INVALID_ARG;
   DeviceGuard guard(g->device);
-  CUDA_TRY(g, cudaMemcpyAsync(g->h_status, g->d_status, sizeof(int), cudaMemcpyDeviceToHost, g->stream));
-  CUDA_TRY(g, cudaStreamSynchronize(g->stream));
-  if (*g->h_status != 0) {
-    const int code = *g->h_status;
-    cudaMemsetAsync(g->d_status, 0, sizeof(int), g->stream);
+  g->idle = false;   // the caller may have queued work of its own on this stream
+  CUDA_TRY(g, wait_idle(g));
+  if (*static_cast<volatile int*>(g->status) != 0) {
+    const int code = *g->status;
+    *g->status = 0;
     return fail(g, B2VX_DEVICE_TIMEOUT, "a tensor-core kernel gave up waiting on a barrier (code " + std::to_string(code) + ")");
   }
   return B2VX_OK;
@@ -2130,6 +2217,7 @@ b2vx_status b2vx_graph_set_stream(b2vx_graph* g, void* cuda_stream) {
   if (!g) return B2VX_INVALID_ARG;
   DeviceGuard guard(g->device);
   cudaStreamSynchronize(g->stream);
+  g->idle = true;
   g->stream = cuda_stream ? static_cast<cudaStream_t>(cuda_stream) : g->own_stream;
   return B2VX_OK;
 }
@@ -2192,6 +2280,7 @@ b2vx_status b2vx_graph_profile(b2vx_graph* g, uint32_t iters) {
     }
   }
   for (uint32_t it = 0; it < iters; ++it) {
+    g->idle = false;
     if (exec) {
       CUDA_TRY(g, cudaGraphLaunch(exec, g->stream));
     } else {

@@ -35,6 +35,36 @@ __device__ __forceinline__ void transpose4x4(uint32_t (&r)[4]) {
   r[3] = __byte_perm(t1, t3, 0x7632);
 }
 
+// Small inputs and outputs between page-locked host memory and the device: one 16-byte piece per thread, so that all of
+// them cross the bus at once.
+__global__ void __launch_bounds__(128) copy16_kernel(const uint4* __restrict__ src, uint4* __restrict__ dst, size_t n16) {
+  pdl_trigger();
+  pdl_wait();
+  const size_t i = blockIdx.x * static_cast<size_t>(128) + threadIdx.x;
+  if (i < n16) dst[i] = src[i];
+}
+
+// Dense rows out of padded ones, 16 bytes of the result per thread: the bus takes them in few writes.
+__global__ void __launch_bounds__(128) pack_rows16_kernel(const uint8_t* __restrict__ src, uint4* __restrict__ dst, int rows, int row_bytes, int pitch) {
+  pdl_trigger();
+  pdl_wait();
+  const int i = blockIdx.x * 128 + threadIdx.x, total = rows * row_bytes;
+  if (16 * i >= total) return;
+  int r = 16 * i / row_bytes, o = 16 * i - r * row_bytes;
+  const uint8_t* at = src + static_cast<size_t>(r) * pitch + o;
+  uint32_t v[4] = {0, 0, 0, 0};
+#pragma unroll
+  for (int k = 0; k < 16; ++k) {
+    if (16 * i + k < total) v[k >> 2] |= static_cast<uint32_t>(*at) << (8 * (k & 3));
+    ++at;
+    if (++o == row_bytes) {
+      o = 0;
+      at += pitch - row_bytes;
+    }
+  }
+  dst[i] = make_uint4(v[0], v[1], v[2], v[3]);
+}
+
 template <bool ALIGNED>
 __global__ void __launch_bounds__(256) whcn_to_cl_u8_kernel(const uint8_t* __restrict__ src, uint8_t* __restrict__ dst, int C,
                                                             int HW, int Cp) {
@@ -1837,6 +1867,17 @@ __global__ void __launch_bounds__(256, 2) fc_small_m_kernel(const uint8_t* __res
 }  // namespace
 
 // ---------------------------------------------------------------- wrappers
+
+void launch_copy16(const void* src, void* dst, size_t n16, cudaStream_t s) {
+  if (n16 == 0) return;
+  launch_pdl(copy16_kernel, dim3(static_cast<unsigned>((n16 + 127) / 128)), dim3(128), 0, s, static_cast<const uint4*>(src), static_cast<uint4*>(dst), n16);
+}
+
+void launch_pack_rows16(const void* src, void* dst, int rows, int row_bytes, int pitch, cudaStream_t s) {
+  const int n16 = (rows * row_bytes + 15) / 16;
+  if (n16 == 0) return;
+  launch_pdl(pack_rows16_kernel, dim3((n16 + 127) / 128), dim3(128), 0, s, static_cast<const uint8_t*>(src), static_cast<uint4*>(dst), rows, row_bytes, pitch);
+}
 
 void launch_whcn_to_cl(const void* src, void* dst, int N, int C, int H, int W, int Cp, int elem, cudaStream_t s) {
   const int HW = H * W;

@@ -144,6 +144,8 @@ class Graph:
             self.ctx = None
             raise B2vxError(st, msg)
         self._keep = []
+        self._layout = {}        # tensor id -> (bytes, numpy type, numpy shape), once the graph is compiled
+        self._compiled = False
 
     def close(self):
         if self.g:
@@ -257,9 +259,11 @@ class Graph:
 
     def compile(self):
         self._check(self.lib.b2vx_graph_compile(self.g))
+        self._compiled = True
 
     def run(self):
         self._check(self.lib.b2vx_graph_run(self.g))
+        self._compiled = True
 
     def run_async(self):
         self._check(self.lib.b2vx_graph_run_async(self.g))
@@ -279,22 +283,32 @@ class Graph:
         d = self.desc(tid)
         return [int(d.dims[i]) for i in range(d.rank)]
 
+    def _layout_of(self, tid):
+        """(bytes, numpy type, numpy shape) of a tensor; fixed once the graph is compiled."""
+        l = self._layout.get(tid)
+        if l is None:
+            d = self.desc(tid)
+            dims = tuple(int(d.dims[i]) for i in range(d.rank))[::-1]
+            dtype = np.dtype(NP_DTYPE[d.dtype])
+            l = (int(np.prod(dims, dtype=np.int64)) * dtype.itemsize, dtype, dims)
+            if self._compiled:
+                self._layout[tid] = l
+        return l
+
     def write(self, tid, array):
-        d = self.desc(tid)
-        a = np.ascontiguousarray(array, dtype=NP_DTYPE[d.dtype])
-        self._check(self.lib.b2vx_tensor_write(self.g, tid, a.ctypes.data_as(C.c_void_p), a.nbytes))
+        a = np.ascontiguousarray(array, dtype=self._layout_of(tid)[1])
+        self._check(self.lib.b2vx_tensor_write(self.g, tid, a.ctypes.data, a.nbytes))
 
     def write_ptr(self, tid, ptr, nbytes):
-        self._check(self.lib.b2vx_tensor_write(self.g, tid, C.c_void_p(ptr), nbytes))
+        self._check(self.lib.b2vx_tensor_write(self.g, tid, ptr, nbytes))
 
     def read_ptr(self, tid, ptr, nbytes):
-        self._check(self.lib.b2vx_tensor_read(self.g, tid, C.c_void_p(ptr), nbytes))
+        self._check(self.lib.b2vx_tensor_read(self.g, tid, ptr, nbytes))
 
     def read(self, tid):
-        d = self.desc(tid)
-        dims = [int(d.dims[i]) for i in range(d.rank)]
-        out = np.empty(dims[::-1], dtype=NP_DTYPE[d.dtype])
-        self._check(self.lib.b2vx_tensor_read(self.g, tid, out.ctypes.data_as(C.c_void_p), out.nbytes))
+        nbytes, dtype, dims = self._layout_of(tid)
+        out = np.empty(dims, dtype=dtype)
+        self._check(self.lib.b2vx_tensor_read(self.g, tid, out.ctypes.data, nbytes))
         return out
 
     def kernels(self):
