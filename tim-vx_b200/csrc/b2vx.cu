@@ -531,6 +531,7 @@ bool fixed_point_columns(const PackedContraction& pk, const OutQuant& out, doubl
                          int* shl) {
   const size_t n = pk.acc_scale.size();
   const double two32 = 4294967296.0;
+  if (!(out.scale > 5.5e-20f && out.scale < 1.8e19f)) return false;   // requant_near_half
   std::vector<double> r(n);   // acc_scale / out scale in units of 2^-32
   double r_max = 0.0;
   for (size_t c = 0; c < n; ++c) {

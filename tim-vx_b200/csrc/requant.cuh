@@ -257,6 +257,8 @@ __device__ __forceinline__ uint4 requant_chunk16(const int (&acc)[16], const int
 // Per element: one multiply-add (2.65 cycles of an SM scheduler measured, 2 for most other integer instructions), half a
 // pack, half a three-input minimum.  The form with two packed float products that it replaced took an addition, an
 // int-to-float conversion, 1.5 packed float operations, two subtractions and a whole pack.
+__device__ __forceinline__ long long mad_wide(int a, int b, long long c) { return static_cast<long long>(a) * b + c; }
+
 struct FixedColumns {                // one N tile, in the order the epilogue threads read it
   alignas(16) int mul[256];
   alignas(16) long long add[256];
@@ -265,23 +267,49 @@ struct FixedColumns {                // one N tile, in the order the epilogue th
   uint32_t window[16];               // per 16 columns
 };
 
-// The exact sequence for those of four columns whose fraction lies in the window.  Not inlined: it is rare,
-// and sixteen copies of it cost the common path registers and instruction cache.
+static __device__ __noinline__ uint32_t requant_replay(float real, float scale, int zp, int lo, int hi) {
+  const OutQuant oq = {scale, zp, lo, hi};
+  return static_cast<uint32_t>(requant(real, oq) - lo) & 0xFFu;
+}
+
+// The reference's answer (as q - lo) where requant_fixed4 left it between hi and hi - 1.  With n the integer above the
+// half b = n - 1/2 in question, the reference compares x = real / scale, rounded, with b.  e = real - b * scale is exact
+// in one fused operation (both lie within 2^-9 scale of each other, on a grid of 2^-24 scale or coarser), and x rounds
+// to b itself exactly when |e| is at most half an ulp of b times the scale; then the even neighbour wins.  Next to 1/2,
+// where x + 0.5f rounds too, the sequence is replayed.  About a dozen instructions instead of the division's hundred:
+// one thread in a warp of a short-K layer takes this path every few blocks, and the other threads wait for it.
+// out.scale between 2^-64 and 2^64 (checked when the constants are made), 0 < hi < 256.
+__device__ __forceinline__ uint32_t requant_near_half(float real, int hi, const OutQuant& oq) {
+  const int n = hi + oq.lo - oq.zp;
+  const float b = __fmul_rn(__int2float_rn(2 * n - 1), 0.5f), ab = fabsf(b);
+  if (ab == 0.5f) return requant_replay(real, oq.scale, oq.zp, oq.lo, oq.hi);
+  const float e = __fmaf_rn(-b, oq.scale, real);
+  const float half_ulp = __fmul_rn(oq.scale, __int_as_float((__float_as_int(ab) & 0x7F800000) - (24 << 23)));
+  const bool down = fabsf(e) <= half_ulp ? (n & 1) : e < 0.0f;
+  return static_cast<uint32_t>(hi - (down ? 1 : 0));
+}
+
+// Those of four columns whose fraction lies in the window, unless the integers on both sides saturate to the same result.
+// Not inlined: sixteen copies of it cost the common path registers and instruction cache.
 static __device__ __noinline__ uint32_t requant_redo4(uint32_t word, int a0, int a1, int a2, int a3, const FixedColumns* cols, int c, uint32_t window,
                                                int shl, OutQuant oq) {
-  const int acc[4] = {a0, a1, a2, a3};
-  const int4 m = *reinterpret_cast<const int4*>(&cols->mul[c]), b = *reinterpret_cast<const int4*>(&cols->bias[c]);
-  const float4 sc = *reinterpret_cast<const float4*>(&cols->scale[c]);
+  const int4 m = *reinterpret_cast<const int4*>(&cols->mul[c]);
   const longlong2 a01 = *reinterpret_cast<const longlong2*>(&cols->add[c]), a23 = *reinterpret_cast<const longlong2*>(&cols->add[c + 2]);
-  const int mul[4] = {m.x, m.y, m.z, m.w}, bias[4] = {b.x, b.y, b.z, b.w};
-  const float scale[4] = {sc.x, sc.y, sc.z, sc.w};
-  const long long add[4] = {a01.x, a01.y, a23.x, a23.y};
-#pragma unroll
-  for (int k = 0; k < 4; ++k) {
-    const uint32_t f = (static_cast<uint32_t>(acc[k]) << shl) * static_cast<uint32_t>(mul[k]) + static_cast<uint32_t>(add[k]);
-    if (f >= window) continue;
-    const float real = __fmul_rn(__int2float_rn(acc[k] + bias[k]), scale[k]);
-    const uint32_t q = static_cast<uint32_t>(requant(real, oq) - oq.lo) & 0xFFu;
+  const long long v0 = mad_wide(a0 << shl, m.x, a01.x), v1 = mad_wide(a1 << shl, m.y, a01.y);
+  const long long v2 = mad_wide(a2 << shl, m.z, a23.x), v3 = mad_wide(a3 << shl, m.w, a23.y);
+  uint32_t hits = (static_cast<uint32_t>(v0) < window ? 1u : 0u) | (static_cast<uint32_t>(v1) < window ? 2u : 0u) |
+                  (static_cast<uint32_t>(v2) < window ? 4u : 0u) | (static_cast<uint32_t>(v3) < window ? 8u : 0u);
+#pragma unroll 1
+  while (hits) {   // seldom more than one
+    const int k = __ffs(hits) - 1;
+    hits &= hits - 1;
+    const int acc = k & 2 ? (k & 1 ? a3 : a2) : (k & 1 ? a1 : a0);
+    const int hi = static_cast<int>((k & 2 ? (k & 1 ? v3 : v2) : (k & 1 ? v1 : v0)) >> 32);
+    const float real = __fmul_rn(__int2float_rn(acc + cols->bias[c + k]), cols->scale[c + k]);
+    uint32_t q;
+    if (window == 0xFFFFFFFFu) q = requant_replay(real, oq.scale, oq.zp, oq.lo, oq.hi);   // no fixed-point constants
+    else if (static_cast<uint32_t>(hi - 1) < 255u) q = requant_near_half(real, hi, oq);
+    else continue;
     word = (word & ~(0xFFu << (8 * k))) | (q << (8 * k));
   }
   return word;
@@ -292,8 +320,8 @@ static __device__ __noinline__ uint32_t requant_redo4(uint32_t word, int a0, int
 // a branch after every four elements kept the scheduler from overlapping their multiply-adds.
 __device__ __forceinline__ uint32_t requant_fixed4(const int (&x)[4], const int4& m, const longlong2& a01, const longlong2& a23, int shl,
                                                    uint32_t& low) {
-  const long long p0 = static_cast<long long>(x[0] << shl) * m.x + a01.x, p1 = static_cast<long long>(x[1] << shl) * m.y + a01.y;
-  const long long p2 = static_cast<long long>(x[2] << shl) * m.z + a23.x, p3 = static_cast<long long>(x[3] << shl) * m.w + a23.y;
+  const long long p0 = mad_wide(x[0] << shl, m.x, a01.x), p1 = mad_wide(x[1] << shl, m.y, a01.y);
+  const long long p2 = mad_wide(x[2] << shl, m.z, a23.x), p3 = mad_wide(x[3] << shl, m.w, a23.y);
   low = min(__vimin3_u32(static_cast<uint32_t>(p0), static_cast<uint32_t>(p1), static_cast<uint32_t>(p2)), static_cast<uint32_t>(p3));
   return pack_sat_u8(static_cast<int>(p1 >> 32), static_cast<int>(p0 >> 32),
                      pack_sat_u8(static_cast<int>(p3 >> 32), static_cast<int>(p2 >> 32), 0u));
