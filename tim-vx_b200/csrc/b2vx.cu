@@ -122,6 +122,7 @@ struct b2vx_graph {
   std::vector<std::function<cudaError_t(cudaStream_t)>> copies_in, copies_out;
   std::vector<void*> allocs;
   std::vector<GemmTcPlan*> gemm_plans;
+  std::vector<DwMmaPlan*> dw_plans;
   std::vector<std::function<b2vx_status()>> finalizers;   // run once device scratch exists
   void* scratch = nullptr;
   size_t scratch_bytes = 0;
@@ -524,19 +525,19 @@ bool weights_fit_s8(const TensorRec& w, int Oc) {
   return true;
 }
 
-// Per-channel constants of the tensor-core epilogue's fixed-point requantization (requant_fixed4).  acc_max bounds the
+// Per-channel constants of the fixed-point requantization (requant_fixed4).  acc_max bounds the
 // accumulators; blocks of blk_w channels, counted from the start of each tile of tile_data, share a window.  Returns false
 // when a channel does not allow it (every element then takes the exact sequence).
-bool fixed_point_columns(const PackedContraction& pk, const OutQuant& out, double acc_max, int tile_data, int blk_w, std::vector<FixedColumn>* cols,
-                         int* shl) {
-  const size_t n = pk.acc_scale.size();
+bool fixed_point_columns(const std::vector<int32_t>& bias_full, const std::vector<float>& acc_scale, const OutQuant& out, double acc_max,
+                         int tile_data, int blk_w, std::vector<FixedColumn>* cols, int* shl) {
+  const size_t n = acc_scale.size();
   const double two32 = 4294967296.0;
   if (!(out.scale > 5.5e-20f && out.scale < 1.8e19f)) return false;   // requant_near_half
   std::vector<double> r(n);   // acc_scale / out scale in units of 2^-32
   double r_max = 0.0;
   for (size_t c = 0; c < n; ++c) {
-    r[c] = static_cast<double>(pk.acc_scale[c]) / static_cast<double>(out.scale) * two32;
-    if (!(r[c] >= 0.0 && std::fabs(static_cast<double>(pk.bias_full[c])) * r[c] < 1e18)) return false;
+    r[c] = static_cast<double>(acc_scale[c]) / static_cast<double>(out.scale) * two32;
+    if (!(r[c] >= 0.0 && std::fabs(static_cast<double>(bias_full[c])) * r[c] < 1e18)) return false;
     r_max = std::max(r_max, r[c]);
   }
   int k = 0;
@@ -568,7 +569,7 @@ bool fixed_point_columns(const PackedContraction& pk, const OutQuant& out, doubl
       for (size_t c = c0; c < c1; ++c) {
         FixedColumn& f = (*cols)[c];
         const double centre = r[c] > 0.0 ? (r[c] - static_cast<double>(f.mul) * (1 << k)) / r[c] * mid * two32 : 0.0;
-        f.add = (static_cast<int64_t>(pk.bias_full[c]) << k) * f.mul + (static_cast<int64_t>(out.zp - out.lo) << 32) + (int64_t(1) << 31) +
+        f.add = (static_cast<int64_t>(bias_full[c]) << k) * f.mul + (static_cast<int64_t>(out.zp - out.lo) << 32) + (int64_t(1) << 31) +
                 half_window + std::llround(centre);
         f.window = static_cast<uint32_t>(2 * half_window);
       }
@@ -921,7 +922,7 @@ b2vx_status plan_contraction(b2vx_graph* g, uint32_t node_index, const char* lab
       std::vector<FixedColumn> fix;
       FixedColumn* dfix = nullptr;
       // raw accumulators, the S term and the border corrections each stay below taps * channels * 255 * 128 * 2
-      if (fixed_point_columns(pk, ep.out, 4.0 * taps * x.C * 255 * 128, tiling.data, tiling.blk_w, &fix, &ep.fix_shl)) {
+      if (fixed_point_columns(pk.bias_full, pk.acc_scale, ep.out, 4.0 * taps * x.C * 255 * 128, tiling.data, tiling.blk_w, &fix, &ep.fix_shl)) {
         st = upload(g, fix, &dfix);
         if (st != B2VX_OK) return st;
         ep.fix = dfix;
@@ -1136,6 +1137,33 @@ b2vx_status plan_conv(b2vx_graph* g, uint32_t idx, NodeRec& n) {
   void* ycl = y.d_cl;
   const int xs = x.d.dtype == B2VX_DT_INT8, zx = x.zp(), mult = c.multiplier;
   const OutQuant oq = out_quant(y);
+  // The tensor-instruction form; B2VX_DW_MMA=0 (or a switch that asks for one of the dp2a forms) turns it off.
+  const bool padded = n.pad[0] || n.pad[1] || n.pad[2] || n.pad[3];
+  const bool want_mma = g->use_tc && !std::getenv("B2VX_DW_STRIP") && !std::getenv("B2VX_DW_PIPE") && !(std::getenv("B2VX_DW_MMA") && std::getenv("B2VX_DW_MMA")[0] == '0');
+  if (want_mma && mult == 1 && kh == 3 && kw == 3 && !(padded && zx != 0) && weights_fit_s8(w, y.C)) {
+    std::vector<int8_t> w8(wd.begin(), wd.end());
+    std::vector<int32_t> bfull(bv);
+    for (int oc = 0; oc < y.C; ++oc)
+      for (int t = 0; t < taps; ++t) bfull[oc] -= zx * wd[static_cast<size_t>(t) * y.Cp + oc];
+    std::vector<FixedColumn> fix;
+    int shl = 0;
+    if (fixed_point_columns(bfull, sc, oq, 9.0 * 255 * 128 * 4, y.Cp, 16, &fix, &shl)) {
+      int8_t* dw8 = nullptr; FixedColumn* dfix = nullptr; int32_t* dbf = nullptr;
+      st = upload(g, w8, &dw8);
+      if (st == B2VX_OK) st = upload(g, fix, &dfix);
+      if (st == B2VX_OK) st = upload(g, bfull, &dbf);
+      if (st != B2VX_OK) return st;
+      DwMmaPlan* plan = dw_mma_plan_create(xcl, xs, dw8, dfix, shl, dbf, dsc, geo, oq, ycl, g->status);
+      if (plan) {
+        g->dw_plans.push_back(plan);
+        Step sm;
+        sm.info = make_info("depthwise_mma", idx, 2 * macs, abytes);
+        sm.fn = [=](cudaStream_t st2) { return dw_mma_launch(plan, st2); };
+        g->steps.push_back(std::move(sm));
+        return B2VX_OK;
+      }
+    }
+  }
   if (mult == 1 && taps <= 64) {
     // dp2a kernel: weights as positioned 16-bit halves, zero-point term folded into the bias
     std::vector<uint32_t> wtab(static_cast<size_t>(taps) * y.Cp, 0u);
@@ -1656,6 +1684,7 @@ void b2vx_graph_destroy(b2vx_graph* g) {
   cudaStreamSynchronize(g->stream);
   if (g->exec) cudaGraphExecDestroy(g->exec);
   for (GemmTcPlan* p : g->gemm_plans) gemm_tc_plan_destroy(p);
+  for (DwMmaPlan* p : g->dw_plans) dw_mma_plan_destroy(p);
   for (void* p : g->allocs) cudaFree(p);
   if (g->status) cudaFreeHost(g->status);
   if (g->h_staging) cudaFreeHost(g->h_staging);

@@ -74,6 +74,7 @@
 #include "kernels.h"
 #include "pdl.cuh"
 #include "requant.cuh"
+#include "tma.cuh"
 
 // Build with -DB2VX_TC_TRACE to record, for CTA 0, when each role passed its waits (a debugging aid
 // for pipeline stalls; the normal build contains none of it).  -DB2VX_TRACE_WARP=<4..19> picks the epilogue
@@ -112,7 +113,6 @@ constexpr int kThreadsTc = (kFirstEpilogueWarp + kEpilogueWarps) * 32;
 constexpr int kMaxStages = 8;
 constexpr int kMaxGroup = 8;
 constexpr int kMaxAccBuffers = 8;
-constexpr long long kWaitLimitCycles = 2000000000LL;  // about one second
 constexpr int kSmemBudget = 226 * 1024;               // dynamic shared memory requested at most
 constexpr int kMinDynSmem = 120 * 1024;               // keeps two CTAs from sharing an SM (and its TMEM)
 
@@ -174,87 +174,8 @@ struct GemmParams {
 #endif
 };
 
-// ---- PTX wrappers -----------------------------------------------------------
+// ---- PTX wrappers (the rest: tma.cuh) ----------------------------------------
 
-__device__ __forceinline__ uint32_t smem_u32(const void* p) { return static_cast<uint32_t>(__cvta_generic_to_shared(p)); }
-
-__device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
-}
-__device__ __forceinline__ void mbar_arrive(uint32_t bar) {
-  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
-}
-__device__ __forceinline__ void mbar_arrive_expect_tx(uint32_t bar, uint32_t bytes) {
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
-}
-// try_wait may suspend the thread in hardware until the phase completes or the hint (ns) runs out,
-// which keeps waiting warps out of the issue slots the epilogue warps need.
-__device__ __forceinline__ uint32_t mbar_try_wait(uint32_t bar, uint32_t parity) {
-  uint32_t ok;
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
-      "selp.u32 %0, 1, 0, p;\n\t}"
-      : "=r"(ok)
-      : "r"(bar), "r"(parity), "r"(20000u)
-      : "memory");
-  return ok;
-}
-
-// Bounded wait.  Returns false when the CTA is aborting.  Polls back off: a wait that is not over after
-// a few tries is a long one (a control warp waiting for the epilogue, say), and a warp that keeps
-// polling takes issue slots from the warps it is waiting for; sleeps grow from 64 ns to 1 us.
-__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag, int* status, int code,
-                                          long long limit = kWaitLimitCycles) {
-  if (mbar_try_wait(bar, parity)) return true;
-  const long long start = clock64();
-  unsigned sleep_ns = 32;
-  while (true) {
-#pragma unroll 1
-    for (int i = 0; i < 4; ++i)
-      if (mbar_try_wait(bar, parity)) return true;
-    if (*abort_flag) return false;
-    if (clock64() - start > limit) {
-      *abort_flag = 1;
-      atomicCAS(status, 0, code);
-      return false;
-    }
-    if (sleep_ns < 1024) sleep_ns <<= 1;
-    __nanosleep(sleep_ns);
-  }
-}
-
-// One lane of a fully converged warp.  The control warps run their loops with all 32 lanes (so that
-// every value feeding a TMA or MMA instruction is warp-uniform and can live in uniform registers)
-// and elect a single lane only for the issue itself.
-__device__ __forceinline__ bool elect_one() {
-  uint32_t pred;
-  asm volatile(
-      "{\n\t.reg .pred P;\n\t"
-      "elect.sync _|P, 0xffffffff;\n\t"
-      "selp.u32 %0, 1, 0, P;\n\t}"
-      : "=r"(pred));
-  return pred != 0;
-}
-
-__device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map, int c0, int c1, uint32_t bar) {
-  asm volatile(
-      "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
-      ::"r"(dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(c0), "r"(c1), "r"(bar)
-      : "memory");
-}
-__device__ __forceinline__ void tma_load_4d(uint32_t dst, const CUtensorMap* map, int c0, int c1, int c2, int c3, uint32_t bar) {
-  asm volatile(
-      "cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5}], [%6];"
-      ::"r"(dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(bar)
-      : "memory");
-}
-// Plain (untiled) bulk copy global -> shared: both addresses 16-byte aligned, bytes a multiple of 16.
-__device__ __forceinline__ void bulk_load(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
-  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-               ::"r"(dst), "l"(reinterpret_cast<uint64_t>(src)), "r"(bytes), "r"(bar)
-               : "memory");
-}
 // Barrier among the epilogue warps only.
 __device__ __forceinline__ void epilogue_barrier() { asm volatile("bar.sync 1, %0;" ::"n"(kEpilogueThreads) : "memory"); }
 
@@ -973,47 +894,6 @@ __global__ void __launch_bounds__(128, 1) int8_peak_kernel(int iters, int n, int
 }
 
 // ---- host side ---------------------------------------------------------------
-
-typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
-                                  const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
-                                  CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-
-EncodeTiledFn get_encode_fn() {
-  static EncodeTiledFn fn = [] {
-    void* ptr = nullptr;
-    cudaDriverEntryPointQueryResult qres;
-    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &ptr, cudaEnableDefault, &qres) != cudaSuccess ||
-        qres != cudaDriverEntryPointSuccess)
-      ptr = nullptr;
-    return reinterpret_cast<EncodeTiledFn>(ptr);
-  }();
-  return fn;
-}
-
-CUtensorMapSwizzle swizzle_of(int span) {
-  return span == 128 ? CU_TENSOR_MAP_SWIZZLE_128B : (span == 64 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_32B);
-}
-
-// uint8 tensor of rank 2 or 4, dense (stride of dim i+1 = stride of dim i * dims[i])
-bool encode_u8(CUtensorMap* map, const void* base, int rank, const uint64_t* dims, const uint32_t* box, const uint32_t* estr,
-               CUtensorMapSwizzle swz) {
-  EncodeTiledFn fn = get_encode_fn();
-  if (!fn) return false;
-  cuuint64_t d[4], strides[3];
-  cuuint32_t b[4], e[4];
-  uint64_t pitch = 1;
-  for (int i = 0; i < rank; ++i) {
-    d[i] = dims[i];
-    b[i] = box[i];
-    e[i] = estr ? estr[i] : 1;
-    pitch *= dims[i];
-    if (i + 1 < rank) strides[i] = pitch;
-  }
-  CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, static_cast<cuuint32_t>(rank), const_cast<void*>(base), d, strides, b, e,
-                  CU_TENSOR_MAP_INTERLEAVE_NONE, swz, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
-                  CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  return r == CUDA_SUCCESS;
-}
 
 }  // namespace
 

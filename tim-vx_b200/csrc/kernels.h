@@ -111,6 +111,16 @@ void launch_depthwise_q(const void* x, int x_signed, int zx, const int16_t* wd, 
 void launch_depthwise_q16(const void* x, int x_signed, int zx, const uint32_t* wtab, const uint32_t* wtab_v, const int32_t* bias_full,
                           const float* acc_scale, const ConvGeom& g, OutQuant out, int exact_only, void* y, cudaStream_t s);
 
+// 3x3, multiplier 1, stride 1 or 2, no dilation, on the warp-level tensor instruction (depthwise_mma.cu).  w: [9][Cp]
+// int8 weights with their zero point subtracted; fix, shl, bias_full, acc_scale: per channel, bias with the input zero
+// point folded in; padding reads as zero, so with padding the input zero point must be 0.  status: device int of the
+// bounded waits.  Null: not this kernel's layer.
+struct DwMmaPlan;
+DwMmaPlan* dw_mma_plan_create(const void* x, int x_signed, const int8_t* w, const FixedColumn* fix, int shl, const int32_t* bias_full,
+                              const float* acc_scale, const ConvGeom& g, OutQuant out, void* y, int* status);
+void dw_mma_plan_destroy(DwMmaPlan* p);
+cudaError_t dw_mma_launch(const DwMmaPlan* p, cudaStream_t s);
+
 // ---- float32 convolution (dense or depthwise), accumulation order ic,ky,kx --
 // w: original WHIcOc layout; bias may be null.
 void launch_conv_f32(const float* x, const float* w, const float* bias, int multiplier, int w_ic,
