@@ -1756,14 +1756,6 @@ __global__ void __launch_bounds__(256) im2col_whcn8_kernel(const uint8_t* __rest
 
 // ---------------------------------------------------------------- FullyConnected with few rows (M <= 16)
 
-// Weights do not depend on the layer before: a block that is resident early asks for its rows (one per lane of the first
-// warp) to be brought into L2 before it waits for its input.
-__device__ __forceinline__ void prefetch_rows_l2(const int8_t* B, int Kp, int row0, int row_end) {
-  const int row = row0 + static_cast<int>(threadIdx.x);
-  if (threadIdx.x < 32 && row < row_end)
-    asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(B + static_cast<size_t>(row) * Kp), "r"(Kp) : "memory");
-}
-
 // Decode-like shapes are bound by streaming the weights once; a 128-row tensor-core tile would spend its
 // time on pipeline latency with a handful of CTAs.  Here a block of eight warps owns CH = 4 output
 // channels and all M input rows, and its 256 lanes split K in 16-byte slices: a lane loads the four
@@ -1776,9 +1768,8 @@ __device__ __forceinline__ void prefetch_rows_l2(const int8_t* B, int Kp, int ro
 template <int CH, int MT, bool XS, bool HAS_DZ>
 __global__ void __launch_bounds__(256, 2) fc_small_m_kernel(const uint8_t* __restrict__ A, const int8_t* __restrict__ B, int M, int Kp,
                                                          int Oc, int Ocp, ContractEpilogue ep, uint8_t* __restrict__ D, int ldd) {
-  pdl_trigger();
-  prefetch_rows_l2(B, Kp, blockIdx.x * CH, min(static_cast<int>(blockIdx.x) * CH + CH, Ocp));
   pdl_wait();
+  pdl_trigger();
   constexpr int V = CH * MT;                        // partial sums per lane: 4 ... 64
   constexpr int KEEP = V >= 64 ? 2 : 1;             // values a lane still holds after the exchange
   __shared__ int partial[8][32 * KEEP];
@@ -2369,9 +2360,8 @@ __device__ __forceinline__ void mma_m16n8k32(int (&c)[4], uint32_t a0, uint32_t 
 template <bool XS, bool HAS_DZ>
 __global__ void __launch_bounds__(256, 2) fc_mma16_kernel(const uint8_t* __restrict__ A, const int8_t* __restrict__ B, int M, int Kp,
                                                           int Oc, int Ocp, ContractEpilogue ep, uint8_t* __restrict__ D, int ldd) {
-  pdl_trigger();
-  prefetch_rows_l2(B, Kp, blockIdx.x * 32, min(static_cast<int>(blockIdx.x) * 32 + 32, Ocp));
   pdl_wait();
+  pdl_trigger();
   constexpr int NT = 4;                              // n-tiles of eight channels per warp
   __shared__ int partial[8][16][NT * 8 + 1];
   __shared__ int s_sum[8][16];
