@@ -42,3 +42,29 @@ def test_round_trip(product_lib, dims):
     g.profile(2)
     np.testing.assert_array_equal(g.read(y), want(a))
     g.close()
+
+
+# 10 bytes in one row, 48 bytes whose layouts coincide, 180 bytes that a kernel writes over the bus, 5 KB, and 300 KB (not staged)
+@pytest.mark.parametrize("dims", [(1, 1, 10, 1), (1, 1, 16, 3), (3, 3, 10, 2), (8, 8, 80, 1), (64, 64, 74, 1)])
+def test_written_output_is_read_back(product_lib, dims):
+    rng = np.random.default_rng(4)
+    a, b, c = (rng.integers(0, 256, size=dims[::-1]).astype(np.uint8) for _ in range(3))
+    want = np.maximum(a, 10)
+    g = B.Graph(product_lib, 0)
+    x = g.tensor(B.DT_UINT8, list(dims), B.ATTR_INPUT, scale=0.1, zero_point=10)
+    y = g.tensor(B.DT_UINT8, list(dims), B.ATTR_OUTPUT, scale=0.1, zero_point=10)
+    g.relu(x, y)
+    g.write(y, b)
+    g.compile()
+    np.testing.assert_array_equal(g.read(y), b)     # written before the graph was compiled
+    g.write(x, a)
+    g.run()
+    np.testing.assert_array_equal(g.read(y), want)
+    g.write(y, c)
+    np.testing.assert_array_equal(g.read(y), c)     # and after a run
+    g.run_async()
+    g.write(y, b)                                   # waits for the run
+    np.testing.assert_array_equal(g.read(y), b)
+    g.run()
+    np.testing.assert_array_equal(g.read(y), want)
+    g.close()

@@ -63,7 +63,8 @@ struct TensorRec {
   bool is_activation = false;
   bool cl_used = false;        // some kernel reads the channels-last copy (decides whether a graph input is converted)
   // Small inputs and outputs go through page-locked memory of the graph (see kStagedBytes): the caller's bytes of an
-  // input, or the result of an output as of the last run.  d_io may point here too.
+  // input; what an output holds, which is the result of the last run or what the caller wrote into it since.  d_io may
+  // point here too.
   uint8_t* h_in = nullptr;
   uint8_t* h_out = nullptr;
   bool io_direct = false;      // a graph output whose producer writes the WHCN copy itself (no conversion at the end)
@@ -1748,12 +1749,12 @@ b2vx_status b2vx_tensor_write(b2vx_graph* g, uint32_t id, const void* src, size_
   }
   if (t.d.attr & B2VX_ATTR_CONSTANT) return fail(g, B2VX_BAD_STATE, "tensor_write: constants are frozen at compile");
   if (!t.d_io) return fail(g, B2VX_BAD_STATE, "tensor_write: tensor has no device storage");
-  if (t.h_in) {
-    if (!g->idle) {   // a queued run may still read the previous bytes
+  if (t.h_in || t.h_out) {
+    if (!g->idle) {   // a queued run may still read the previous bytes, or has yet to store its result
       DeviceGuard guard(g->device);
       CUDA_TRY(g, wait_idle(g));
     }
-    std::memcpy(t.h_in, src, bytes);
+    std::memcpy(t.h_in ? t.h_in : t.h_out, src, bytes);
     return B2VX_OK;
   }
   DeviceGuard guard(g->device);
@@ -2170,8 +2171,8 @@ b2vx_status b2vx_graph_compile(b2vx_graph* g) {
   // 4. data that was supplied before compile: inputs written early, constant activations
   for (TensorRec& t : g->tensors) {
     if (!t.is_activation || !t.host_valid || !t.d_io) continue;
-    if (t.h_in) {
-      std::memcpy(t.h_in, t.host.data(), t.io_bytes);
+    if (t.h_in || t.h_out) {
+      std::memcpy(t.h_in ? t.h_in : t.h_out, t.host.data(), t.io_bytes);
       continue;
     }
     CUDA_TRY(g, cudaMemcpyAsync(t.d_io, t.host.data(), t.io_bytes, cudaMemcpyHostToDevice, g->stream));
