@@ -68,3 +68,33 @@ def test_written_output_is_read_back(product_lib, dims):
     g.run()
     np.testing.assert_array_equal(g.read(y), want)
     g.close()
+
+
+# staged in one piece, by rows, over the bus, and not staged
+@pytest.mark.parametrize("dims", [(8, 8, 80, 1), (1, 1, 1000, 7), (3, 3, 10, 2), (64, 64, 74, 1)])
+def test_run_recorded_on_a_stream_of_the_caller(product_lib, dims):
+    """The caller records the first run_async into a CUDA graph of its own and launches that without this library's
+    knowing: what is written before a launch goes into it, and a read waits for it."""
+    import torch
+    rng = np.random.default_rng(5)
+    data = [rng.integers(0, 256, size=dims[::-1]).astype(np.uint8) for _ in range(4)]
+    g, x, y = relu(product_lib, list(dims))
+    st = torch.cuda.Stream()
+    g.set_stream(st.cuda_stream)
+    recorded = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(recorded, stream=st, capture_error_mode="thread_local"):
+        g.run_async()
+    for a in data:
+        g.write(x, a)
+        with torch.cuda.stream(st):
+            torch.cuda._sleep(20_000_000)   # about 10 ms: the launch behind it is still queued when the read begins
+            recorded.replay()
+        np.testing.assert_array_equal(g.read(y), np.maximum(a, 10))
+    with torch.cuda.stream(st):
+        torch.cuda._sleep(20_000_000)
+        recorded.replay()
+    g.write(x, data[0])                     # waits for that launch, which still reads the last one's bytes
+    np.testing.assert_array_equal(g.read(y), np.maximum(data[-1], 10))
+    torch.cuda.synchronize()
+    recorded.reset()
+    g.close()

@@ -129,7 +129,10 @@ struct b2vx_graph {
   size_t scratch_bytes = 0;
   int* status = nullptr;       // page-locked: kernels that gave up on a barrier store a code here
   uint8_t* h_staging = nullptr;
-  bool idle = true;            // nothing queued since the stream was last waited for
+  bool idle = true;            // no call of ours has queued anything since the stream was last waited for
+  // The caller has handed over a stream of its own at some time: it may have recorded runs of this graph there and launch
+  // them without our knowing, so `idle` says nothing.
+  bool shared_stream = false;
   bool compiled = false;
   bool use_tc = false;
   bool fuse_add = true;      // residual Add into the preceding convolution's epilogue (B2VX_FUSE_ADD=0 disables)
@@ -218,7 +221,8 @@ constexpr size_t kTinyBytes = 4096;
 
 // Waits for everything of this graph that is queued on its stream.
 cudaError_t wait_idle(b2vx_graph* g) {
-  if (g->idle) return cudaSuccess;
+  if (g->idle && !g->shared_stream) return cudaSuccess;
+  DeviceGuard guard(g->device);
   const cudaError_t e = cudaStreamSynchronize(g->stream);
   if (e == cudaSuccess) g->idle = true;
   return e;
@@ -1750,10 +1754,7 @@ b2vx_status b2vx_tensor_write(b2vx_graph* g, uint32_t id, const void* src, size_
   if (t.d.attr & B2VX_ATTR_CONSTANT) return fail(g, B2VX_BAD_STATE, "tensor_write: constants are frozen at compile");
   if (!t.d_io) return fail(g, B2VX_BAD_STATE, "tensor_write: tensor has no device storage");
   if (t.h_in || t.h_out) {
-    if (!g->idle) {   // a queued run may still read the previous bytes, or has yet to store its result
-      DeviceGuard guard(g->device);
-      CUDA_TRY(g, wait_idle(g));
-    }
+    CUDA_TRY(g, wait_idle(g));   // a queued run may still read the previous bytes, or has yet to store its result
     std::memcpy(t.h_in ? t.h_in : t.h_out, src, bytes);
     return B2VX_OK;
   }
@@ -1779,10 +1780,7 @@ b2vx_status b2vx_tensor_read(b2vx_graph* g, uint32_t id, void* dst, size_t bytes
     return B2VX_OK;
   }
   if (t.h_in || t.h_out) {
-    if (!g->idle) {
-      DeviceGuard guard(g->device);
-      CUDA_TRY(g, wait_idle(g));
-    }
+    CUDA_TRY(g, wait_idle(g));
     std::memcpy(dst, t.h_in ? t.h_in : t.h_out, bytes);
     return B2VX_OK;
   }
@@ -2249,6 +2247,7 @@ b2vx_status b2vx_graph_set_stream(b2vx_graph* g, void* cuda_stream) {
   DeviceGuard guard(g->device);
   cudaStreamSynchronize(g->stream);
   g->idle = true;
+  g->shared_stream = g->shared_stream || cuda_stream != nullptr;
   g->stream = cuda_stream ? static_cast<cudaStream_t>(cuda_stream) : g->own_stream;
   return B2VX_OK;
 }
