@@ -192,9 +192,10 @@ struct DeviceGuard {
   }
 };
 
+// Whole 16-byte pieces: launch_copy16 reads and writes the last one in full.
 b2vx_status dev_alloc(b2vx_graph* g, void** out, size_t bytes) {
   *out = nullptr;
-  if (bytes == 0) bytes = 16;
+  bytes = bytes ? (bytes + 15) & ~static_cast<size_t>(15) : 16;
   cudaError_t e = cudaMalloc(out, bytes);
   if (e != cudaSuccess) return fail(g, B2VX_OOM, std::string("cudaMalloc: ") + cudaGetErrorString(e));
   g->allocs.push_back(*out);
