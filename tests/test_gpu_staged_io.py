@@ -98,3 +98,83 @@ def test_run_recorded_on_a_stream_of_the_caller(product_lib, dims):
     torch.cuda.synchronize()
     recorded.reset()
     g.close()
+
+
+def add(lib, n):
+    """Two inputs of n elements each, one output: rows of one pixel where n is a multiple of 16, else 3 x 3 pixels."""
+    dims = [1, 1, n, 1] if n % 16 == 0 else [3, 3, n // 9, 1]
+    g = B.Graph(lib, 0)
+    a, b = (g.tensor(B.DT_UINT8, dims, B.ATTR_INPUT, scale=0.1, zero_point=0) for _ in range(2))
+    y = g.tensor(B.DT_UINT8, dims, B.ATTR_OUTPUT, scale=0.1, zero_point=0)
+    g.add(a, b, y)
+    return g, a, b, y, dims[::-1]
+
+
+@pytest.mark.parametrize("n", [16, 90, 9009, 65536])
+def test_one_of_two_inputs_changes(product_lib, n):
+    """Runs that wait and runs that do not, in turn, with one input or none written in between."""
+    rng = np.random.default_rng(6)
+    g, a, b, y, shape = add(product_lib, n)
+    g.compile()
+    v = [np.zeros(shape, np.uint8), np.zeros(shape, np.uint8)]
+    for step in range(24):
+        which = (None, 0, None, 1, 0, 1)[step % 6]
+        if which is not None:
+            v[which] = rng.integers(0, 128, size=shape).astype(np.uint8)
+            g.write((a, b)[which], v[which])
+        if step % 5 < 2:
+            g.run()
+        elif step % 5 == 2:
+            g.profile(1)
+        else:
+            for _ in range(step % 3 + 1):
+                g.run_async()
+        if step % 4:
+            np.testing.assert_array_equal(g.read(y), v[0] + v[1])
+    g.close()
+
+
+@pytest.mark.parametrize("n", [16, 90, 9009, 65536])
+def test_stream_handed_over_between_runs(product_lib, n):
+    """What was written or computed before the graph gets a stream of the caller's is there afterwards."""
+    import torch
+    rng = np.random.default_rng(7)
+    g, a, b, y, shape = add(product_lib, n)
+    u, v, w = (rng.integers(0, 80, size=shape).astype(np.uint8) for _ in range(3))
+    g.write(a, u)
+    g.compile()
+    g.write(b, v)
+    g.run()
+    st = torch.cuda.Stream()
+    g.set_stream(st.cuda_stream)
+    np.testing.assert_array_equal(g.read(y), u + v)
+    g.write(a, w)
+    g.run_async()
+    np.testing.assert_array_equal(g.read(y), w + v)
+    g.write(y, u)
+    np.testing.assert_array_equal(g.read(y), u)
+    g.set_stream(None)
+    np.testing.assert_array_equal(g.read(y), u)
+    g.run()
+    np.testing.assert_array_equal(g.read(y), w + v)
+    g.close()
+
+
+@pytest.mark.parametrize("spec", ["gemm:16:4096:4096", "conv:3:64:64:56:1"])
+def test_resident_data_is_not_moved_again(product_lib, spec):
+    """run_async on data that is there launches the kernels of the plan and nothing else."""
+    import torch
+    import opworkloads
+    g = B.Graph(product_lib, 0)
+    work = opworkloads.build(spec, 1, g, np.random.default_rng(8))
+    for t, a in work["inputs"]:
+        g.write(t, a)
+    g.run_async()
+    g.sync()
+    with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA], acc_events=True) as prof:
+        for _ in range(3):
+            g.run_async()
+        g.sync()
+    launched = [e.name for e in prof.events() if e.device_type == torch.autograd.DeviceType.CUDA]
+    assert len(launched) == 3 * len(g.kernels()), launched
+    g.close()

@@ -63,10 +63,14 @@ struct TensorRec {
   bool is_activation = false;
   bool cl_used = false;        // some kernel reads the channels-last copy (decides whether a graph input is converted)
   // Small inputs and outputs go through page-locked memory of the graph (see kStagedBytes): the caller's bytes of an
-  // input; what an output holds, which is the result of the last run or what the caller wrote into it since.  d_io may
-  // point here too.
+  // input; what an output holds, which is the result of the last run or what the caller wrote into it since.
   uint8_t* h_in = nullptr;
   uint8_t* h_out = nullptr;
+  bool in_pending = false;     // h_in holds bytes that have not been copied to the device
+  bool out_behind = false;     // the device holds a result that has not been copied to h_out
+  // d_io is the page-locked copy during a run that brings its outputs along, and this device buffer otherwise (set_io)
+  bool over_bus = false;
+  void* d_dev = nullptr;
   bool io_direct = false;      // a graph output whose producer writes the WHCN copy itself (no conversion at the end)
 
   size_t elems() const {
@@ -119,8 +123,6 @@ struct b2vx_graph {
   std::vector<NodeRec> nodes;
   std::vector<uint32_t> order;
   std::vector<Step> steps;
-  // transfers of small inputs and outputs before and after the steps of a run (kStagedBytes)
-  std::vector<std::function<cudaError_t(cudaStream_t)>> copies_in, copies_out;
   std::vector<void*> allocs;
   std::vector<GemmTcPlan*> gemm_plans;
   std::vector<DwMmaPlan*> dw_plans;
@@ -129,9 +131,10 @@ struct b2vx_graph {
   size_t scratch_bytes = 0;
   int* status = nullptr;       // page-locked: kernels that gave up on a barrier store a code here
   uint8_t* h_staging = nullptr;
+  std::vector<uint32_t> staged;   // tensors with h_in or h_out
   bool idle = true;            // no call of ours has queued anything since the stream was last waited for
   // The caller has handed over a stream of its own at some time: it may have recorded runs of this graph there and launch
-  // them without our knowing, so `idle` says nothing.
+  // them without our knowing.
   bool shared_stream = false;
   bool compiled = false;
   bool use_tc = false;
@@ -141,8 +144,9 @@ struct b2vx_graph {
   bool fuse_done = false;
   bool fc_small_m = true;    // FullyConnected with <= 16 rows on the CUDA-core streaming kernel
   int add_mode = 0;          // quantized Add: 0 choose by size, 1 table kernel, 2 arithmetic kernel
-  // the whole launch plan captured once as a CUDA graph; replays cost one launch on the host
-  cudaGraphExec_t exec = nullptr;
+  // the whole launch plan captured once as a CUDA graph, in the forms of launch_plan that are used; replays cost one
+  // launch on the host
+  cudaGraphExec_t exec[3] = {nullptr, nullptr, nullptr};
   bool capture_failed = false;
   bool use_cuda_graph = true;
 };
@@ -213,20 +217,66 @@ b2vx_status upload(b2vx_graph* g, const std::vector<T>& v, T** out) {
 }
 
 // Inputs and outputs of up to this many bytes are not copied by the copy engine: a write is a memcpy into page-locked
-// memory, which a copy kernel at the head of the run reads over the bus, and the last kernel of a run leaves the output in
-// page-locked memory, where a read finds it (in 16-byte pieces: 64 x 1000 results as single bytes took 117 us).  A copy call of its own costs 8 - 13 us from call to
-// return whatever its size; at 50 GB/s over the bus and about 15 GB/s for the memcpy, 256 KB costs about as much.
+// memory, which the next run reads over the bus, by a copy kernel at its head; a run that waits for its result
+// leaves the outputs in page-locked memory, where a read finds them (in 16-byte pieces: 64 x 1000 results as single bytes
+// took 117 us).  A copy call of its own costs 8 - 13 us from call to return whatever its size; at 50 GB/s over the bus and
+// about 15 GB/s for the memcpy, 256 KB costs about as much.
+// Runs on data that is on the device already (run_async again and again) move nothing over the bus: with the copies in
+// every run, 16 rows through a 4096 x 4096 layer took 22.5 us for 14.3.
 constexpr size_t kStagedBytes = 256 * 1024;
-// Inputs this small are read over the bus by the kernels themselves, without a copy on the device.
+// Inputs and outputs this small are read and written over the bus by the kernels of a run that waits for its result,
+// without a copy on the device.
 constexpr size_t kTinyBytes = 4096;
 
 // Waits for everything of this graph that is queued on its stream.
 cudaError_t wait_idle(b2vx_graph* g) {
-  if (g->idle && !g->shared_stream) return cudaSuccess;
+  if (g->idle) return cudaSuccess;
   DeviceGuard guard(g->device);
   const cudaError_t e = cudaStreamSynchronize(g->stream);
   if (e == cudaSuccess) g->idle = true;
   return e;
+}
+
+void* device_io(const TensorRec& t) { return t.over_bus ? t.d_dev : t.d_io; }
+
+cudaError_t copy_staged(b2vx_graph* g, const void* from, void* to, size_t bytes) {
+  DeviceGuard guard(g->device);
+  g->idle = false;
+  launch_copy16(from, to, (bytes + 15) / 16, g->stream);
+  return cudaGetLastError();
+}
+
+// Whether a run copies this input to the device once it has been written.
+bool copied_in(const TensorRec& t, bool to_host) { return t.h_in && !(t.over_bus && to_host); }
+
+// Inputs that were written since their last copy to the device.
+cudaError_t push_inputs(b2vx_graph* g, bool to_host) {
+  for (uint32_t id : g->staged) {
+    TensorRec& t = g->tensors[id];
+    if (!t.in_pending || !copied_in(t, to_host)) continue;
+    const cudaError_t e = copy_staged(g, t.h_in, device_io(t), t.io_bytes);
+    if (e != cudaSuccess) return e;
+    t.in_pending = false;
+  }
+  return cudaSuccess;
+}
+
+// Once the caller shares a stream with the graph, the page-locked copies are no longer used: a run that the caller has
+// recorded there knows nothing of them.
+cudaError_t share_staging(b2vx_graph* g) {
+  cudaError_t e = push_inputs(g, false);
+  for (uint32_t id : g->staged) {
+    const TensorRec& t = g->tensors[id];
+    if (e == cudaSuccess && t.h_out && !t.out_behind) e = copy_staged(g, t.h_out, device_io(t), t.io_bytes);
+  }
+  return e;
+}
+
+void set_io(b2vx_graph* g, bool to_host) {
+  for (uint32_t id : g->staged) {
+    TensorRec& t = g->tensors[id];
+    if (t.over_bus) t.d_io = !to_host ? t.d_dev : t.h_in ? t.h_in : t.h_out;
+  }
 }
 
 // ---------------------------------------------------------------- shapes
@@ -977,20 +1027,20 @@ b2vx_status plan_contraction(b2vx_graph* g, uint32_t node_index, const char* lab
     void* ycl = fused_out ? fused_out : y.d_cl;
     const int ldd = y.Cp, Oc = y.C, y_signed = y.d.dtype == B2VX_DT_INT8;
     if (mode == WHCN8) {
-      const void* xio = x.d_io;
+      const size_t xid = &x - g->tensors.data();
       Step s_col;
       s_col.info = make_info(padk == 8 ? "im2col_whcn8" : "im2col_whcn4", node_index, 0, x.elems() + static_cast<uint64_t>(M) * Kp);
       s_col.fn = [=](cudaStream_t st2) {
-        launch_im2col_whcn8(xio, Kp, zx, geo, padk, g->scratch, st2);
+        launch_im2col_whcn8(g->tensors[xid].d_io, Kp, zx, geo, padk, g->scratch, st2);
         return cudaGetLastError();
       };
       g->steps.push_back(std::move(s_col));
     } else if (mode == WHCN) {
-      const void* xio = x.d_io;
+      const size_t xid = &x - g->tensors.data();
       Step s_col;
       s_col.info = make_info("im2col_whcn", node_index, 0, x.elems() + static_cast<uint64_t>(M) * Kp);
       s_col.fn = [=](cudaStream_t st2) {
-        launch_im2col_whcn(xio, Kp, zx, geo, g->scratch, st2);
+        launch_im2col_whcn(g->tensors[xid].d_io, Kp, zx, geo, g->scratch, st2);
         return cudaGetLastError();
       };
       g->steps.push_back(std::move(s_col));
@@ -1478,12 +1528,16 @@ b2vx_status plan_move(b2vx_graph* g, uint32_t idx, NodeRec& n) {
   } else {
     return fail(g, B2VX_UNSUPPORTED, "dataconvert: supported are 8-bit <-> 8-bit, float32 <-> 8-bit and float32 -> float32");
   }
-  const void* xp = x_dense ? x.d_io : cl_in(x);
-  void* yp = y_dense ? y.d_io : y.d_cl;
+  const void* xcl = x_dense ? nullptr : cl_in(x);
+  void* ycl = y_dense ? nullptr : y.d_cl;
+  const uint32_t xid = n.in[0], yid = n.out;
   if (y_dense) y.io_direct = true;
   Step s;
   s.info = make_info(name, idx, 0, x.bytes() + y.bytes());
-  s.fn = [=](cudaStream_t st2) { launch_relayout(xp, yp, p, st2); return cudaGetLastError(); };
+  s.fn = [=](cudaStream_t st2) {
+    launch_relayout(xcl ? xcl : g->tensors[xid].d_io, ycl ? ycl : g->tensors[yid].d_io, p, st2);
+    return cudaGetLastError();
+  };
   g->steps.push_back(std::move(s));
   return B2VX_OK;
 }
@@ -1688,7 +1742,8 @@ void b2vx_graph_destroy(b2vx_graph* g) {
   if (!g) return;
   DeviceGuard guard(g->device);
   cudaStreamSynchronize(g->stream);
-  if (g->exec) cudaGraphExecDestroy(g->exec);
+  for (cudaGraphExec_t e : g->exec)
+    if (e) cudaGraphExecDestroy(e);
   for (GemmTcPlan* p : g->gemm_plans) gemm_tc_plan_destroy(p);
   for (DwMmaPlan* p : g->dw_plans) dw_mma_plan_destroy(p);
   for (void* p : g->allocs) cudaFree(p);
@@ -1754,14 +1809,16 @@ b2vx_status b2vx_tensor_write(b2vx_graph* g, uint32_t id, const void* src, size_
   }
   if (t.d.attr & B2VX_ATTR_CONSTANT) return fail(g, B2VX_BAD_STATE, "tensor_write: constants are frozen at compile");
   if (!t.d_io) return fail(g, B2VX_BAD_STATE, "tensor_write: tensor has no device storage");
-  if (t.h_in || t.h_out) {
+  if ((t.h_in || t.h_out) && !g->shared_stream) {
     CUDA_TRY(g, wait_idle(g));   // a queued run may still read the previous bytes, or has yet to store its result
     std::memcpy(t.h_in ? t.h_in : t.h_out, src, bytes);
+    t.in_pending = t.h_in != nullptr;
+    t.out_behind = false;
     return B2VX_OK;
   }
   DeviceGuard guard(g->device);
   g->idle = false;
-  CUDA_TRY(g, cudaMemcpyAsync(t.d_io, src, bytes, cudaMemcpyHostToDevice, g->stream));
+  CUDA_TRY(g, cudaMemcpyAsync(device_io(t), src, bytes, cudaMemcpyHostToDevice, g->stream));
   CUDA_TRY(g, wait_idle(g));
   return B2VX_OK;
 }
@@ -1780,7 +1837,11 @@ b2vx_status b2vx_tensor_read(b2vx_graph* g, uint32_t id, void* dst, size_t bytes
     std::memcpy(dst, t.host.data(), bytes);
     return B2VX_OK;
   }
-  if (t.h_in || t.h_out) {
+  if ((t.h_in || t.h_out) && !g->shared_stream) {
+    if (t.out_behind) {
+      CUDA_TRY(g, copy_staged(g, device_io(t), t.h_out, bytes));
+      t.out_behind = false;
+    }
     CUDA_TRY(g, wait_idle(g));
     std::memcpy(dst, t.h_in ? t.h_in : t.h_out, bytes);
     return B2VX_OK;
@@ -1788,7 +1849,7 @@ b2vx_status b2vx_tensor_read(b2vx_graph* g, uint32_t id, void* dst, size_t bytes
   DeviceGuard guard(g->device);
   if (t.d_io) {
     g->idle = false;
-    CUDA_TRY(g, cudaMemcpyAsync(dst, t.d_io, bytes, cudaMemcpyDeviceToHost, g->stream));
+    CUDA_TRY(g, cudaMemcpyAsync(dst, device_io(t), bytes, cudaMemcpyDeviceToHost, g->stream));
     CUDA_TRY(g, wait_idle(g));
     return B2VX_OK;
   }
@@ -2071,13 +2132,18 @@ b2vx_status b2vx_graph_compile(b2vx_graph* g) {
   }
 
   if (staging) {
+    if (g->h_staging) cudaFreeHost(g->h_staging);   // of a Compile that failed
+    g->h_staging = nullptr;
     CUDA_TRY(g, cudaHostAlloc(reinterpret_cast<void**>(&g->h_staging), staging, cudaHostAllocDefault));
     std::memset(g->h_staging, 0, staging);
+    g->staged.clear();
     for (const auto& s : staged) {
       TensorRec& t = g->tensors[s.first];
       (t.d.attr & B2VX_ATTR_INPUT ? t.h_in : t.h_out) = g->h_staging + s.second;
-      // tiny ones are read and written over the bus by the graph's own kernels
-      if (t.d_io != t.d_cl && t.io_bytes <= kTinyBytes) t.d_io = g->h_staging + s.second;
+      g->staged.push_back(static_cast<uint32_t>(s.first));
+      t.in_pending = t.h_in != nullptr;
+      t.over_bus = t.d_io != t.d_cl && t.io_bytes <= kTinyBytes;
+      t.d_dev = t.d_io;
     }
   }
 
@@ -2116,20 +2182,13 @@ b2vx_status b2vx_graph_compile(b2vx_graph* g) {
     std::vector<Step> head;
     for (size_t i = 0; i < g->tensors.size(); ++i) {
       TensorRec& t = g->tensors[i];
-      if (t.is_activation && t.h_in && t.d_io != t.h_in) {
-        const void* from = t.h_in;
-        void* to = t.d_io;
-        const size_t n16 = (t.io_bytes + 15) / 16;
-        g->copies_in.push_back([=](cudaStream_t st2) { launch_copy16(from, to, n16, st2); return cudaGetLastError(); });
-      }
       if (!t.is_activation || !t.cl_used || !(t.d.attr & (B2VX_ATTR_INPUT | B2VX_ATTR_VARIABLE))) continue;
       if (t.d_io == t.d_cl) continue;
-      const void* src = t.d_io;
       void* dst = t.d_cl;
       const int N = t.N, C = t.C, H = t.H, W = t.W, Cp = t.Cp, el = static_cast<int>(dtype_size(t.d.dtype));
       Step s;
       s.info = make_info("whcn_to_cl", B2VX_NO_TENSOR, 0, t.io_bytes + t.cl_bytes);
-      s.fn = [=](cudaStream_t st2) { launch_whcn_to_cl(src, dst, N, C, H, W, Cp, el, st2); return cudaGetLastError(); };
+      s.fn = [=](cudaStream_t st2) { launch_whcn_to_cl(g->tensors[i].d_io, dst, N, C, H, W, Cp, el, st2); return cudaGetLastError(); };
       head.push_back(std::move(s));
     }
     g->steps.insert(g->steps.begin(), std::make_move_iterator(head.begin()), std::make_move_iterator(head.end()));
@@ -2137,25 +2196,17 @@ b2vx_status b2vx_graph_compile(b2vx_graph* g) {
   for (size_t i = 0; i < g->tensors.size(); ++i) {
     TensorRec& t = g->tensors[i];
     if (!t.is_activation || !(t.d.attr & B2VX_ATTR_OUTPUT)) continue;
-    if (t.d_io != t.d_cl && !t.io_direct) {
-      const void* src = t.d_cl;
-      // one pixel per image: the rows lose their padding on the way to the host
-      const bool rows = t.h_out != nullptr && t.H * t.W == 1;
-      void* dst = rows ? t.h_out : t.d_io;
-      const int N = t.N, C = t.C, H = t.H, W = t.W, Cp = t.Cp, el = static_cast<int>(dtype_size(t.d.dtype));
-      Step s;
-      s.info = make_info("cl_to_whcn", B2VX_NO_TENSOR, 0, t.io_bytes + t.cl_bytes);
-      if (rows) s.fn = [=](cudaStream_t st2) { launch_pack_rows16(src, dst, N, C * el, Cp * el, st2); return cudaGetLastError(); };
-      else s.fn = [=](cudaStream_t st2) { launch_cl_to_whcn(src, dst, N, C, H, W, Cp, el, st2); return cudaGetLastError(); };
-      g->steps.push_back(std::move(s));
-      if (rows) continue;
-    }
-    if (t.h_out && t.d_io != t.h_out) {
-      const void* from = t.d_io;
-      void* to = t.h_out;
-      const size_t n16 = (t.io_bytes + 15) / 16;
-      g->copies_out.push_back([=](cudaStream_t st2) { launch_copy16(from, to, n16, st2); return cudaGetLastError(); });
-    }
+    if (t.d_io == t.d_cl || t.io_direct) continue;
+    const void* src = t.d_cl;
+    // one pixel per image: the rows lose their padding on the way to the host
+    const bool rows = t.h_out != nullptr && t.H * t.W == 1;
+    if (rows) t.over_bus = true;
+    const int N = t.N, C = t.C, H = t.H, W = t.W, Cp = t.Cp, el = static_cast<int>(dtype_size(t.d.dtype));
+    Step s;
+    s.info = make_info("cl_to_whcn", B2VX_NO_TENSOR, 0, t.io_bytes + t.cl_bytes);
+    if (rows) s.fn = [=](cudaStream_t st2) { launch_pack_rows16(src, g->tensors[i].d_io, N, C * el, Cp * el, st2); return cudaGetLastError(); };
+    else s.fn = [=](cudaStream_t st2) { launch_cl_to_whcn(src, g->tensors[i].d_io, N, C, H, W, Cp, el, st2); return cudaGetLastError(); };
+    g->steps.push_back(std::move(s));
   }
   if (g->scratch_bytes) {
     b2vx_status st = dev_alloc(g, &g->scratch, g->scratch_bytes);
@@ -2178,50 +2229,85 @@ b2vx_status b2vx_graph_compile(b2vx_graph* g) {
     if ((t.d.attr & B2VX_ATTR_CONSTANT) && t.d_io != t.d_cl)
       launch_whcn_to_cl(t.d_io, t.d_cl, t.N, t.C, t.H, t.W, t.Cp, static_cast<int>(dtype_size(t.d.dtype)), g->stream);
   }
+  if (g->shared_stream) CUDA_TRY(g, share_staging(g));
   CUDA_TRY(g, cudaStreamSynchronize(g->stream));
   CUDA_TRY(g, cudaGetLastError());
   g->compiled = true;
   return B2VX_OK;
 }
 
-b2vx_status b2vx_graph_run_async(b2vx_graph* g) {
-  if (!g) return B2VX_INVALID_ARG;
-  b2vx_status st = b2vx_graph_compile(g);
-  if (st != B2VX_OK) return st;
+}  // extern "C"
+
+namespace {
+
+// Queues one pass.  to_host: the staged outputs come along, and tensors that can be are read and written over the bus;
+// otherwise the pass works on device memory alone and the outputs follow when they are read.
+// With to_host and every copied input written since the last run, the copies are part of the recorded plan (form 1: a
+// launch of their own costs 4 us of the 78 that a row through twelve 4096 x 4096 layers takes); otherwise those that are
+// needed go in front of it (forms 0 and 2).
+b2vx_status launch_plan(b2vx_graph* g, bool to_host) {
   DeviceGuard guard(g->device);
   g->idle = false;
-  if (g->use_cuda_graph && !g->exec && !g->capture_failed && !g->steps.empty()) {
+  set_io(g, to_host);
+  bool with_inputs = to_host;
+  for (uint32_t id : g->staged) with_inputs = with_inputs && (g->tensors[id].in_pending || !copied_in(g->tensors[id], true));
+  auto enqueue = [&]() -> b2vx_status {
+    for (uint32_t id : g->staged) {
+      const TensorRec& t = g->tensors[id];
+      if (with_inputs && copied_in(t, true)) CUDA_TRY(g, copy_staged(g, t.h_in, t.d_io, t.io_bytes));
+    }
+    for (Step& s : g->steps) {
+      const cudaError_t e = s.fn(g->stream);
+      if (e != cudaSuccess) return fail(g, B2VX_CUDA_ERROR, std::string(s.info.name) + ": " + cudaGetErrorString(e));
+    }
+    for (uint32_t id : g->staged) {
+      const TensorRec& t = g->tensors[id];
+      if (to_host && t.h_out && !t.over_bus) CUDA_TRY(g, copy_staged(g, t.d_io, t.h_out, t.io_bytes));
+    }
+    return B2VX_OK;
+  };
+  cudaGraphExec_t& exec = g->exec[!to_host ? 0 : with_inputs ? 1 : 2];
+  if (g->use_cuda_graph && !exec && !g->capture_failed && !g->steps.empty()) {
     // Record the plan once; on any failure fall back to launching kernel by kernel.
     cudaGraph_t graph = nullptr;
     bool ok = cudaStreamBeginCapture(g->stream, cudaStreamCaptureModeThreadLocal) == cudaSuccess;
     if (ok) {
-      for (auto& copy : g->copies_in) ok = ok && copy(g->stream) == cudaSuccess;
-      for (Step& s : g->steps) ok = ok && s.fn(g->stream) == cudaSuccess;
-      for (auto& copy : g->copies_out) ok = ok && copy(g->stream) == cudaSuccess;
+      ok = enqueue() == B2VX_OK;
       ok = (cudaStreamEndCapture(g->stream, &graph) == cudaSuccess) && ok && graph != nullptr;
     }
-    if (ok) ok = cudaGraphInstantiate(&g->exec, graph, 0) == cudaSuccess;
+    if (ok) ok = cudaGraphInstantiate(&exec, graph, 0) == cudaSuccess;
     if (graph) cudaGraphDestroy(graph);
     if (!ok) {
       cudaGetLastError();
-      g->exec = nullptr;
+      exec = nullptr;
       g->capture_failed = true;
     }
   }
-  if (g->exec) {
-    cudaError_t e = cudaGraphLaunch(g->exec, g->stream);
+  if (!with_inputs) CUDA_TRY(g, push_inputs(g, to_host));
+  if (exec) {
+    cudaError_t e = cudaGraphLaunch(exec, g->stream);
     if (e != cudaSuccess) return fail(g, B2VX_CUDA_ERROR, std::string("cudaGraphLaunch: ") + cudaGetErrorString(e));
-    return B2VX_OK;
+  } else {
+    const b2vx_status st = enqueue();
+    if (st != B2VX_OK) return st;
   }
-  for (auto& copy : g->copies_in) CUDA_TRY(g, copy(g->stream));
-  for (Step& s : g->steps) {
-    cudaError_t e = s.fn(g->stream);
-    if (e != cudaSuccess) {
-      return fail(g, B2VX_CUDA_ERROR, std::string(s.info.name) + ": " + cudaGetErrorString(e));
-    }
+  for (uint32_t id : g->staged) {
+    TensorRec& t = g->tensors[id];
+    if (with_inputs && copied_in(t, true)) t.in_pending = false;
+    t.out_behind = t.h_out != nullptr && !to_host;
   }
-  for (auto& copy : g->copies_out) CUDA_TRY(g, copy(g->stream));
   return B2VX_OK;
+}
+
+}  // namespace
+
+extern "C" {
+
+b2vx_status b2vx_graph_run_async(b2vx_graph* g) {
+  if (!g) return B2VX_INVALID_ARG;
+  b2vx_status st = b2vx_graph_compile(g);
+  if (st != B2VX_OK) return st;
+  return launch_plan(g, false);
 }
 
 b2vx_status b2vx_graph_sync(b2vx_graph* g) {
@@ -2238,7 +2324,9 @@ b2vx_status b2vx_graph_sync(b2vx_graph* g) {
 }
 
 b2vx_status b2vx_graph_run(b2vx_graph* g) {
-  b2vx_status st = b2vx_graph_run_async(g);
+  if (!g) return B2VX_INVALID_ARG;
+  b2vx_status st = b2vx_graph_compile(g);
+  if (st == B2VX_OK) st = launch_plan(g, !g->shared_stream);
   if (st != B2VX_OK) return st;
   return b2vx_graph_sync(g);
 }
@@ -2246,6 +2334,7 @@ b2vx_status b2vx_graph_run(b2vx_graph* g) {
 b2vx_status b2vx_graph_set_stream(b2vx_graph* g, void* cuda_stream) {
   if (!g) return B2VX_INVALID_ARG;
   DeviceGuard guard(g->device);
+  if (cuda_stream && !g->shared_stream && g->compiled) CUDA_TRY(g, share_staging(g));
   cudaStreamSynchronize(g->stream);
   g->idle = true;
   g->shared_stream = g->shared_stream || cuda_stream != nullptr;
@@ -2281,7 +2370,9 @@ b2vx_status b2vx_graph_print(b2vx_graph* g) {
 b2vx_status b2vx_graph_profile(b2vx_graph* g, uint32_t iters) {
   if (!g) return B2VX_INVALID_ARG;
   if (iters == 0) iters = 1;
-  b2vx_status st = b2vx_graph_run(g);   // warm-up
+  b2vx_status st = b2vx_graph_compile(g);
+  if (st == B2VX_OK) st = launch_plan(g, false);   // warm-up
+  if (st == B2VX_OK) st = b2vx_graph_sync(g);
   if (st != B2VX_OK) return st;
   DeviceGuard guard(g->device);
   std::vector<cudaEvent_t> ev(g->steps.size() + 1);
