@@ -82,7 +82,9 @@ def conv2d_q(W, H, C, N, kw, kh, Oc, stride=(1, 1), dilation=(1, 1), pad_type=B.
 
 
 def depthwise_q(W, H, C, N, kw, kh, multiplier=1, stride=(1, 1), pad_type=B.PAD_SAME, w_kind="u8", in_q=(0.03, 120),
-                out_q=(0.06, 0), relu6=True, x_dtype=B.DT_UINT8, pad=(0, 0, 0, 0)):
+                out_q=(0.06, 0), relu6=True, x_dtype=B.DT_UINT8, pad=(0, 0, 0, 0), out_dtype=B.DT_UINT8, w_zp=None, w_range=(0, 256),
+                bias=(-500, 501)):
+    """w_kind 's8pc': per-channel int8; else uint8 with values in w_range and zero point w_zp (None: drawn in [100,156])."""
     def build(g, rng):
         Oc = C * multiplier
         x = g.tensor(x_dtype, [W, H, C, N], B.ATTR_INPUT, scale=in_q[0], zero_point=in_q[1])
@@ -93,16 +95,16 @@ def depthwise_q(W, H, C, N, kw, kh, multiplier=1, stride=(1, 1), pad_type=B.PAD_
             w = g.tensor(B.DT_INT8, wshape, B.ATTR_CONSTANT, scales=ws, channel_dim=2, data=wd)
             bq = dict(scales=np.float32(in_q[0]) * ws, channel_dim=0)
         else:
-            zw = int(rng.integers(100, 157))
-            wd = rng.integers(0, 256, size=wshape[::-1]).astype(np.uint8)
+            zw = int(rng.integers(100, 157)) if w_zp is None else w_zp
+            wd = rng.integers(w_range[0], w_range[1], size=wshape[::-1]).astype(np.uint8)
             w = g.tensor(B.DT_UINT8, wshape, B.ATTR_CONSTANT, scale=0.02, zero_point=zw, data=wd)
             bq = dict(scale=float(np.float32(in_q[0]) * np.float32(0.02)), zero_point=0)
-        b = g.tensor(B.DT_INT32, [Oc], B.ATTR_CONSTANT, data=rng.integers(-500, 501, size=Oc).astype(np.int32), **bq)
-        y = g.tensor(B.DT_UINT8, [], B.ATTR_TRANSIENT if relu6 else B.ATTR_OUTPUT, scale=out_q[0], zero_point=out_q[1])
+        b = g.tensor(B.DT_INT32, [Oc], B.ATTR_CONSTANT, data=rng.integers(bias[0], bias[1], size=Oc).astype(np.int32), **bq)
+        y = g.tensor(out_dtype, [], B.ATTR_TRANSIENT if relu6 else B.ATTR_OUTPUT, scale=out_q[0], zero_point=out_q[1])
         g.conv2d(x, w, b, y, stride=stride, pad_type=pad_type, pad=pad, multiplier=multiplier)
         z = y
         if relu6:
-            z = g.tensor(B.DT_UINT8, [], B.ATTR_OUTPUT, scale=out_q[0], zero_point=out_q[1])
+            z = g.tensor(out_dtype, [], B.ATTR_OUTPUT, scale=out_q[0], zero_point=out_q[1])
             g.relu6(y, z)
         return [(x, _act(rng, [W, H, C, N], x_dtype))], [z]
     return build

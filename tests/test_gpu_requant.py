@@ -10,7 +10,7 @@ import pyb2vx as B
 pytestmark = pytest.mark.gpu
 
 
-def conv1x1(C, Oc, N, W, out_scale, zp=0, w_scale=0.01, w_zp=None, spread=255, out_dtype=B.DT_UINT8, residual=False):
+def conv1x1(C, Oc, N, W, out_scale, zp=0, w_scale=0.01, w_zp=None, spread=255, out_dtype=B.DT_UINT8, residual=False, bias=(-3000, 3001)):
     """1x1 convolution on [W, W, C, N]; w_zp None: int8 kernel, per-tensor scale; else uint8 with `spread` values about w_zp."""
     def build(g, rng):
         x = g.tensor(B.DT_UINT8, [W, W, C, N], B.ATTR_INPUT, scale=0.02, zero_point=7)
@@ -22,7 +22,7 @@ def conv1x1(C, Oc, N, W, out_scale, zp=0, w_scale=0.01, w_zp=None, spread=255, o
             w = g.tensor(B.DT_UINT8, [1, 1, C, Oc], B.ATTR_CONSTANT, scale=w_scale, zero_point=w_zp,
                          data=rng.integers(lo, hi + 1, size=(Oc, C, 1, 1)).astype(np.uint8))
         b = g.tensor(B.DT_INT32, [Oc], B.ATTR_CONSTANT, scale=float(np.float32(0.02) * np.float32(w_scale)), zero_point=0,
-                     data=rng.integers(-3000, 3001, size=Oc).astype(np.int32))
+                     data=rng.integers(bias[0], bias[1], size=Oc).astype(np.int32))
         y = g.tensor(out_dtype, [], B.ATTR_TRANSIENT if residual else B.ATTR_OUTPUT, scale=out_scale, zero_point=zp)
         g.conv2d(x, w, b, y, pad_type=B.PAD_VALID)
         inputs = [(x, rng.integers(0, 256, size=(N, C, W, W)).astype(np.uint8))]
@@ -58,4 +58,21 @@ def test_fixed_point_requantization(product_lib, oracle_lib, name):
     want, _ = G.run_case(oracle_lib, CASES[name], 11)
     got, kernels = G.run_case(product_lib, CASES[name], 11)
     assert any(k["name"].startswith("gemm_i8_tc") for k in kernels)
+    G.assert_same(want, got)
+
+
+# The sum of accumulator and bias wraps in 32 bits for some elements of every channel and for others not: the wrapped sum
+# counts, like in the reference's integer arithmetic, and 64-bit intermediates must not hide it.
+NEAR_2_31 = (2**31 - 60000, 2**31)
+WRAP = {
+    "conv": conv1x1(32, 48, 1, 13, 4000.0, zp=128, bias=NEAR_2_31),
+    "depthwise": G.depthwise_q(17, 9, 48, 2, 3, 3, w_kind="u8", in_q=(0.03, 0), out_q=(12000.0, 128), relu6=False, w_zp=128, bias=NEAR_2_31),
+}
+
+
+@pytest.mark.parametrize("name", sorted(WRAP))
+def test_accumulator_and_bias_wrap(product_lib, oracle_lib, name):
+    want, _ = G.run_case(oracle_lib, WRAP[name], 13)
+    got, _ = G.run_case(product_lib, WRAP[name], 13)
+    assert {int(v) for v in np.unique(want[0])} >= {128 - 107, 128 + 107}   # both sides of the wrap
     G.assert_same(want, got)

@@ -583,7 +583,8 @@ bool weights_fit_s8(const TensorRec& w, int Oc) {
 
 // Per-channel constants of the fixed-point requantization (requant_fixed4).  acc_max bounds the
 // accumulators; blocks of blk_w channels, counted from the start of each tile of tile_data, share a window.  Returns false
-// when a channel does not allow it (every element then takes the exact sequence).
+// when a channel does not allow it (every element then takes the exact sequence).  So does one whose bias can carry the
+// accumulator past 32 bits: the reference's sum wraps there, the 64-bit one would not.
 bool fixed_point_columns(const std::vector<int32_t>& bias_full, const std::vector<float>& acc_scale, const OutQuant& out, double acc_max,
                          int tile_data, int blk_w, std::vector<FixedColumn>* cols, int* shl) {
   const size_t n = acc_scale.size();
@@ -593,7 +594,8 @@ bool fixed_point_columns(const std::vector<int32_t>& bias_full, const std::vecto
   double r_max = 0.0;
   for (size_t c = 0; c < n; ++c) {
     r[c] = static_cast<double>(acc_scale[c]) / static_cast<double>(out.scale) * two32;
-    if (!(r[c] >= 0.0 && std::fabs(static_cast<double>(bias_full[c])) * r[c] < 1e18)) return false;
+    const double bias = std::fabs(static_cast<double>(bias_full[c]));
+    if (!(r[c] >= 0.0 && bias * r[c] < 1e18) || acc_max + bias >= 2147483648.0) return false;
     r_max = std::max(r_max, r[c]);
   }
   int k = 0;
