@@ -581,59 +581,107 @@ bool weights_fit_s8(const TensorRec& w, int Oc) {
   return true;
 }
 
-// Per-channel constants of the fixed-point requantization (requant_fixed4).  acc_max bounds the
-// accumulators; blocks of blk_w channels, counted from the start of each tile of tile_data, share a window.  Returns false
-// when a channel does not allow it (every element then takes the exact sequence).  So does one whose bias can carry the
-// accumulator past 32 bits: the reference's sum wraps there, the 64-bit one would not.
-bool fixed_point_columns(const std::vector<int32_t>& bias_full, const std::vector<float>& acc_scale, const OutQuant& out, double acc_max,
-                         int tile_data, int blk_w, std::vector<FixedColumn>* cols, int* shl) {
+// Bound of each channel's |accumulator|, the sum over its weights of x * (w - zero point) with any x of the input's type,
+// its zero point and the zeros of padding among them: from the number of weights alone, or from their values (a pass over
+// the kernel, for layers whose other bound is too coarse).
+std::vector<double> accumulator_bounds(const TensorRec& x, const TensorRec& w, int Oc, int Ocp, bool from_values) {
+  const bool u8 = w.d.dtype == B2VX_DT_UINT8, per_ch = w.d.quant_type == B2VX_QUANT_SYMMETRIC_PER_CHANNEL, xs = x.d.dtype == B2VX_DT_INT8;
+  const double x_lo = std::min({xs ? -128 : 0, x.zp(), 0}), x_hi = std::max({xs ? 127 : 255, x.zp(), 0});
+  const size_t per_oc = w.elems() / Oc;
+  std::vector<double> bound(Ocp, 0.0);
+  for (int oc = 0; oc < Oc; ++oc) {
+    const int zw = per_ch ? (w.zps.empty() ? 0 : w.zps[oc]) : w.zp();
+    double pos, neg;   // sums of the positive and of the negative w - zero point
+    if (from_values) {
+      const uint8_t* row = w.host.data() + static_cast<size_t>(oc) * per_oc;
+      int64_t up = 0, down = 0;
+      for (size_t i = 0; i < per_oc; ++i) {
+        const int v = (u8 ? static_cast<int>(row[i]) : static_cast<int>(static_cast<int8_t>(row[i]))) - zw;
+        up += std::max(v, 0);
+        down += std::min(v, 0);
+      }
+      pos = static_cast<double>(up);
+      neg = static_cast<double>(down);
+      bound[oc] = std::max(x_hi * pos + x_lo * neg, -(x_lo * pos + x_hi * neg));
+    } else {
+      const double w_abs = std::max(std::abs((u8 ? 0 : -128) - zw), std::abs((u8 ? 255 : 127) - zw));
+      bound[oc] = static_cast<double>(per_oc) * w_abs * std::max(-x_lo, x_hi);
+    }
+  }
+  return bound;
+}
+
+// Per-channel constants of the fixed-point requantization (requant_fixed4).  acc_max bounds the accumulators of each
+// channel; blocks of blk_w channels, counted from the start of each tile of tile_data, share a window.  A block with a channel that does
+// not allow it is marked for the exact sequence (window 0xFFFFFFFF); returns the number of channels in such blocks.
+// Not allowed are negative or huge scales, and a bias that can carry the accumulator past 32 bits: the reference's sum
+// wraps there, the 64-bit one would not.
+size_t fixed_point_columns(const std::vector<int32_t>& bias_full, const std::vector<float>& acc_scale, const OutQuant& out,
+                           const std::vector<double>& acc_max, int tile_data, int blk_w, std::vector<FixedColumn>* cols, int* shl) {
   const size_t n = acc_scale.size();
-  const double two32 = 4294967296.0;
-  if (!(out.scale > 5.5e-20f && out.scale < 1.8e19f)) return false;   // requant_near_half
-  std::vector<double> r(n);   // acc_scale / out scale in units of 2^-32
+  const double two31 = 2147483648.0, two32 = 4294967296.0;
+  *shl = 0;
+  if (!(out.scale > 5.5e-20f && out.scale < 1.8e19f) || out.zp < -1000000 || out.zp > 1000000) return n;   // requant_near_half; 64 bits
+  std::vector<double> r(n), most(n);   // acc_scale / out scale in units of 2^-32 (below 0: not allowed); largest |accumulator + bias|
   double r_max = 0.0;
   for (size_t c = 0; c < n; ++c) {
     r[c] = static_cast<double>(acc_scale[c]) / static_cast<double>(out.scale) * two32;
     const double bias = std::fabs(static_cast<double>(bias_full[c]));
-    if (!(r[c] >= 0.0 && bias * r[c] < 1e18) || acc_max + bias >= 2147483648.0) return false;
+    most[c] = acc_max[c] + bias;
+    if (!(r[c] >= 0.0 && bias * r[c] < 1e18) || r[c] >= 2147483000.0 * (1 << 20) || most[c] >= two31) r[c] = -1.0;
     r_max = std::max(r_max, r[c]);
   }
   int k = 0;
-  while (k < 20 && r_max / (1 << k) >= 2147483000.0) ++k;
-  if (!(r_max / (1 << k) < 2147483000.0) || acc_max * (1 << k) >= 2147483647.0) return false;
+  while (r_max / (1 << k) >= 2147483000.0) ++k;
   *shl = k;
   // |real / scale| of an output that does not saturate, and the middle of its range
   const double top = std::max(out.hi - out.zp, out.zp - out.lo) + 1.0, half = 0.5 * (out.hi - out.lo) + 1.0, mid = 0.5 * (out.hi + out.lo) - out.zp;
+  size_t exact = 0;
   cols->resize(n);
+  std::vector<double> centre(tile_data);
   for (size_t tile = 0; tile < n; tile += tile_data) {
     const size_t tile_end = std::min(n, tile + tile_data);
     for (size_t c0 = tile; c0 < tile_end; c0 += blk_w) {
       const size_t c1 = std::min(tile_end, c0 + blk_w);
       double w = 0.0;
       for (size_t c = c0; c < c1; ++c) {
+        FixedColumn& f = (*cols)[c];
+        f.mul = 0;
+        centre[c - c0] = 0.0;
+        if (r[c] < 0.0 || acc_max[c] * (1 << k) >= 2147483647.0) { w = 1.0; break; }
+        // what |real / scale| can reach at all; a channel that cannot leave the zero point needs no multiplier
+        const double reach = most[c] * r[c] / two32;
+        if (reach < 0.49) continue;
         const double mul = std::nearbyint(r[c] / (1 << k));
-        (*cols)[c].mul = static_cast<int32_t>(mul);
-        if (r[c] == 0.0) continue;
+        f.mul = static_cast<int32_t>(mul);
         // what the rounding of the multiplier costs over the range, once its value at the middle has gone into the addend;
         // and what the reference rounds: product and quotient (half an ulp each), an accumulator beyond 2^24 when it
         // becomes a float.  (The addition in its floor(|x| + 0.5f) moves no result across an integer except just below
         // x = 0.5, by less than 2^-24.)
-        const double err = std::fabs(r[c] - mul * (1 << k)) / r[c] * half;
-        const double ref = top * (top * two32 < r[c] * 16777216.0 ? 2.02 : 3.03) / 16777216.0 + 1.0 / 8388608.0;
-        w = std::max(w, err + ref);
+        const double lost = (r[c] - mul * (1 << k)) / r[c];
+        double y_lo = std::max(mid - half, -reach), y_hi = std::min(mid + half, reach);
+        if (y_lo > y_hi) y_lo = y_hi = mid < 0.0 ? -reach : reach;   // saturates always: exact at the end next to the range
+        const double t = std::min(top, reach);
+        const double ref = t * (t * two32 < r[c] * 16777216.0 ? 2.02 : 3.03) / 16777216.0 + 1.0 / 8388608.0;
+        w = std::max(w, std::fabs(lost) * 0.5 * (y_hi - y_lo) + ref);
+        centre[c - c0] = lost * 0.5 * (y_hi + y_lo) * two32;
       }
-      if (!(w < 0.25)) return false;
+      const bool fixed = w < 0.25;
       const int64_t half_window = static_cast<int64_t>(w * two32) + 4;
       for (size_t c = c0; c < c1; ++c) {
         FixedColumn& f = (*cols)[c];
-        const double centre = r[c] > 0.0 ? (r[c] - static_cast<double>(f.mul) * (1 << k)) / r[c] * mid * two32 : 0.0;
-        f.add = (static_cast<int64_t>(bias_full[c]) << k) * f.mul + (static_cast<int64_t>(out.zp - out.lo) << 32) + (int64_t(1) << 31) +
-                half_window + std::llround(centre);
+        if (!fixed) {
+          f = FixedColumn{0, 0, 0xFFFFFFFFu};
+          ++exact;
+          continue;
+        }
+        f.add = static_cast<int64_t>(bias_full[c]) * (int64_t(1) << k) * f.mul + (static_cast<int64_t>(out.zp - out.lo) * (int64_t(1) << 32)) + (int64_t(1) << 31) +
+                half_window + std::llround(centre[c - c0]);
         f.window = static_cast<uint32_t>(2 * half_window);
       }
     }
   }
-  return true;
+  return exact;
 }
 
 // Weight element (kx,ky,ic,oc) of a WHIcOc kernel as a signed value together
@@ -979,11 +1027,16 @@ b2vx_status plan_contraction(b2vx_graph* g, uint32_t node_index, const char* lab
     {
       std::vector<FixedColumn> fix;
       FixedColumn* dfix = nullptr;
-      // raw accumulators, the S term and the border corrections each stay below taps * channels * 255 * 128 * 2
-      if (fixed_point_columns(pk.bias_full, pk.acc_scale, ep.out, 4.0 * taps * x.C * 255 * 128, tiling.data, tiling.blk_w, &fix, &ep.fix_shl)) {
+      size_t exact = 1;
+      for (int from_values = 0; from_values < 2 && exact; ++from_values)
+        exact = fixed_point_columns(pk.bias_full, pk.acc_scale, ep.out, accumulator_bounds(x, w, y.C, y.Cp, from_values != 0), tiling.data, tiling.blk_w, &fix,
+                                    &ep.fix_shl);
+      if (exact < pk.acc_scale.size()) {
         st = upload(g, fix, &dfix);
         if (st != B2VX_OK) return st;
         ep.fix = dfix;
+      } else {
+        ep.fix_shl = 0;
       }
     }
     void* fused_out = nullptr;
@@ -1205,7 +1258,7 @@ b2vx_status plan_conv(b2vx_graph* g, uint32_t idx, NodeRec& n) {
       for (int t = 0; t < taps; ++t) bfull[oc] -= zx * wd[static_cast<size_t>(t) * y.Cp + oc];
     std::vector<FixedColumn> fix;
     int shl = 0;
-    if (fixed_point_columns(bfull, sc, oq, 9.0 * 255 * 128 * 4, y.Cp, 16, &fix, &shl)) {
+    if (fixed_point_columns(bfull, sc, oq, accumulator_bounds(x, w, y.C, y.Cp, false), y.Cp, 16, &fix, &shl) == 0) {
       int8_t* dw8 = nullptr; FixedColumn* dfix = nullptr; int32_t* dbf = nullptr;
       st = upload(g, w8, &dw8);
       if (st == B2VX_OK) st = upload(g, fix, &dfix);
