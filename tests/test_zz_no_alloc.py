@@ -79,12 +79,12 @@ def entry_point(product_lib):
     return fn
 
 
-def run_problem(product_lib, oracle_lib, p, seed, calls, stream=None):
+def run_problem(product_lib, oracle_lib, p, seed, calls, stream=None, wscale=None):
     import torch
     fn = entry_point(product_lib)
     rng = np.random.default_rng(seed)
     weights = rng.integers(-127, 128, size=(p.oc, p.c, p.kh, p.kw)).astype(np.int8)
-    wscales = rng.uniform(0.001, 0.01, p.oc).astype(np.float32)
+    wscales = rng.uniform(0.001, 0.01, p.oc).astype(np.float32) if wscale is None else np.full(p.oc, wscale, np.float32)
     bias = rng.integers(-1000, 1001, size=p.oc).astype(np.int32)
     images = [rng.integers(0, 256, size=(p.n, p.c, p.h, p.w)).astype(np.uint8) for _ in range(calls)]
     # operands in the layout the entry point documents; every device buffer is made here, once
@@ -147,3 +147,11 @@ def test_noalloc_conv_equals_graph_conv_and_oracle(product_lib, oracle_lib):
         err.value = b""
         assert fn(C.byref(bad), *args, err, len(err)) == 1 and err.value, field
     assert fn(C.byref(desc), None, *args[1:], err, len(err)) == 1 and b"null" in err.value
+
+
+# (out_scale, out_zp, weight scale) of a 1x1 filter: every other accumulator on an exact half; halves around zero; an output
+# scale below the range in which quotients near a half are decided without a division, and one above it
+@pytest.mark.parametrize("out_scale,out_zp,wscale", [(1.0, 0, 0.5), (256.0, 128, 1.0), (1e-21, 7, 1e-22), (3e19, 200, 1e16)])
+def test_noalloc_requantization(product_lib, oracle_lib, out_scale, out_zp, wscale):
+    p = Problem(1, 23, 31, 3, 1, 1, 40, (1, 1), (1, 1), (0, 0, 0, 0), 1.0, 100, out_scale, out_zp)
+    run_problem(product_lib, oracle_lib, p, 7, calls=1, wscale=wscale)

@@ -289,10 +289,30 @@ __device__ __forceinline__ uint32_t requant_near_half(float real, int hi, const 
   return static_cast<uint32_t>(hi - (down ? 1 : 0));
 }
 
+// Four columns without fixed-point constants, as q - lo.  The product with 1 / scale lies within 2^-11 of the reference's
+// quotient wherever the output does not saturate (|zero point| <= 1000); only next to a half does that leave two answers,
+// and requant_near_half decides.
+static __device__ __noinline__ uint32_t requant_exact4(int a0, int a1, int a2, int a3, int4 b, float4 s, OutQuant oq) {
+  const float real[4] = {__fmul_rn(__int2float_rn(a0 + b.x), s.x), __fmul_rn(__int2float_rn(a1 + b.y), s.y),
+                         __fmul_rn(__int2float_rn(a2 + b.z), s.z), __fmul_rn(__int2float_rn(a3 + b.w), s.w)};
+  const bool plain = oq.scale > 5.5e-20f && oq.scale < 1.8e19f && abs(oq.zp) <= 1000;
+  const float inv = __frcp_rn(oq.scale), bias = __int2float_rn(oq.zp - oq.lo) + (0.5f + 0.0009765625f);
+  int q[4];
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    const float u = fminf(fmaxf(__fadd_rn(__fmul_rn(real[k], inv), bias), -1.0f), 257.0f);   // a NaN becomes -1 and is replayed below
+    q[k] = __float2int_rd(u);
+    if (!plain || !(real[k] == real[k])) q[k] = static_cast<int>(requant_replay(real[k], oq.scale, oq.zp, oq.lo, oq.hi));
+    else if (u - __int2float_rn(q[k]) < 0.001953125f && static_cast<uint32_t>(q[k] - 1) < 255u) q[k] = static_cast<int>(requant_near_half(real[k], q[k], oq));
+  }
+  return pack_sat_u8(q[1], q[0], pack_sat_u8(q[3], q[2], 0u));
+}
+
 // Those of four columns whose fraction lies in the window, unless the integers on both sides saturate to the same result.
 // Not inlined: sixteen copies of it cost the common path registers and instruction cache.
 static __device__ __noinline__ uint32_t requant_redo4(uint32_t word, int a0, int a1, int a2, int a3, const FixedColumns* cols, int c, uint32_t window,
                                                int shl, OutQuant oq) {
+  if (window == 0xFFFFFFFFu) return requant_exact4(a0, a1, a2, a3, *reinterpret_cast<const int4*>(&cols->bias[c]), *reinterpret_cast<const float4*>(&cols->scale[c]), oq);
   const int4 m = *reinterpret_cast<const int4*>(&cols->mul[c]);
   const longlong2 a01 = *reinterpret_cast<const longlong2*>(&cols->add[c]), a23 = *reinterpret_cast<const longlong2*>(&cols->add[c + 2]);
   const long long v0 = mad_wide(a0 << shl, m.x, a01.x), v1 = mad_wide(a1 << shl, m.y, a01.y);
@@ -305,12 +325,9 @@ static __device__ __noinline__ uint32_t requant_redo4(uint32_t word, int a0, int
     hits &= hits - 1;
     const int acc = k & 2 ? (k & 1 ? a3 : a2) : (k & 1 ? a1 : a0);
     const int hi = static_cast<int>((k & 2 ? (k & 1 ? v3 : v2) : (k & 1 ? v1 : v0)) >> 32);
+    if (static_cast<uint32_t>(hi - 1) >= 255u) continue;
     const float real = __fmul_rn(__int2float_rn(acc + cols->bias[c + k]), cols->scale[c + k]);
-    uint32_t q;
-    if (window == 0xFFFFFFFFu) q = requant_replay(real, oq.scale, oq.zp, oq.lo, oq.hi);   // no fixed-point constants
-    else if (static_cast<uint32_t>(hi - 1) < 255u) q = requant_near_half(real, hi, oq);
-    else continue;
-    word = (word & ~(0xFFu << (8 * k))) | (q << (8 * k));
+    word = (word & ~(0xFFu << (8 * k))) | requant_near_half(real, hi, oq) << (8 * k);
   }
   return word;
 }
