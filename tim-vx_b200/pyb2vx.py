@@ -7,6 +7,7 @@ tim::vx order (shape listed fastest dimension first, i.e. the reversed numpy
 shape of a C-contiguous array).
 """
 import ctypes as C
+import math
 import os
 
 import numpy as np
@@ -288,9 +289,9 @@ class Graph:
         l = self._layout.get(tid)
         if l is None:
             d = self.desc(tid)
-            dims = tuple(int(d.dims[i]) for i in range(d.rank))[::-1]
+            dims = tuple(d.dims[:d.rank][::-1])
             dtype = np.dtype(NP_DTYPE[d.dtype])
-            l = (int(np.prod(dims, dtype=np.int64)) * dtype.itemsize, dtype, dims)
+            l = (math.prod(dims) * dtype.itemsize, dtype, dims)
             if self._compiled:
                 self._layout[tid] = l
         return l
