@@ -1248,9 +1248,11 @@ b2vx_status plan_conv(b2vx_graph* g, uint32_t idx, NodeRec& n) {
   void* ycl = y.d_cl;
   const int xs = x.d.dtype == B2VX_DT_INT8, zx = x.zp(), mult = c.multiplier;
   const OutQuant oq = out_quant(y);
-  // The tensor-instruction form; B2VX_DW_MMA=0 (or a switch that asks for one of the dp2a forms) turns it off.
+  // The tensor-instruction form; B2VX_DW_MMA=0 (or a switch that asks for one of the dp2a forms: B2VX_DW_STRIP=0, B2VX_DW_PIPE)
+  // turns it off.
   const bool padded = n.pad[0] || n.pad[1] || n.pad[2] || n.pad[3];
-  const bool want_mma = g->use_tc && !std::getenv("B2VX_DW_STRIP") && !std::getenv("B2VX_DW_PIPE") && !(std::getenv("B2VX_DW_MMA") && std::getenv("B2VX_DW_MMA")[0] == '0');
+  auto off = [](const char* name) { const char* v = std::getenv(name); return v && v[0] == '0'; };
+  const bool want_mma = g->use_tc && !off("B2VX_DW_MMA") && !off("B2VX_DW_STRIP") && !std::getenv("B2VX_DW_PIPE");
   if (want_mma && mult == 1 && kh == 3 && kw == 3 && !(padded && zx != 0) && weights_fit_s8(w, y.C)) {
     std::vector<int8_t> w8(wd.begin(), wd.end());
     std::vector<int32_t> bfull(bv);
