@@ -31,7 +31,7 @@ struct OutQuant {
 
 // Constants of one output channel for requant_fixed4: the multiplier acc_scale / out.scale in units of 2^(fix_shl - 32);
 // bias, zero point, rounding half and half the window folded into one addend; the window of the column block the channel
-// lies in (results with a smaller fraction are redone exactly).
+// lies in (results with a smaller fraction are redone exactly; 0xFFFFFFFF, with the rest 0: all of the block's are).
 struct alignas(16) FixedColumn {
   long long add;
   int32_t mul;

@@ -429,8 +429,8 @@ __global__ void __launch_bounds__(256, 2) depthwise_q16_kernel(const uint8_t* __
   }
   const RequantConsts rc = make_requant_consts(p.out, p.exact_only);
   uint8_t* out = y + ((static_cast<size_t>(n) * g.Ho + ho) * g.Wo + wo0) * g.Ocp + c0;
-  *reinterpret_cast<uint4*>(out) = requant_chunk16<false>(acc0, p.bias_full + c0, p.acc_scale + c0, rc, 0, nullptr);
-  if (second) *reinterpret_cast<uint4*>(out + g.Ocp) = requant_chunk16<false>(acc1, p.bias_full + c0, p.acc_scale + c0, rc, 0, nullptr);
+  *reinterpret_cast<uint4*>(out) = requant_chunk16(acc0, p.bias_full + c0, p.acc_scale + c0, rc);
+  if (second) *reinterpret_cast<uint4*>(out + g.Ocp) = requant_chunk16(acc1, p.bias_full + c0, p.acc_scale + c0, rc);
 }
 
 // The same computation with the input staged in shared memory: a block owns a slab of CK = 1, 2 or 4
@@ -515,9 +515,9 @@ __global__ void __launch_bounds__(256, (KH == 3 ? 3 : 2)) depthwise_q16s_kernel(
   const int ho = ho0 + tr, wo = wo0 + tc, c0 = c_slab + 16 * chunk;
   if (ho >= g.Ho) return;
   uint8_t* out = y + ((static_cast<size_t>(n) * g.Ho + ho) * g.Wo + wo) * g.Ocp + c0;
-  if (wo < g.Wo) *reinterpret_cast<uint4*>(out) = requant_chunk16<false>(acc0, p.bias_full + c0, p.acc_scale + c0, rc, 0, nullptr);
+  if (wo < g.Wo) *reinterpret_cast<uint4*>(out) = requant_chunk16(acc0, p.bias_full + c0, p.acc_scale + c0, rc);
   if (two && wo + 8 < g.Wo)
-    *reinterpret_cast<uint4*>(out + 8 * g.Ocp) = requant_chunk16<false>(acc1, p.bias_full + c0, p.acc_scale + c0, rc, 0, nullptr);
+    *reinterpret_cast<uint4*>(out + 8 * g.Ocp) = requant_chunk16(acc1, p.bias_full + c0, p.acc_scale + c0, rc);
 }
 
 // The 3x3 form for strides 1 and 2: a thread owns FOUR channels (one 32-bit word of a pixel) of a strip of eight

@@ -148,7 +148,7 @@ __device__ __forceinline__ uint32_t pack_sat_s8(int hi, int lo, uint32_t upper) 
 // far inside the range where adding 1.5*2^23 leaves the integer in the low mantissa bits.
 #define B2VX_FAST_ROUND_LIMIT 2097152.0f   /* 2^21 */
 
-// Requantization of one 16-column chunk of an accumulator row: acc + folded bias -> float ->
+// Requantization of sixteen neighbouring channels (depthwise kernels on CUDA cores): acc + folded bias -> float ->
 // * accumulator scale -> quantized bytes (the exact sequence is requant() in requant.cuh).
 //
 // Fast form.  The reference computes q = R(real / scale) + zp with R = round-half-even except within an
@@ -195,24 +195,11 @@ __device__ __forceinline__ RequantConsts make_requant_consts(const OutQuant& oq,
   return rc;
 }
 
-// EXTRA: the row has a term to subtract from every accumulator (sub = dz * S of this row) and/or a
-// border correction (corr: 16 values for this chunk's channels, or null); without EXTRA both are
-// ignored.  A template parameter because as run-time conditions they were compiled into instructions
-// every chunk pays for.
-template <bool EXTRA>
-__device__ __forceinline__ uint4 requant_chunk16(const int (&acc)[16], const int* bias, const float* scale,
-                                                 const RequantConsts& rc, int sub, const int32_t* corr) {
+__device__ __forceinline__ uint4 requant_chunk16(const int (&acc)[16], const int* bias, const float* scale, const RequantConsts& rc) {
   f32x2 real[8];
 #pragma unroll
   for (int g4 = 0; g4 < 4; ++g4) {
-    int4 b4 = *reinterpret_cast<const int4*>(bias + g4 * 4);
-    if (EXTRA) {
-      b4.x -= sub; b4.y -= sub; b4.z -= sub; b4.w -= sub;
-      if (corr) {
-        const int4 c4 = __ldg(reinterpret_cast<const int4*>(corr + g4 * 4));
-        b4.x += c4.x; b4.y += c4.y; b4.z += c4.z; b4.w += c4.w;
-      }
-    }
+    const int4 b4 = *reinterpret_cast<const int4*>(bias + g4 * 4);
     const float4 s4 = *reinterpret_cast<const float4*>(scale + g4 * 4);
     real[2 * g4] = f2_mul(f2_pack(__int2float_rn(acc[g4 * 4 + 0] + b4.x), __int2float_rn(acc[g4 * 4 + 1] + b4.y)), f2_pack(s4.x, s4.y));
     real[2 * g4 + 1] = f2_mul(f2_pack(__int2float_rn(acc[g4 * 4 + 2] + b4.z), __int2float_rn(acc[g4 * 4 + 3] + b4.w)), f2_pack(s4.z, s4.w));
@@ -252,7 +239,7 @@ __device__ __forceinline__ uint4 requant_chunk16(const int (&acc)[16], const int
 //     P = acc * M + A          high word = floor(acc * r + bias * r + zp - lo + 1/2 + W),  low word = its fraction,
 // costs one multiply-add per element; the high words go straight into the saturating pack.  W bounds how far P and the
 // reference's float quotient (two or three roundings) can lie apart wherever the output does not saturate.  A fraction
-// of 2 W (the window of the 16 columns) or more says that no half-integer lies between the two: the high word is then
+// of 2 W (the window of the block of columns) or more says that no half-integer lies between the two: the high word is then
 // the reference's answer, its tie rule included.  The few elements below (2 W is about 1e-4) are redone exactly.
 // Per element: one multiply-add (2.65 cycles of an SM scheduler measured, 2 for most other integer instructions), half a
 // pack, half a three-input minimum.  The form with two packed float products that it replaced took an addition, an
@@ -264,7 +251,7 @@ struct FixedColumns {                // one N tile, in the order the epilogue th
   alignas(16) long long add[256];
   alignas(16) int bias[256];         // for the exact sequence: folded bias and accumulator scale
   alignas(16) float scale[256];
-  uint32_t window[16];               // per 16 columns
+  uint32_t window[16];               // per 16 columns in reading order; the same throughout a block (GemmTcTiling::blk_w)
 };
 
 static __device__ __noinline__ uint32_t requant_replay(float real, float scale, int zp, int lo, int hi) {
@@ -274,8 +261,10 @@ static __device__ __noinline__ uint32_t requant_replay(float real, float scale, 
 
 // The reference's answer (as q - lo) where requant_fixed4 left it between hi and hi - 1.  With n the integer above the
 // half b = n - 1/2 in question, the reference compares x = real / scale, rounded, with b.  e = real - b * scale is exact
-// in one fused operation (both lie within 2^-9 scale of each other, on a grid of 2^-24 scale or coarser), and x rounds
-// to b itself exactly when |e| is at most half an ulp of b times the scale; then the even neighbour wins.  Next to 1/2,
+// in one fused operation: with 2^E <= scale < 2^(E+1), both terms are multiples of 2^(E-24) (|b| >= 3/2 has its last bit
+// at 1/2, and real is as large as b * scale within the window), and they differ by less than 2^E, half the scale at most
+// (windows stay below 1/2).  x rounds to b itself exactly when |e| is at most half an ulp of b times the scale; then the
+// even neighbour wins.  Next to 1/2,
 // where x + 0.5f rounds too, the sequence is replayed.  About a dozen instructions instead of the division's hundred:
 // one thread in a warp of a short-K layer takes this path every few blocks, and the other threads wait for it.
 // out.scale between 2^-64 and 2^64 (checked when the constants are made), 0 < hi < 256.
