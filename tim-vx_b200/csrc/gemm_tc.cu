@@ -271,16 +271,18 @@ struct SmemHeader {
   FixedColumns cols;                 // this CTA's N tile
 };
 
-// EXTRA: rows carry a weight-zero-point term (p.dz, S column) and/or border corrections
-// (p.ep.border_corr), or the fixed-point multipliers had to be halved (p.ep.fix_shl); the plain form contains no code
-// for any of these.
+// EXTRA: 2: rows carry a weight-zero-point term (p.dz, S column) and/or border corrections (p.ep.border_corr); 1 and 2: the
+// fixed-point multipliers may have been halved (p.ep.fix_shl) and the output may be int8; 0 contains no code for any of these.
+// (1 is a form of its own because half of MobileNetV2's expanding layers have halved multipliers and nothing else, and every
+// subtraction and test costs a short-K layer, which the epilogue bounds, its share: at batch 1024, 24 -> 144 at 56 x 56 340 -> 252 us,
+// 32 -> 192 at 28 x 28 107 -> 81; without the exclusive or for int8 outputs 16 -> 96 at 112 x 112 640 -> 500.)
 // FUSE: a residual Add follows the convolution and is done here: the 64 KB table of that Add sits in
 // shared memory behind the operand ring, the epilogue loads the residual's bytes beside its own
 // and stores the table's answers instead.
 // STEPS: column blocks of 16 * STEPS (1, 2 or 4) columns.  A template parameter because small layers are bound by
 // instruction fetch (a launch executes every line of the kernel about once per warp): code for the other widths in the
 // same kernel costs them.
-template <bool EXTRA, bool FUSE, int STEPS>
+template <int EXTRA, bool FUSE, int STEPS>
 __global__ void __launch_bounds__(kThreadsTc, 1)
 gemm_i8_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                   const __grid_constant__ CUtensorMap map_r, const GemmParams p) {
@@ -632,7 +634,7 @@ gemm_i8_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
     const int row_in_tile = quarter * 32 + lane;
     const int g = lane >> 2, q = lane & 3;        // this thread's rows are g + 8 k of the warp's 32, its columns the q-th quarter of a block
     const OutQuant oq = p.ep.out;
-    const uint32_t out_flip = oq.lo < 0 ? 0x80808080u : 0u;
+    const uint32_t out_flip = EXTRA && oq.lo < 0 ? 0x80808080u : 0u;
     const int shl = EXTRA ? p.ep.fix_shl : 0;
     const int nblk = p.BNd / w;
     const int blk0 = p.teams ? 0 : col_group * p.blk_per_group, blk1 = p.teams ? nblk : min(nblk, blk0 + p.blk_per_group);
@@ -648,7 +650,7 @@ gemm_i8_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
       const int wo = tw * p.TW + i, ho = th * p.TH + jh, n = tn * p.TN + l;
       if (l < p.TN && wo < p.Wo && ho < p.Ho && n < p.Nimg) {
         row = (n * p.Ho + ho) * p.Wo + wo;
-        if (EXTRA && p.ep.border_corr) cls = __ldg(p.ep.row_class + ho) * p.ep.n_col_classes + __ldg(p.ep.col_class + wo);
+        if (EXTRA == 2 && p.ep.border_corr) cls = __ldg(p.ep.row_class + ho) * p.ep.n_col_classes + __ldg(p.ep.col_class + wo);
       }
     };
     bool alive = true;
@@ -666,7 +668,7 @@ gemm_i8_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
           row[k] = __shfl_sync(0xffffffffu, my_row, g + 8 * k);
-          cls[k] = EXTRA ? __shfl_sync(0xffffffffu, my_cls, g + 8 * k) : 0;
+          cls[k] = EXTRA == 2 ? __shfl_sync(0xffffffffu, my_cls, g + 8 * k) : 0;
         }
       } else {
 #pragma unroll
@@ -697,7 +699,7 @@ gemm_i8_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
       tc_fence_after();
       const uint32_t taddr = tmem_base + a * p.acc_stride + (static_cast<uint32_t>(quarter * 32) << 16);
       int sub[4] = {0, 0, 0, 0};
-      if (EXTRA && p.dz != 0) {
+      if (EXTRA == 2 && p.dz != 0) {
         // S = sum of a row's inputs: the accumulator column of the all-ones weight row
         int s_val;
         tc_ld_32x1(taddr + p.BNd, s_val);
@@ -724,7 +726,7 @@ gemm_i8_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
           for (int k = 0; k < 4; ++k) {
             const int b0 = (k >> 1) * 8 + (k & 1) * 2;
             x[k][0] = acc[b0]; x[k][1] = acc[b0 + 1]; x[k][2] = acc[b0 + 4]; x[k][3] = acc[b0 + 5];
-            if (EXTRA) {
+            if (EXTRA == 2) {
               x[k][0] -= sub[k]; x[k][1] -= sub[k]; x[k][2] -= sub[k]; x[k][3] -= sub[k];
               const int oc = n_tile * p.BNd + cb + q * 4 * STEPS + 4 * s;
               if (cls[k] && oc < p.Ocp) {
@@ -919,13 +921,18 @@ namespace {
 
 typedef void (*GemmKernel)(CUtensorMap, CUtensorMap, CUtensorMap, GemmParams);
 
-template <bool EXTRA, bool FUSE>
+template <int EXTRA, bool FUSE>
 GemmKernel kernel_of_width(int blk_w) {
   return blk_w == 64 ? gemm_i8_tc_kernel<EXTRA, FUSE, 4> : blk_w == 32 ? gemm_i8_tc_kernel<EXTRA, FUSE, 2> : gemm_i8_tc_kernel<EXTRA, FUSE, 1>;
 }
-GemmKernel kernel_variant(bool extra, bool fuse, int blk_w) {
-  return extra ? (fuse ? kernel_of_width<true, true>(blk_w) : kernel_of_width<true, false>(blk_w))
-               : (fuse ? kernel_of_width<false, true>(blk_w) : kernel_of_width<false, false>(blk_w));
+template <bool FUSE>
+GemmKernel kernel_of_form(int extra, int blk_w) {
+  return extra == 2 ? kernel_of_width<2, FUSE>(blk_w) : extra == 1 ? kernel_of_width<1, FUSE>(blk_w) : kernel_of_width<0, FUSE>(blk_w);
+}
+int extra_of(const GemmParams& p) { return p.dz != 0 || p.ep.border_corr != nullptr ? 2 : p.ep.fix_shl != 0 || p.ep.out.lo < 0 ? 1 : 0; }
+GemmKernel kernel_variant(const GemmParams& p) {
+  const int extra = extra_of(p);
+  return p.ep.add_residual != nullptr ? kernel_of_form<true>(extra, p.blk_w) : kernel_of_form<false>(extra, p.blk_w);
 }
 
 // Everything of a plan that does not depend on how A is addressed: N tiling, K block / swizzle mode,
@@ -1051,19 +1058,18 @@ bool finish_plan(GemmTcPlan* plan, const int8_t* B, int a_signed, int Np, int Kp
   size_t smem = ((static_cast<size_t>(stages) * stage_bytes + 1023) & ~static_cast<size_t>(1023)) + bres + staging + add_table_bytes + sizeof(SmemHeader) + 1024;
   if (smem < static_cast<size_t>(kMinDynSmem)) smem = kMinDynSmem;
   plan->smem = smem;
-  // the attribute belongs to the function on one device: set it once per device of this process
-  static bool attr_set[64] = {false};
+  // the attribute belongs to the function on one device: set it once per device of this process, and only for the functions
+  // that are used (asking loads the function)
+  static std::atomic<uint32_t> raised[64];
+  const uint32_t bit = 1u << (extra_of(p) * 6 + (e.add_residual != nullptr ? 3 : 0) + (p.blk_w == 64 ? 2 : p.blk_w == 32 ? 1 : 0));
   int dev = 0;
   cudaGetDevice(&dev);
-  if (dev < 0 || dev >= 64 || !attr_set[dev]) {
-    bool raised = true;
-    for (int v = 0; v < 12; ++v)
-      raised = raised && cudaFuncSetAttribute(kernel_variant(v & 1, v & 2, 16 << (v >> 2)), cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024) == cudaSuccess;
-    if (!raised) {
+  if (dev < 0 || dev >= 64 || !(raised[dev].load(std::memory_order_relaxed) & bit)) {
+    if (cudaFuncSetAttribute(kernel_variant(p), cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024) != cudaSuccess) {
       *why = "gemm_tc: cannot raise the dynamic shared memory limit";
       return false;
     }
-    if (dev >= 0 && dev < 64) attr_set[dev] = true;
+    if (dev >= 0 && dev < 64) raised[dev].fetch_or(bit, std::memory_order_relaxed);
   }
   return true;
 }
@@ -1416,9 +1422,7 @@ cudaError_t gemm_tc_launch(const GemmTcPlan* plan, cudaStream_t s) {
     stalled.params.tx_extra = 16;
     plan = &stalled;
   }
-  const bool extra = plan->params.dz != 0 || plan->params.ep.border_corr != nullptr || plan->params.ep.fix_shl != 0;
-  const bool fuse = plan->params.ep.add_residual != nullptr;
-  const cudaError_t launched = launch_pdl(kernel_variant(extra, fuse, plan->params.blk_w), dim3(plan->grid), dim3(kThreadsTc), plan->smem, s, plan->map_a, plan->map_b,
+  const cudaError_t launched = launch_pdl(kernel_variant(plan->params), dim3(plan->grid), dim3(kThreadsTc), plan->smem, s, plan->map_a, plan->map_b,
                         plan->map_r, plan->params);
   if (launched != cudaSuccess) return launched;
 #ifdef B2VX_TC_TRACE
