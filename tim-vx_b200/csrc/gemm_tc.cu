@@ -110,6 +110,7 @@ constexpr int kEpilogueWarps = B2VX_EPI_WARPS;   // a multiple of four: one warp
 constexpr int kGroups = kEpilogueWarps / 4;      // column groups of a wide tile, or teams on narrow tiles
 constexpr int kEpilogueThreads = kEpilogueWarps * 32;
 constexpr int kThreadsTc = (kFirstEpilogueWarp + kEpilogueWarps) * 32;
+constexpr int kRun = 4;              // 128-row pieces of a tile in run mode
 constexpr int kMaxStages = 8;
 constexpr int kMaxGroup = 8;
 constexpr int kMaxAccBuffers = 8;
@@ -161,6 +162,11 @@ struct GemmParams {
   // (about 56 bytes per clock) could not feed.  The price: both accumulators are in use, so a pair's epilogue does
   // not overlap the next pair's main loop; chosen only where the main loop is many times longer.
   int pair;
+  // Run mode (template RUN): narrow tiles in great number.  A tile of 128 x 16 or 128 x 32 outputs with a short K is little work,
+  // and the waits and hand-overs of the producer and the issuing warp, about 1180 cycles a tile whatever its width, bound it.
+  // So a tile is RUN x 128 consecutive rows here: one stage, RUN accumulators side by side, one hand-over.  MobileNetV2 at batch
+  // 1024: stem GEMM (K = 48, 32 channels) 418 -> 200 us, 32 -> 16 at 112 x 112 382 -> 131 us (617 MB: 0.72 of HBM), 96 -> 24 at 56 x 56 118 -> 74.
+  int run;
   // Columns are dealt to the epilogue warps in blocks of blk_w (64, 32 or 16), blk_per_group consecutive blocks to a
   // warp group (all of them in team mode).  plain_order: the weight rows are not permuted (blk_w is 16 then).
   int blk_w, blk_per_group, plain_order;
@@ -282,7 +288,8 @@ struct SmemHeader {
 // STEPS: column blocks of 16 * STEPS (1, 2 or 4) columns.  A template parameter because small layers are bound by
 // instruction fetch (a launch executes every line of the kernel about once per warp): code for the other widths in the
 // same kernel costs them.
-template <int EXTRA, bool FUSE, int STEPS>
+// RUN: 128-row pieces of a tile (run mode), else 1.
+template <int EXTRA, bool FUSE, int STEPS, int RUN = 1>
 __global__ void __launch_bounds__(kThreadsTc, 1)
 gemm_i8_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                   const __grid_constant__ CUtensorMap map_r, const GemmParams p) {
@@ -293,7 +300,7 @@ gemm_i8_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
   const uint32_t raw_addr = smem_u32(smem_raw);
   const uint32_t tiles_addr = (raw_addr + 1023u) & ~1023u;
   uint8_t* tiles = smem_raw + (tiles_addr - raw_addr);
-  const uint32_t a_bytes = p.halo ? p.a_stage_bytes : static_cast<uint32_t>(kBlockM) * p.BK;
+  const uint32_t a_bytes = p.halo ? p.a_stage_bytes : static_cast<uint32_t>(RUN * kBlockM) * p.BK;
   const uint32_t b_bytes = static_cast<uint32_t>(p.BN) * p.BK;
   const uint32_t sub_bytes = (p.pair ? 2u : 1u) * a_bytes + (p.b_resident ? 0u : b_bytes);   // one k-block: whole swizzle atoms, see the host-side plan
   const uint32_t b_off = (p.pair ? 2u : 1u) * a_bytes;   // B behind the A block(s) of a k-block
@@ -420,7 +427,9 @@ gemm_i8_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
                 if (++t_kx == p.kw) { t_kx = 0; ++t_ky; }
               }
             } else if (is_a) {
-              tma_load_2d(dst, &map_a, (kb0 + gi) * p.BK, m_tile * kBlockM, full);
+              tma_load_2d(dst, &map_a, (kb0 + gi) * p.BK, m_tile * RUN * kBlockM, full);
+#pragma unroll
+              for (int r = 2; r < RUN; r += 2) tma_load_2d(dst + r * kBlockM * p.BK, &map_a, (kb0 + gi) * p.BK, (m_tile * RUN + r) * kBlockM, full);
               if (two) tma_load_2d(dst + a_bytes, &map_a, (kb0 + gi) * p.BK, (m_tile + m_step) * kBlockM, full);
             } else {
               tma_load_2d(dst + b_off, &map_b, (kb0 + gi) * p.BK, n_tile * p.BN, full);
@@ -540,6 +549,14 @@ gemm_i8_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
                 tc_mma_i8_halves<1>(tmem_d2, a_lo + a2 + 2u * k, a_hi, b_lo + 2u * k, b_hi, p.idesc);
               }
             }
+          } else if (RUN > 1) {
+            const uint32_t piece = static_cast<uint32_t>(kBlockM * p.BK) >> 4, d_step = static_cast<uint32_t>(p.acc_stride) / RUN;
+            for (int gi = 0; gi < cnt; ++gi, a_lo += da_step, b_lo += db_step)
+              for (int k = 0; k < ksteps; ++k) {
+#pragma unroll
+                for (int r = 0; r < RUN; ++r) tc_mma_i8(tmem_d + r * d_step, (static_cast<uint64_t>(a_hi) << 32) + (a_lo + r * piece + 2u * k), (static_cast<uint64_t>(b_hi) << 32) + (b_lo + 2u * k), p.idesc, !first);
+                first = false;
+              }
           } else {
             for (int gi = 0; gi < cnt; ++gi, a_lo += da_step, b_lo += db_step) {
               if (first) {
@@ -673,8 +690,8 @@ gemm_i8_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
       } else {
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
-          row[k] = m_tile * kBlockM + quarter * 32 + g + 8 * k;
-          if (row[k] >= p.M) row[k] = -1;
+          row[k] = m_tile * RUN * kBlockM + quarter * 32 + g + 8 * k;
+          if (RUN == 1 && row[k] >= p.M) row[k] = -1;
           cls[k] = 0;
         }
       }
@@ -697,7 +714,7 @@ gemm_i8_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
       TC_EPI(j, 2);
       if (warp == kFirstEpilogueWarp && lane == 0) TC_TRACE(2, j, 0);
       tc_fence_after();
-      const uint32_t taddr = tmem_base + a * p.acc_stride + (static_cast<uint32_t>(quarter * 32) << 16);
+      uint32_t taddr = tmem_base + a * p.acc_stride + (static_cast<uint32_t>(quarter * 32) << 16);
       int sub[4] = {0, 0, 0, 0};
       if (EXTRA == 2 && p.dz != 0) {
         // S = sum of a row's inputs: the accumulator column of the all-ones weight row
@@ -754,7 +771,7 @@ gemm_i8_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
           const size_t at = static_cast<size_t>(row[k]) * p.ldd + col;
-          const bool ok = row[k] >= 0 && col_ok;
+          const bool ok = (RUN == 1 ? row[k] >= 0 : row[k] < p.M) && col_ok;
           if (FUSE) {
             uint32_t res[STEPS];
             if (p.res_tma) {
@@ -809,7 +826,15 @@ gemm_i8_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
         }
       };
 #pragma unroll 1
-      for (int blk = blk0; blk < blk1; ++blk) block(blk * w);
+      for (int r = 0; r < RUN; ++r) {
+#pragma unroll 1
+        for (int blk = blk0; blk < blk1; ++blk) block(blk * w);
+        if (RUN > 1) {
+          taddr += static_cast<uint32_t>(p.acc_stride) / RUN;
+#pragma unroll
+          for (int k = 0; k < 4; ++k) row[k] += kBlockM;
+        }
+      }
       TC_EPI(j, 3);
       // accumulator buffer (and residual buffer) free again
       tc_fence_before();
@@ -932,6 +957,8 @@ GemmKernel kernel_of_form(int extra, int blk_w) {
 int extra_of(const GemmParams& p) { return p.dz != 0 || p.ep.border_corr != nullptr ? 2 : p.ep.fix_shl != 0 || p.ep.out.lo < 0 ? 1 : 0; }
 GemmKernel kernel_variant(const GemmParams& p) {
   const int extra = extra_of(p);
+  if (p.run > 1) return extra ? (p.blk_w == 32 ? gemm_i8_tc_kernel<1, false, 2, kRun> : gemm_i8_tc_kernel<1, false, 1, kRun>)
+                              : (p.blk_w == 32 ? gemm_i8_tc_kernel<0, false, 2, kRun> : gemm_i8_tc_kernel<0, false, 1, kRun>);
   return p.ep.add_residual != nullptr ? kernel_of_form<true>(extra, p.blk_w) : kernel_of_form<false>(extra, p.blk_w);
 }
 
@@ -942,7 +969,7 @@ GemmKernel kernel_variant(const GemmParams& p) {
 // turns out to allow the halo mode of the implicit convolution (0: not asked for).
 bool finish_plan(GemmTcPlan* plan, const int8_t* B, int a_signed, int Np, int Kp, int Kspan, int taps, int ldd,
                  const ContractEpilogue& e, void* D, int* status, const char** why, const GemmTcTiling* tiling, int halo_w = 0,
-                 int halo_h = 0, bool want_pair = false, bool wide_teams = false) {
+                 int halo_h = 0, bool want_pair = false, bool wide_teams = false, bool want_run = false) {
   GemmParams& p = plan->params;
   p.Ocp = ldd;
   p.ldd = ldd;
@@ -1018,7 +1045,11 @@ bool finish_plan(GemmTcPlan* plan, const int8_t* B, int a_signed, int Np, int Kp
   const char* pair_env = std::getenv("B2VX_TC_PAIR");   // read per plan, so that one process can build both forms
   const bool no_pair = pair_env && std::strcmp(pair_env, "0") == 0;
   p.pair = (want_pair && !no_pair && !p.halo && !p.b_resident && !p.teams && e.add_residual == nullptr && p.BN > 128) ? 1 : 0;
-  const size_t sub_bytes = p.halo ? p.a_stage_bytes : static_cast<size_t>((p.pair ? 2 : 1) * kBlockM + (p.b_resident ? 0 : p.BN)) * p.BK;
+  // Run mode: weights resident, a team per tile, four accumulator buffers of four pieces (up to 32 columns a piece), at least
+  // three stages.
+  p.run = want_run && p.b_resident && p.teams && p.BN <= 32 && p.dz == 0 && e.add_residual == nullptr && !p.plain_order &&
+          3 * static_cast<size_t>(kRun * kBlockM) * p.BK + bres + 8192 + sizeof(SmemHeader) <= static_cast<size_t>(kSmemBudget) ? kRun : 1;
+  const size_t sub_bytes = p.halo ? p.a_stage_bytes : static_cast<size_t>((p.pair ? 2 : p.run) * kBlockM + (p.b_resident ? 0 : p.BN)) * p.BK;
   const size_t ring_budget = kSmemBudget - 2048 - sizeof(SmemHeader) - staging - add_table_bytes - bres;
   int group = static_cast<int>((64 * 1024) / sub_bytes);
   if (p.halo) group = 1;
@@ -1035,7 +1066,7 @@ bool finish_plan(GemmTcPlan* plan, const int8_t* B, int a_signed, int Np, int Kp
   // the epilogue reads 16 columns at a time; buffers start on 32-column boundaries
   // As many accumulator buffers as the 512 TMEM columns hold (2, 4 or 8): with narrow tiles the
   // epilogue of a tile is a latency chain, and more tiles in flight hide it.
-  p.acc_stride = (p.BN + 31) & ~31;
+  p.acc_stride = p.run * ((p.BN + 31) & ~31);
   p.acc_shift = 1;
   while (p.acc_shift < 3 && (2 << p.acc_shift) * p.acc_stride <= 512) ++p.acc_shift;
   if (p.teams && (1 << p.acc_shift) < kGroups) p.teams = 0;   // every team's tile needs an accumulator buffer
@@ -1061,7 +1092,7 @@ bool finish_plan(GemmTcPlan* plan, const int8_t* B, int a_signed, int Np, int Kp
   // the attribute belongs to the function on one device: set it once per device of this process, and only for the functions
   // that are used (asking loads the function)
   static std::atomic<uint32_t> raised[64];
-  const uint32_t bit = 1u << (extra_of(p) * 6 + (e.add_residual != nullptr ? 3 : 0) + (p.blk_w == 64 ? 2 : p.blk_w == 32 ? 1 : 0));
+  const uint32_t bit = 1u << (p.run > 1 ? 18 + (extra_of(p) != 0 ? 2 : 0) + (p.blk_w == 32 ? 1 : 0) : extra_of(p) * 6 + (e.add_residual != nullptr ? 3 : 0) + (p.blk_w == 64 ? 2 : p.blk_w == 32 ? 1 : 0));
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev < 0 || dev >= 64 || !(raised[dev].load(std::memory_order_relaxed) & bit)) {
@@ -1123,18 +1154,21 @@ GemmTcPlan* gemm_tc_plan_create(const void* A, int a_signed, const int8_t* B, in
   const long long tiles_256 = static_cast<long long>((M + kBlockM - 1) / kBlockM) * ((Np + 255) / 256);
   const bool want_pair = Kp >= 4096 && tiles_256 >= 2LL * sms;
   const bool wide_teams = Kp <= 128 && static_cast<long long>((M + kBlockM - 1) / kBlockM) >= 8LL * sms;
-  if (!finish_plan(plan, B, a_signed, Np, Kp, Kp, 1, ldd, e, D, status, &why, tiling, 0, 0, want_pair, wide_teams)) {
+  // run mode where every team of a CTA gets two tiles or more
+  static const bool no_run = [] { const char* e2 = std::getenv("B2VX_TC_RUN"); return e2 && std::strcmp(e2, "0") == 0; }();
+  const bool want_run = !no_run && Kp <= 128 && M >= kRun * kBlockM * 8LL * sms;
+  if (!finish_plan(plan, B, a_signed, Np, Kp, Kp, 1, ldd, e, D, status, &why, tiling, 0, 0, want_pair, wide_teams, want_run)) {
     delete plan;
     return fail(why);
   }
   p.M = M;
   p.num_kb = (Kp + p.BK - 1) / p.BK;
-  p.m_tiles = (M + kBlockM - 1) / kBlockM;
+  p.m_tiles = (M + p.run * kBlockM - 1) / (p.run * kBlockM);
   // Rows past the end are left out of the box: filled with zeros they cost the TMA unit time (host to host, eight layers of
   // 4096 x 4096: 17 rows 150 -> 101 us, 24 rows 149 -> 105; twelve of 2048 x 2048, 49 rows: 120 -> 104; from 64 rows on level).
   // What lies in the tile's other rows is multiplied into accumulators that nobody reads.
-  p.box_rows = M < kBlockM ? M : kBlockM;
-  p.a_tx_bytes = static_cast<uint32_t>(p.box_rows) * p.BK;
+  p.box_rows = M < kBlockM ? M : p.run > 1 ? 2 * kBlockM : kBlockM;   // run mode: two pieces a box
+  p.a_tx_bytes = static_cast<uint32_t>(p.run > 1 ? p.run * kBlockM : p.box_rows) * p.BK;
   const uint64_t adims[2] = {static_cast<uint64_t>(Kp), static_cast<uint64_t>(M)};
   const uint32_t abox[2] = {static_cast<uint32_t>(p.BK), static_cast<uint32_t>(p.box_rows)};
   bool ok = encode_u8(&plan->map_a, A, 2, adims, abox, nullptr, swizzle_of(p.BK));
