@@ -325,11 +325,13 @@ DwMmaPlan* dw_mma_plan_create(const void* x, int x_signed, const int8_t* w, cons
   std::memset(pl, 0, sizeof(*pl));
   DwMmaPlan::Params& p = pl->p;
   // Channel groups of a slab: all of them up to nine, else whole sectors (an even number), the split that leaves the
-  // fewest groups idle, the widest among equals.
+  // fewest groups idle; among equals the one that fills a block with eight warps (8 groups, or 4 of two strips) before the one
+  // that makes six: two blocks of either share an SM.  Batch 256: 28 x 28 x 192 57.1 us with 6 groups, 43.0 with 4; 14 x 14 x 576
+  // 46.1 and 34.5; 7 x 7 x 960 25.1 and 22.5.
   p.groups = all;
   if (all > kMaxWarps) {
     int best_idle = 1 << 30;
-    for (int c : {8, 6, 4}) {
+    for (int c : {8, 4, 6}) {
       const int idle = (all + c - 1) / c * c - all;
       if (idle < best_idle) { best_idle = idle; p.groups = c; }
     }
@@ -338,11 +340,11 @@ DwMmaPlan* dw_mma_plan_create(const void* x, int x_signed, const int8_t* w, cons
   const int ns = G == 1 ? 8 : G == 2 ? 4 : G <= 4 ? 2 : 1;
   pl->warps = G * ns;
   p.pitch = 16 * (G | 1);
-  // Tile: strips side by side x rows x images.  Three blocks of up to seven warps per SM or two larger ones, each with its
-  // share of the shared memory.  A tile costs its units (two rows of a strip) or the bytes it moves, whichever is more,
+  // Tile: strips side by side x rows x images.  Three blocks per SM where their registers fit (up to six warps), or two, each
+  // with its share of the shared memory.  A tile costs its units (two rows of a strip) or the bytes it moves, whichever is more,
   // plus a fixed part (units of 2 rows; 8.4 KB is what an SM moves from DRAM in the time of one); the launch as many
   // waves of that as the tiles make.
-  const int per_sm_target = pl->warps + 1 <= 7 ? 3 : 2;
+  const int per_sm_target = pl->warps + 1 <= 6 ? 3 : 2;
   const size_t budget = (per_sm_target == 3 ? 74 : 112) * 1024;
   const int strips_w = (g.Wo + 7) / 8;
   double best_cost = -1.0;
