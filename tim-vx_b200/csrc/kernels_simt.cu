@@ -1670,17 +1670,18 @@ __global__ void im2col_whcn_kernel(const uint8_t* __restrict__ x, int Kp, int zx
 // taps, kw <= 8, dilation 1): the 8 bytes of one (pixel, ky, c) are 8 consecutive input bytes, so a
 // 16-byte piece of the matrix is two unaligned 8-byte reads of the staged rows instead of sixteen
 // gathered bytes.  The byte in the padding slot (kx >= kw) belongs to the neighbouring pixel; its
-// weight is zero.  One block per output row (n, ho); staged rows have pitch `pitch` (a multiple of 4,
+// weight is zero.  A block takes out_rows output rows of an image; staged rows have pitch `pitch` (a multiple of 4,
 // at least 8 bytes beyond the last input column used).
 template <int PADK>
 __global__ void __launch_bounds__(256) im2col_whcn8_kernel(const uint8_t* __restrict__ x, int Kp, int zx, ConvGeom g, int pitch,
-                                                           uint8_t* __restrict__ col) {
+                                                           int out_rows, uint8_t* __restrict__ col) {
   pdl_wait();
   pdl_trigger();
   extern __shared__ uint32_t sm_words[];
-  uint8_t* img = reinterpret_cast<uint8_t*>(sm_words);     // [kh*C][pitch]
-  const int n = blockIdx.y, ho = blockIdx.x;
-  const int rows = g.kh * g.C;
+  uint8_t* img = reinterpret_cast<uint8_t*>(sm_words);     // [((out_rows-1)*sy + kh)*C][pitch]
+  const int n = blockIdx.y, ho = blockIdx.x * out_rows, here = min(out_rows, g.Ho - ho);
+  const int taps = g.kh * g.C, row_step = g.sy * g.C;     // staged rows of an output row, and from one output row to the next
+  const int rows = taps + (here - 1) * row_step;
   // Staged column j holds input column j - lead; lead = pad_left rounded up to 4 keeps input words
   // aligned with shared-memory words.  First everything becomes the zero point, then the in-bounds
   // part of each row is copied (as 32-bit words when the input rows allow it).
@@ -1719,19 +1720,20 @@ __global__ void __launch_bounds__(256) im2col_whcn8_kernel(const uint8_t* __rest
   __syncthreads();
   const int shift0 = lead - g.pl;                          // staged column of output pixel 0, tap 0
   const int chunks = Kp >> 4;
-  uint8_t* out = col + (static_cast<size_t>(n) * g.Ho + ho) * g.Wo * Kp;
-  // piece q = wo * chunks + ch; a thread's next piece is 256 further, stepped without divisions
-  int wo = threadIdx.x / chunks, ch = threadIdx.x - wo * chunks;
-  const int step_wo = 256 / chunks, step_ch = 256 - step_wo * chunks;
-  for (int q = threadIdx.x; q < g.Wo * chunks; q += 256, wo += step_wo, ch += step_ch) {
+  uint4* out = reinterpret_cast<uint4*>(col + (static_cast<size_t>(n) * g.Ho + ho) * g.Wo * Kp);
+  // piece q = (output row * Wo + wo) * chunks + ch; a thread's next piece is 256 further, stepped without divisions
+  int wo = threadIdx.x / chunks, ch = threadIdx.x - wo * chunks, r0 = 0;   // r0: first staged row of the output row
+  const int step_wo = 256 / chunks, step_ch = 256 - step_wo * chunks, pieces = here * g.Wo * chunks;
+  for (int q = threadIdx.x; q < pieces; q += 256, wo += step_wo, ch += step_ch) {
     if (ch >= chunks) { ch -= chunks; ++wo; }
+    while (wo >= g.Wo) { wo -= g.Wo; r0 += row_step; }
     uint32_t w4[4] = {0, 0, 0, 0};
     if (PADK == 8) {
 #pragma unroll
       for (int h = 0; h < 2; ++h) {
         const int r = 2 * ch + h;
-        if (r < rows) {
-          const int byte = r * pitch + wo * g.sx + shift0;
+        if (r < taps) {
+          const int byte = (r0 + r) * pitch + wo * g.sx + shift0;
           const uint32_t* wp = sm_words + (byte >> 2);
           const uint32_t sh = (byte & 3) * 8;
           const uint32_t a0 = wp[0], a1 = wp[1], a2 = wp[2];
@@ -1743,14 +1745,14 @@ __global__ void __launch_bounds__(256) im2col_whcn8_kernel(const uint8_t* __rest
 #pragma unroll
       for (int h = 0; h < 4; ++h) {
         const int r = 4 * ch + h;
-        if (r < rows) {
-          const int byte = r * pitch + wo * g.sx + shift0;
+        if (r < taps) {
+          const int byte = (r0 + r) * pitch + wo * g.sx + shift0;
           const uint32_t* wp = sm_words + (byte >> 2);
           w4[h] = __funnelshift_r(wp[0], wp[1], (byte & 3) * 8);
         }
       }
     }
-    *reinterpret_cast<uint4*>(out + static_cast<size_t>(wo) * Kp + ch * 16) = make_uint4(w4[0], w4[1], w4[2], w4[3]);
+    out[q] = make_uint4(w4[0], w4[1], w4[2], w4[3]);
   }
 }
 
@@ -2490,14 +2492,21 @@ void launch_fc_small_m(const void* A, int a_signed, const int8_t* B, int M, int 
 void launch_im2col_whcn8(const void* x, int Kp, int zx, const ConvGeom& g, int padk, void* col, cudaStream_t s) {
   if (g.N == 0 || g.Ho == 0 || g.Wo == 0) return;
   const int pitch = im2col_whcn8_pitch(g, padk);
-  const size_t smem = static_cast<size_t>(g.C) * g.kh * pitch + 16;
-  dim3 grid(g.Ho, g.N);
-  if (padk == 8)
-    launch_pdl(im2col_whcn8_kernel<8>, dim3(grid), dim3(256), smem, s, static_cast<const uint8_t*>(x), Kp, zx, g, pitch,
-               static_cast<uint8_t*>(col));
-  else
-    launch_pdl(im2col_whcn8_kernel<4>, dim3(grid), dim3(256), smem, s, static_cast<const uint8_t*>(x), Kp, zx, g, pitch,
-               static_cast<uint8_t*>(col));
+  // Output rows of a block: eight pieces of 16 bytes for each thread where that leaves six blocks or more for every SM and the
+  // staged rows fit.  With one row a block, two barriers and the loads' latency came for as little as a third of a piece a
+  // thread: LeNet at batch 256 / 1000 host to host 88.8 -> 82.2 / 158 -> 127 us, MobileNetV2 at 64 / 1024 749 -> 743 / 8173 -> 8018,
+  // ResNet-50 at 64 1140 -> 1133.  Fewer blocks than six an SM are left alone: batch 1 keeps one row each.
+  const int per_row = g.Wo * (Kp / 16);
+  int out_rows = (2048 + per_row - 1) / per_row;
+  const long long room = static_cast<long long>(g.N) * g.Ho / (148 * 6);
+  if (out_rows > room) out_rows = static_cast<int>(room);
+  if (out_rows > g.Ho) out_rows = g.Ho;
+  auto bytes = [&](int r) { return static_cast<size_t>(g.C) * (g.kh + (r - 1) * g.sy) * pitch + 16; };
+  while (out_rows > 1 && bytes(out_rows) > 40u * 1024u) --out_rows;
+  if (out_rows < 1) out_rows = 1;
+  const dim3 grid((g.Ho + out_rows - 1) / out_rows, g.N);
+  launch_pdl(padk == 8 ? im2col_whcn8_kernel<8> : im2col_whcn8_kernel<4>, grid, dim3(256), bytes(out_rows), s, static_cast<const uint8_t*>(x), Kp, zx, g, pitch,
+             out_rows, static_cast<uint8_t*>(col));
 }
 int im2col_whcn8_pitch(const ConvGeom& g, int padk) {
   // up to 3 bytes of alignment lead, the padk-byte read of the last pixel, the last word of the funnel
