@@ -36,3 +36,26 @@ def test_one_tile_with_fused_add(product_lib, oracle_lib, spec, batch):
         g.close()
     assert any("+add" in n for n in names), names
     G.assert_same(*outs)
+
+
+@pytest.mark.parametrize("channels", [32, 48, 64, 96, 150, 288])
+@pytest.mark.parametrize("form", ["1x1", "3x3", "add"])
+def test_one_narrow_tile_for_each_block(product_lib, oracle_lib, channels, form):
+    """Launches of about a wave with tiles of 16 to 64 columns: all epilogue warps share the only tile of a block."""
+    for hw, batch in ((56, 1), (19, 4), (65, 2)):
+        if form == "add":
+            outs = []
+            for lib in (oracle_lib, product_lib):
+                g = B.Graph(lib)
+                w = opworkloads.build("convadd:1:64:%d:%d:1" % (channels, hw), batch, g, np.random.default_rng(channels))
+                g.compile()
+                for t, a in w["inputs"]:
+                    g.write(t, a)
+                g.run()
+                outs.append([g.read(t) for t in w["outputs"]])
+                g.close()
+            G.assert_same(*outs)
+        else:
+            k = int(form[0])
+            build = G.conv2d_q(hw, hw, 32, batch, k, k, channels)
+            G.assert_same(*(G.run_case(lib, build, channels)[0] for lib in (oracle_lib, product_lib)))

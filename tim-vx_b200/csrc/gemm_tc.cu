@@ -64,6 +64,7 @@
 #include <cuda.h>
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <atomic>
 #include <cmath>
 #include <cstdio>
@@ -125,7 +126,7 @@ struct GemmParams {
   int tmem_cols;
   int acc_stride;          // TMEM columns between accumulator buffers (BN rounded up to 32)
   int acc_shift;           // log2 of the number of accumulator buffers (2, 4 or 8 of them)
-  // Narrow tiles (at most four 16-column chunks): the sixteen epilogue warps split into four teams of four
+  // Narrow tiles (at most four 16-column chunks), several to a CTA: the sixteen epilogue warps split into four teams of four
   // (one warp per TMEM lane quarter), each team takes every fourth tile of the CTA and all of its chunks, so
   // that a warp's per-tile work (waits, row arithmetic) is spread over four chunks as it is with wide tiles.
   int teams;
@@ -962,6 +963,8 @@ GemmKernel kernel_variant(const GemmParams& p) {
   return p.ep.add_residual != nullptr ? kernel_of_form<true>(extra, p.blk_w) : kernel_of_form<false>(extra, p.blk_w);
 }
 
+bool one_tile_each(long long m_tiles, int n_tiles, int sms) { return m_tiles * n_tiles <= sms / n_tiles * n_tiles; }
+
 // Everything of a plan that does not depend on how A is addressed: N tiling, K block / swizzle mode,
 // column blocks, stage count, TMEM columns, instruction descriptor, the B tensor map.
 // Kspan is the K extent one tap (or the whole GEMM) covers, used to pick BK.
@@ -969,7 +972,7 @@ GemmKernel kernel_variant(const GemmParams& p) {
 // turns out to allow the halo mode of the implicit convolution (0: not asked for).
 bool finish_plan(GemmTcPlan* plan, const int8_t* B, int a_signed, int Np, int Kp, int Kspan, int taps, int ldd,
                  const ContractEpilogue& e, void* D, int* status, const char** why, const GemmTcTiling* tiling, int halo_w = 0,
-                 int halo_h = 0, bool want_pair = false, bool wide_teams = false, bool want_run = false) {
+                 int halo_h = 0, bool want_pair = false, bool wide_teams = false, bool want_run = false, bool one_each = false) {
   GemmParams& p = plan->params;
   p.Ocp = ldd;
   p.ldd = ldd;
@@ -1004,7 +1007,9 @@ bool finish_plan(GemmTcPlan* plan, const int8_t* B, int a_signed, int Np, int Kp
   static const bool no_teams = [] { const char* e2 = std::getenv("B2VX_TC_TEAMS"); return e2 && std::strcmp(e2, "0") == 0; }();
   // (wide_teams: the caller found the launch bound by its epilogue, short K and many tiles per CTA, so tiles of up to 128
   // columns also go one per warp group: four tiles in flight instead of four passes over every tile)
-  p.teams = ((p.BNd <= 64 || (wide_teams && p.BN <= 128)) && !no_teams) ? kGroups : 0;
+  // (one_each: no CTA gets a second tile, so three teams would have nothing to do; all sixteen warps share the one, in column
+  // blocks of 16.  Host to host: ResNet-50 batch 1 / 4 314.6 -> 308.2 / 387 -> 375 us, MobileNetV2 batch 1 / 8 234.3 -> 227.5 / 301 -> 294.)
+  p.teams = ((p.BNd <= 64 || (wide_teams && p.BN <= 128)) && !no_teams && !(one_each && p.BNd >= 32)) ? kGroups : 0;
   p.blk_per_group = (p.BNd / p.blk_w + kGroups - 1) / kGroups;
   p.res_tma = e.add_residual != nullptr && !p.plain_order ? 1 : 0;
   p.res_shift = p.teams ? 2 : 1;
@@ -1157,7 +1162,8 @@ GemmTcPlan* gemm_tc_plan_create(const void* A, int a_signed, const int8_t* B, in
   // run mode where every team of a CTA gets two tiles or more
   static const bool no_run = [] { const char* e2 = std::getenv("B2VX_TC_RUN"); return e2 && std::strcmp(e2, "0") == 0; }();
   const bool want_run = !no_run && Kp <= 128 && M >= kRun * kBlockM * 8LL * sms;
-  if (!finish_plan(plan, B, a_signed, Np, Kp, Kp, 1, ldd, e, D, status, &why, tiling, 0, 0, want_pair, wide_teams, want_run)) {
+  if (!finish_plan(plan, B, a_signed, Np, Kp, Kp, 1, ldd, e, D, status, &why, tiling, 0, 0, want_pair, wide_teams, want_run,
+                   one_tile_each((M + kBlockM - 1) / kBlockM, tiling ? tiling->n_tiles : (Np + 255) / 256, sms))) {
     delete plan;
     return fail(why);
   }
@@ -1210,10 +1216,6 @@ GemmTcPlan* gemm_tc_conv_plan_create(const void* X, int x_signed, const int8_t* 
     const double covered = static_cast<double>((g.Wo + 7) / 8 * 8) * ((g.Ho + 15) / 16 * 16);
     if (static_cast<double>(g.Wo) * g.Ho >= 0.85 * covered) { halo_w = 8 + g.kw - 1; halo_h = 16 + g.kh - 1; }
   }
-  if (!finish_plan(plan, B, x_signed, Np, Kp, g.Cp, g.kh * g.kw, g.Ocp, e, D, status, &why, tiling, halo_w, halo_h)) {
-    delete plan;
-    return fail(why);
-  }
   // M tile = TW x TH x TN output pixels, at most 128: the shape that leaves the fewest tile rows unused.
   int bw = 1, bh = 1, bn = 1;
   double best = -1.0;
@@ -1229,6 +1231,18 @@ GemmTcPlan* gemm_tc_conv_plan_create(const void* X, int x_signed, const int8_t* 
       // prefer wider rows at equal efficiency: longer contiguous runs per TMA box
       if (eff > best + 1e-9 || (eff > best - 1e-9 && tw > bw)) { best = eff; bw = tw; bh = th; bn = tn; }
     }
+  }
+  int sms = 148;
+  {
+    int dev = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  }
+  auto tiles_of = [&](int tw, int th, int tn) { return static_cast<long long>((g.Wo + tw - 1) / tw) * ((g.Ho + th - 1) / th) * ((g.N + tn - 1) / tn); };
+  const bool one_each = one_tile_each(std::max(tiles_of(bw, bh, bn), halo_w ? tiles_of(8, 16, 1) : 0), tiling ? tiling->n_tiles : (Np + 255) / 256, sms);
+  if (!finish_plan(plan, B, x_signed, Np, Kp, g.Cp, g.kh * g.kw, g.Ocp, e, D, status, &why, tiling, halo_w, halo_h, false, false, false, one_each)) {
+    delete plan;
+    return fail(why);
   }
   if (p.halo) { bw = 8; bh = 16; bn = 1; }
   p.conv = 1;
@@ -1351,7 +1365,8 @@ GemmTcTiling gemm_tc_choose_tiling(long long M, int Ocp, int Kp, int with_s) {
     best.rows = best.data + extra;
   }
   // (the same test as wide_teams in gemm_tc_plan_create; block widths are free to choose, a mismatch costs only time)
-  best.blk_w = column_block(best.data, best.data <= 64 || (best.rows <= 128 && Kp <= 128 && m_tiles >= 8LL * sms));
+  best.blk_w = column_block(best.data, (best.data <= 64 && !(best.data >= 32 && one_tile_each(m_tiles, best.n_tiles, sms))) ||
+                                          (best.rows <= 128 && Kp <= 128 && m_tiles >= 8LL * sms));
   return best;
 }
 
