@@ -29,3 +29,39 @@ def test_float_rows_between_images(product_lib, oracle_lib):
     want, _ = G.run_case(oracle_lib, build, 2)
     got, _ = G.run_case(product_lib, build, 2)
     G.assert_same(want, got, float_tol=1e-5)
+
+
+@pytest.mark.parametrize("outputs,batch", [(2, 1), (3, 300), (5, 7), (9, 2)])
+def test_several_outputs_share_a_launch(product_lib, oracle_lib, outputs, batch):
+    """Row counts equal, row lengths not (1 to 50 bytes); read after a run, after an asynchronous one, and after a second input."""
+    def build(g, rng):
+        x = g.tensor(B.DT_UINT8, [40, batch], B.ATTR_INPUT, scale=0.02, zero_point=128)
+        ys = []
+        for k in range(outputs):
+            n = [10, 50, 1, 33, 17, 9, 47, 3, 21][k]
+            w = g.tensor(B.DT_INT8, [40, n], B.ATTR_CONSTANT, scales=rng.uniform(0.001, 0.01, n).astype(np.float32), channel_dim=1,
+                         data=rng.integers(-127, 128, size=(n, 40)).astype(np.int8))
+            ys.append(g.tensor(B.DT_UINT8, [], B.ATTR_OUTPUT, scale=0.02, zero_point=100))
+            g.fully_connected(x, w, None, ys[-1], axis=0, weights=n)
+        return x, ys
+
+    results = []
+    for lib in (oracle_lib, product_lib):
+        rng = np.random.default_rng(outputs)
+        g = B.Graph(lib)
+        x, ys = build(g, rng)
+        g.compile()
+        got = []
+        for k in range(3):
+            g.write(x, rng.integers(0, 256, size=(batch, 40)).astype(np.uint8))
+            if k == 1 and hasattr(g, "run_async"):
+                g.run_async()
+                g.sync()
+            else:
+                g.run()
+            got += [g.read(y) for y in ys]
+        names = [k["name"] for k in g.kernels()]
+        g.close()
+        results.append(got)
+    assert names.count("cl_to_whcn") == (outputs + 3) // 4, names
+    G.assert_same(*results)

@@ -83,9 +83,14 @@ struct ContractEpilogue {
 // n16 16-byte pieces from src to dst, either of which may be page-locked host memory.
 void launch_copy16(const void* src, void* dst, size_t n16, cudaStream_t s);
 
-// Rows of row_bytes each, pitch bytes apart, to one dense array in page-locked host memory (whole 16-byte pieces: the
-// array's space is rounded up to them).
-void launch_pack_rows16(const void* src, void* dst, int rows, int row_bytes, int pitch, cudaStream_t s);
+// Of each of n tensors: rows of row_bytes each, pitch bytes apart, to one dense array (whole 16-byte pieces: the array's
+// space is rounded up to them), which may be page-locked host memory.  One launch for all outputs of a graph.
+struct PackRows {
+  const void* src[4];
+  void* dst[4];
+  int rows[4], row_bytes[4], pitch[4], n;
+};
+void launch_pack_rows16(const PackRows& p, cudaStream_t s);
 
 // ---- layout converters (elem = 1 or 4 bytes) -------------------------------
 void launch_whcn_to_cl(const void* src, void* dst, int N, int C, int H, int W, int Cp, int elem, cudaStream_t s);

@@ -45,9 +45,12 @@ __global__ void __launch_bounds__(128) copy16_kernel(const uint4* __restrict__ s
 }
 
 // Dense rows out of padded ones, 16 bytes of the result per thread: the bus takes them in few writes.
-__global__ void __launch_bounds__(128) pack_rows16_kernel(const uint8_t* __restrict__ src, uint4* __restrict__ dst, int rows, int row_bytes, int pitch) {
+__global__ void __launch_bounds__(128) pack_rows16_kernel(const __grid_constant__ PackRows p) {
   pdl_trigger();
   pdl_wait();
+  const uint8_t* src = static_cast<const uint8_t*>(p.src[blockIdx.y]);
+  uint4* dst = static_cast<uint4*>(p.dst[blockIdx.y]);
+  const int rows = p.rows[blockIdx.y], row_bytes = p.row_bytes[blockIdx.y], pitch = p.pitch[blockIdx.y];
   const int i = blockIdx.x * 128 + threadIdx.x, total = rows * row_bytes;
   if (16 * i >= total) return;
   int r = 16 * i / row_bytes, o = 16 * i - r * row_bytes;
@@ -1548,6 +1551,8 @@ __device__ __forceinline__ float load_real(const void* x, int kind, long long i,
 // One thread per slice; slices are short (class scores).
 __global__ void softmax_kernel(const void* __restrict__ x, int x_kind, float sx, int zx, void* __restrict__ y, int y_kind,
                                OutQuant out, float beta, SoftmaxGeom g) {
+  pdl_trigger();
+  pdl_wait();
   const long long slices = static_cast<long long>(g.o[0]) * g.o[1] * g.o[2];
   long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x;
   if (i >= slices) return;
@@ -1875,10 +1880,11 @@ void launch_copy16(const void* src, void* dst, size_t n16, cudaStream_t s) {
   launch_pdl(copy16_kernel, dim3(static_cast<unsigned>((n16 + 127) / 128)), dim3(128), 0, s, static_cast<const uint4*>(src), static_cast<uint4*>(dst), n16);
 }
 
-void launch_pack_rows16(const void* src, void* dst, int rows, int row_bytes, int pitch, cudaStream_t s) {
-  const int n16 = (rows * row_bytes + 15) / 16;
+void launch_pack_rows16(const PackRows& p, cudaStream_t s) {
+  int n16 = 0;
+  for (int i = 0; i < p.n; ++i) n16 = max(n16, (p.rows[i] * p.row_bytes[i] + 15) / 16);
   if (n16 == 0) return;
-  launch_pdl(pack_rows16_kernel, dim3((n16 + 127) / 128), dim3(128), 0, s, static_cast<const uint8_t*>(src), static_cast<uint4*>(dst), rows, row_bytes, pitch);
+  launch_pdl(pack_rows16_kernel, dim3((n16 + 127) / 128, p.n), dim3(128), 0, s, p);
 }
 
 void launch_whcn_to_cl(const void* src, void* dst, int N, int C, int H, int W, int Cp, int elem, cudaStream_t s) {
@@ -2328,7 +2334,7 @@ void launch_softmax(const void* x, int x_kind, float sx, int zx, void* y, int y_
                     const SoftmaxGeom& g, cudaStream_t s) {
   const long long slices = static_cast<long long>(g.o[0]) * g.o[1] * g.o[2];
   if (slices == 0 || g.len == 0) return;
-  softmax_kernel<<<grid_for(slices, 128), 128, 0, s>>>(x, x_kind, sx, zx, y, y_kind, out, beta, g);
+  launch_pdl(softmax_kernel, dim3(grid_for(slices, 128)), dim3(128), 0, s, x, x_kind, sx, zx, y, y_kind, out, beta, g);
 }
 
 void launch_im2col(const void* x, int Cs, int Kp, int zx, const ConvGeom& g, void* col, cudaStream_t s) {
