@@ -14,7 +14,10 @@ CASES = {
     "whole_tiles": (112, 112, 64, 32, 16, (0.05, 0), B.DT_UINT8), "8_rows_left": (67, 29, 312, 16, 32, (0.05, 3), B.DT_UINT8),
     "129_rows_left": (173, 9, 421, 32, 16, (0.05, 0), B.DT_UINT8), "last_piece_partly": (128, 37, 129, 48, 32, (0.05, 0), B.DT_UINT8),
     "int8_k96": (67, 29, 314, 96, 24, (0.05, -5), B.DT_INT8), "halved": (67, 29, 313, 48, 17, (1.5e-4, 100), B.DT_UINT8),
-    "one_tile_less": (67, 29, 311, 16, 32, (0.05, 3), B.DT_UINT8),
+    # two pieces a tile: 33 to 64 channels, from 303104 rows on
+    "c64": (56, 56, 97, 64, 64, (0.05, 0), B.DT_UINT8), "c48_k192": (67, 29, 157, 192, 48, (0.05, 3), B.DT_UINT8), "c64_int8": (173, 9, 211, 144, 50, (0.05, -5), B.DT_INT8),
+    "c64_halved": (128, 37, 65, 48, 64, (1.5e-4, 100), B.DT_UINT8), "c40": (1024, 1, 297, 256, 40, (0.05, 0), B.DT_UINT8), "k256": (112, 112, 49, 256, 32, (0.05, 0), B.DT_UINT8),
+    "c64_below": (67, 29, 155, 16, 64, (0.05, 3), B.DT_UINT8), "one_tile_less": (67, 29, 311, 16, 32, (0.05, 3), B.DT_UINT8),
 }
 
 

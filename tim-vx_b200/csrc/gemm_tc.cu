@@ -111,7 +111,6 @@ constexpr int kEpilogueWarps = B2VX_EPI_WARPS;   // a multiple of four: one warp
 constexpr int kGroups = kEpilogueWarps / 4;      // column groups of a wide tile, or teams on narrow tiles
 constexpr int kEpilogueThreads = kEpilogueWarps * 32;
 constexpr int kThreadsTc = (kFirstEpilogueWarp + kEpilogueWarps) * 32;
-constexpr int kRun = 4;              // 128-row pieces of a tile in run mode
 constexpr int kMaxStages = 8;
 constexpr int kMaxGroup = 8;
 constexpr int kMaxAccBuffers = 8;
@@ -163,10 +162,12 @@ struct GemmParams {
   // (about 56 bytes per clock) could not feed.  The price: both accumulators are in use, so a pair's epilogue does
   // not overlap the next pair's main loop; chosen only where the main loop is many times longer.
   int pair;
-  // Run mode (template RUN): narrow tiles in great number.  A tile of 128 x 16 or 128 x 32 outputs with a short K is little work,
+  // Run mode (template RUN): narrow tiles in great number.  A tile of 128 x 16 - 64 outputs with a short K is little work,
   // and the waits and hand-overs of the producer and the issuing warp, about 1180 cycles a tile whatever its width, bound it.
-  // So a tile is RUN x 128 consecutive rows here: one stage, RUN accumulators side by side, one hand-over.  MobileNetV2 at batch
-  // 1024: stem GEMM (K = 48, 32 channels) 418 -> 200 us, 32 -> 16 at 112 x 112 382 -> 131 us (617 MB: 0.72 of HBM), 96 -> 24 at 56 x 56 118 -> 74.
+  // So a tile is RUN x 128 consecutive rows here: one stage, RUN accumulators side by side, one hand-over; four of up to 32 columns,
+  // two of up to 64, which is what TMEM holds for four teams.  MobileNetV2 at batch 1024: stem GEMM (K = 48, 32 channels) 418 -> 200 us,
+  // 32 -> 16 at 112 x 112 382 -> 131 us (617 MB: 0.72 of HBM), 96 -> 24 at 56 x 56 118 -> 74, 144 -> 32 at 28 x 28 42 -> 38.  With two pieces
+  // the epilogue is nearly level with the overhead: ResNet-50's stem GEMM (K = 192, 64 channels) at batch 64 35.9 -> 33.3.
   int run;
   // Columns are dealt to the epilogue warps in blocks of blk_w (64, 32 or 16), blk_per_group consecutive blocks to a
   // warp group (all of them in team mode).  plain_order: the weight rows are not permuted (blk_w is 16 then).
@@ -958,8 +959,10 @@ GemmKernel kernel_of_form(int extra, int blk_w) {
 int extra_of(const GemmParams& p) { return p.dz != 0 || p.ep.border_corr != nullptr ? 2 : p.ep.fix_shl != 0 || p.ep.out.lo < 0 ? 1 : 0; }
 GemmKernel kernel_variant(const GemmParams& p) {
   const int extra = extra_of(p);
-  if (p.run > 1) return extra ? (p.blk_w == 32 ? gemm_i8_tc_kernel<1, false, 2, kRun> : gemm_i8_tc_kernel<1, false, 1, kRun>)
-                              : (p.blk_w == 32 ? gemm_i8_tc_kernel<0, false, 2, kRun> : gemm_i8_tc_kernel<0, false, 1, kRun>);
+  if (p.run == 4) return extra ? (p.blk_w == 32 ? gemm_i8_tc_kernel<1, false, 2, 4> : gemm_i8_tc_kernel<1, false, 1, 4>)
+                               : (p.blk_w == 32 ? gemm_i8_tc_kernel<0, false, 2, 4> : gemm_i8_tc_kernel<0, false, 1, 4>);
+  if (p.run == 2) return extra ? (p.blk_w == 64 ? gemm_i8_tc_kernel<1, false, 4, 2> : gemm_i8_tc_kernel<1, false, 1, 2>)
+                               : (p.blk_w == 64 ? gemm_i8_tc_kernel<0, false, 4, 2> : gemm_i8_tc_kernel<0, false, 1, 2>);
   return p.ep.add_residual != nullptr ? kernel_of_form<true>(extra, p.blk_w) : kernel_of_form<false>(extra, p.blk_w);
 }
 
@@ -972,7 +975,7 @@ bool one_tile_each(long long m_tiles, int n_tiles, int sms) { return m_tiles * n
 // turns out to allow the halo mode of the implicit convolution (0: not asked for).
 bool finish_plan(GemmTcPlan* plan, const int8_t* B, int a_signed, int Np, int Kp, int Kspan, int taps, int ldd,
                  const ContractEpilogue& e, void* D, int* status, const char** why, const GemmTcTiling* tiling, int halo_w = 0,
-                 int halo_h = 0, bool want_pair = false, bool wide_teams = false, bool want_run = false, bool one_each = false) {
+                 int halo_h = 0, bool want_pair = false, bool wide_teams = false, int max_run = 1, bool one_each = false) {
   GemmParams& p = plan->params;
   p.Ocp = ldd;
   p.ldd = ldd;
@@ -1050,10 +1053,12 @@ bool finish_plan(GemmTcPlan* plan, const int8_t* B, int a_signed, int Np, int Kp
   const char* pair_env = std::getenv("B2VX_TC_PAIR");   // read per plan, so that one process can build both forms
   const bool no_pair = pair_env && std::strcmp(pair_env, "0") == 0;
   p.pair = (want_pair && !no_pair && !p.halo && !p.b_resident && !p.teams && e.add_residual == nullptr && p.BN > 128) ? 1 : 0;
-  // Run mode: weights resident, a team per tile, four accumulator buffers of four pieces (up to 32 columns a piece), at least
-  // three stages.
-  p.run = want_run && p.b_resident && p.teams && p.BN <= 32 && p.dz == 0 && e.add_residual == nullptr && !p.plain_order &&
-          3 * static_cast<size_t>(kRun * kBlockM) * p.BK + bres + 8192 + sizeof(SmemHeader) <= static_cast<size_t>(kSmemBudget) ? kRun : 1;
+  // Run mode: weights resident, a team per tile, four accumulator buffers of four pieces of up to 32 columns or two of up to 64, at
+  // least three stages.
+  p.run = p.BN <= 32 ? 4 : p.BN <= 64 && p.blk_w != 32 ? 2 : 1;
+  if (p.run > max_run || !p.b_resident || !p.teams || p.dz != 0 || e.add_residual != nullptr || p.plain_order ||
+      3 * static_cast<size_t>(p.run * kBlockM) * p.BK + bres + 8192 + sizeof(SmemHeader) > static_cast<size_t>(kSmemBudget))
+    p.run = 1;
   const size_t sub_bytes = p.halo ? p.a_stage_bytes : static_cast<size_t>((p.pair ? 2 : p.run) * kBlockM + (p.b_resident ? 0 : p.BN)) * p.BK;
   const size_t ring_budget = kSmemBudget - 2048 - sizeof(SmemHeader) - staging - add_table_bytes - bres;
   int group = static_cast<int>((64 * 1024) / sub_bytes);
@@ -1097,7 +1102,7 @@ bool finish_plan(GemmTcPlan* plan, const int8_t* B, int a_signed, int Np, int Kp
   // the attribute belongs to the function on one device: set it once per device of this process, and only for the functions
   // that are used (asking loads the function)
   static std::atomic<uint32_t> raised[64];
-  const uint32_t bit = 1u << (p.run > 1 ? 18 + (extra_of(p) != 0 ? 2 : 0) + (p.blk_w == 32 ? 1 : 0) : extra_of(p) * 6 + (e.add_residual != nullptr ? 3 : 0) + (p.blk_w == 64 ? 2 : p.blk_w == 32 ? 1 : 0));
+  const uint32_t bit = 1u << (p.run > 1 ? (p.run == 4 ? 18 : 22) + (extra_of(p) != 0 ? 2 : 0) + (p.blk_w != 16 ? 1 : 0) : extra_of(p) * 6 + (e.add_residual != nullptr ? 3 : 0) + (p.blk_w == 64 ? 2 : p.blk_w == 32 ? 1 : 0));
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev < 0 || dev >= 64 || !(raised[dev].load(std::memory_order_relaxed) & bit)) {
@@ -1161,8 +1166,8 @@ GemmTcPlan* gemm_tc_plan_create(const void* A, int a_signed, const int8_t* B, in
   const bool wide_teams = Kp <= 128 && static_cast<long long>((M + kBlockM - 1) / kBlockM) >= 8LL * sms;
   // run mode where every team of a CTA gets two tiles or more
   static const bool no_run = [] { const char* e2 = std::getenv("B2VX_TC_RUN"); return e2 && std::strcmp(e2, "0") == 0; }();
-  const bool want_run = !no_run && Kp <= 128 && M >= kRun * kBlockM * 8LL * sms;
-  if (!finish_plan(plan, B, a_signed, Np, Kp, Kp, 1, ldd, e, D, status, &why, tiling, 0, 0, want_pair, wide_teams, want_run,
+  const int max_run = no_run || Kp > 256 ? 1 : static_cast<int>(std::min<long long>(4, M / (kBlockM * 8LL * sms)));
+  if (!finish_plan(plan, B, a_signed, Np, Kp, Kp, 1, ldd, e, D, status, &why, tiling, 0, 0, want_pair, wide_teams, max_run,
                    one_tile_each((M + kBlockM - 1) / kBlockM, tiling ? tiling->n_tiles : (Np + 255) / 256, sms))) {
     delete plan;
     return fail(why);
@@ -1240,7 +1245,7 @@ GemmTcPlan* gemm_tc_conv_plan_create(const void* X, int x_signed, const int8_t* 
   }
   auto tiles_of = [&](int tw, int th, int tn) { return static_cast<long long>((g.Wo + tw - 1) / tw) * ((g.Ho + th - 1) / th) * ((g.N + tn - 1) / tn); };
   const bool one_each = one_tile_each(std::max(tiles_of(bw, bh, bn), halo_w ? tiles_of(8, 16, 1) : 0), tiling ? tiling->n_tiles : (Np + 255) / 256, sms);
-  if (!finish_plan(plan, B, x_signed, Np, Kp, g.Cp, g.kh * g.kw, g.Ocp, e, D, status, &why, tiling, halo_w, halo_h, false, false, false, one_each)) {
+  if (!finish_plan(plan, B, x_signed, Np, Kp, g.Cp, g.kh * g.kw, g.Ocp, e, D, status, &why, tiling, halo_w, halo_h, false, false, 1, one_each)) {
     delete plan;
     return fail(why);
   }
