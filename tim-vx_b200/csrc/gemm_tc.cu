@@ -66,6 +66,7 @@
 
 #include <algorithm>
 #include <atomic>
+#include <climits>
 #include <cmath>
 #include <cstdio>
 #include <cstdlib>
@@ -1135,6 +1136,13 @@ void set_grid(GemmTcPlan* plan) {
 
 }  // namespace
 
+// Run mode where every team of a CTA gets two tiles or more.  A row index there counts on past M to the end of the last tile and a
+// piece beyond it, less than five pieces in all, and must not wrap: it is only compared with M, so a negative row would be stored.
+int gemm_tc_max_pieces(int M, int Kp, int sms) {
+  if (Kp > 256 || M > INT_MAX - 5 * kBlockM) return 1;
+  return static_cast<int>(std::max<long long>(1, std::min<long long>(4, M / (kBlockM * 8LL * sms))));
+}
+
 GemmTcPlan* gemm_tc_plan_create(const void* A, int a_signed, const int8_t* B, int M, int Np, int Kp, int Oc, void* D,
                                 int ldd, int d_signed, const ContractEpilogue& e, int* status, char* err,
                                 size_t err_len, const GemmTcTiling* tiling) {
@@ -1164,9 +1172,8 @@ GemmTcPlan* gemm_tc_plan_create(const void* A, int a_signed, const int8_t* B, in
   const long long tiles_256 = static_cast<long long>((M + kBlockM - 1) / kBlockM) * ((Np + 255) / 256);
   const bool want_pair = Kp >= 4096 && tiles_256 >= 2LL * sms;
   const bool wide_teams = Kp <= 128 && static_cast<long long>((M + kBlockM - 1) / kBlockM) >= 8LL * sms;
-  // run mode where every team of a CTA gets two tiles or more
   static const bool no_run = [] { const char* e2 = std::getenv("B2VX_TC_RUN"); return e2 && std::strcmp(e2, "0") == 0; }();
-  const int max_run = no_run || Kp > 256 ? 1 : static_cast<int>(std::min<long long>(4, M / (kBlockM * 8LL * sms)));
+  const int max_run = no_run ? 1 : gemm_tc_max_pieces(M, Kp, sms);
   if (!finish_plan(plan, B, a_signed, Np, Kp, Kp, 1, ldd, e, D, status, &why, tiling, 0, 0, want_pair, wide_teams, max_run,
                    one_tile_each((M + kBlockM - 1) / kBlockM, tiling ? tiling->n_tiles : (Np + 255) / 256, sms))) {
     delete plan;

@@ -249,6 +249,8 @@ int gemm_tc_row_of_channel(const GemmTcTiling& t, int c);
 // Picks the tiling for M x Ocp x Kp from a small cost model (waves of tiles over the SMs, operand
 // bytes per tile, epilogue work per tile).  with_s: reserve 16 rows per tile for the ones row.
 GemmTcTiling gemm_tc_choose_tiling(long long M, int Ocp, int Kp, int with_s);
+// The most 128-row pieces a tile of an M x Kp plain GEMM may have on a device of `sms` SMs (1 to 4).
+int gemm_tc_max_pieces(int M, int Kp, int sms);
 // tiling == null: ceil(Np / 256) equal tiles of Np / n_tiles rows in channel order, no ones row.
 GemmTcPlan* gemm_tc_plan_create(const void* A, int a_signed, const int8_t* B, int M, int Np, int Kp, int Oc,
                                 void* D, int ldd, int d_signed, const ContractEpilogue& e, int* status,
