@@ -41,8 +41,9 @@ def test_one_tile_with_fused_add(product_lib, oracle_lib, spec, batch):
 @pytest.mark.parametrize("channels", [32, 48, 64, 96, 150, 288])
 @pytest.mark.parametrize("form", ["1x1", "3x3", "add"])
 def test_one_narrow_tile_for_each_block(product_lib, oracle_lib, channels, form):
-    """Launches of about a wave with tiles of 16 to 64 columns: all epilogue warps share the only tile of a block."""
-    for hw, batch in ((56, 1), (19, 4), (65, 2)):
+    """Launches of about a wave with tiles of 16 to 64 columns: all epilogue warps share the only tile of a block, or, on 19 x 19 at batch
+    47 and 75 x 75 at batch 3, where a convolution's spatial tiles are more than a wave and its pixels / 128 are not, teams take them."""
+    for hw, batch in ((56, 1), (19, 4), (65, 2), (19, 47), (75, 3)):
         if form == "add":
             outs = []
             for lib in (oracle_lib, product_lib):

@@ -39,3 +39,20 @@ def test_pieces_by_rows(ask):
     rows = {1: 1, one: 1, two - 1: 1, two: 2, four - 1: 3, four: 4, 2 * four: 4}
     assert ask([("pieces", m, 256, 148) for m in rows]) == [(p,) for p in rows.values()]
     assert ask([("pieces", four, 272, 148), ("pieces", four // 2, 16, 74)]) == [(1,), (4,)]
+
+
+def test_column_blocks_follow_the_tiles_of_a_convolution(ask):
+    """Tiles of 32 to 64 columns: blocks of 16 where all warps share a CTA's only tile, the widest where a team takes it.  Sizes around
+    a wave of 148 tiles, where ceil(M / 128) and the spatial tiles differ."""
+    sizes = [(n, hw, k, stride, oc) for hw, k, stride, images in ((56, 3, 1, (4, 5, 6, 7)), (19, 3, 1, (44, 45, 46, 52, 53)), (33, 3, 1, (16, 17, 18)),
+                                                                  (7, 3, 1, (384, 385, 386, 387)), (75, 3, 1, (2, 3, 4)), (38, 3, 2, (46, 50)), (112, 1, 2, (5, 6)))
+             for n in images for oc in (32, 64)]
+    one = {}
+    for (n, hw, k, stride, oc), (m_tiles, n_tiles, data, blk_w, one_each) in zip(sizes, ask([("conv", n, hw, hw, k, stride, 64, oc) for n, hw, k, stride, oc in sizes])):
+        out = (hw + stride - 1) // stride
+        assert m_tiles >= -(-n * out * out // 128)
+        assert one_each == (m_tiles * n_tiles <= 148 // n_tiles * n_tiles)
+        assert blk_w == (16 if one_each and data >= 32 else data), (n, hw, oc)
+        one[n, hw, oc] = one_each
+    # 147 tiles by pixels, but 168 and more by 8 x 16 pieces of the images
+    assert [one[n, 56, 64] for n in (4, 5, 6, 7)] == [1, 1, 0, 0] and not one[47 - 1, 19, 64] and not one[17, 33, 64] and not one[385, 7, 64] and not one[3, 75, 64]

@@ -970,7 +970,7 @@ b2vx_status plan_contraction(b2vx_graph* g, uint32_t node_index, const char* lab
     // Measured at N = K = 4096: faster than the 128-row tile up to 8 rows (1.8x at one row); at 16 rows the
     // dp4a rate bounds it and the tensor-core kernel is level or better.
     if (g->fc_small_m && mode == IDENTITY && M <= 16 && (!any_dz || x.C == x.Cp)) {
-      pack_contraction(x, w, bias, kw, kh, x.C, Cs, Kp, y.C, y.Cp, GemmTcTiling{1, y.Cp, y.Cp, 0}, 0, centred, &pk);
+      pack_contraction(x, w, bias, kw, kh, x.C, Cs, Kp, y.C, y.Cp, GemmTcTiling{1, y.Cp, y.Cp, 0, 0}, 0, centred, &pk);
       int8_t* dw8s = nullptr; int32_t* dbias_s = nullptr; float* dscale_s = nullptr;
       b2vx_status sts = upload(g, pk.w8, &dw8s);
       if (sts == B2VX_OK) sts = upload(g, pk.bias_full, &dbias_s);
@@ -990,7 +990,7 @@ b2vx_status plan_contraction(b2vx_graph* g, uint32_t node_index, const char* lab
       g->steps.push_back(std::move(s_fc));
       return B2VX_OK;
     }
-    const GemmTcTiling tiling = gemm_tc_choose_tiling(M, y.Cp, Kp, any_dz ? 1 : 0);
+    const GemmTcTiling tiling = gemm_tc_choose_tiling(M, y.Cp, Kp, any_dz ? 1 : 0, mode == IMPLICIT ? gemm_tc_conv_m_tiles(geo) : 0);
     const int Np = tiling.n_tiles * tiling.rows;
     pack_contraction(x, w, bias, kw, kh, x.C, Cs, Kp, y.C, y.Cp, tiling, mode == WHCN ? 1 : (mode == WHCN8 ? (padk == 8 ? 2 : 3) : 0), centred, &pk);
     ep.dz_uniform = any_dz ? dz_value : 0;
@@ -1153,7 +1153,7 @@ b2vx_status plan_contraction(b2vx_graph* g, uint32_t node_index, const char* lab
 
   // CUDA-core path: K = tap*Cp + c, out-of-bounds taps are skipped and corrected per tap.
   const int Kp = taps * x.Cp;
-  pack_contraction(x, w, bias, kw, kh, x.C, x.Cp, Kp, y.C, y.Cp, GemmTcTiling{1, y.Cp, y.Cp + 1, 0}, 0, centred, &pk);
+  pack_contraction(x, w, bias, kw, kh, x.C, x.Cp, Kp, y.C, y.Cp, GemmTcTiling{1, y.Cp, y.Cp + 1, 0, 0}, 0, centred, &pk);
   int8_t* dw8 = nullptr; int32_t *dbias = nullptr, *ddz = nullptr, *dtapc = nullptr; float* dscale = nullptr;
   b2vx_status st = upload(g, pk.w8, &dw8);
   if (st == B2VX_OK) st = upload(g, pk.bias_full, &dbias);

@@ -976,7 +976,7 @@ bool one_tile_each(long long m_tiles, int n_tiles, int sms) { return m_tiles * n
 // turns out to allow the halo mode of the implicit convolution (0: not asked for).
 bool finish_plan(GemmTcPlan* plan, const int8_t* B, int a_signed, int Np, int Kp, int Kspan, int taps, int ldd,
                  const ContractEpilogue& e, void* D, int* status, const char** why, const GemmTcTiling* tiling, int halo_w = 0,
-                 int halo_h = 0, bool want_pair = false, bool wide_teams = false, int max_run = 1, bool one_each = false) {
+                 int halo_h = 0, bool want_pair = false, bool wide_teams = false, int max_run = 1) {
   GemmParams& p = plan->params;
   p.Ocp = ldd;
   p.ldd = ldd;
@@ -1013,7 +1013,7 @@ bool finish_plan(GemmTcPlan* plan, const int8_t* B, int a_signed, int Np, int Kp
   // columns also go one per warp group: four tiles in flight instead of four passes over every tile)
   // (one_each: no CTA gets a second tile, so three teams would have nothing to do; all sixteen warps share the one, in column
   // blocks of 16.  Host to host: ResNet-50 batch 1 / 4 314.6 -> 308.2 / 387 -> 375 us, MobileNetV2 batch 1 / 8 234.3 -> 227.5 / 301 -> 294.)
-  p.teams = ((p.BNd <= 64 || (wide_teams && p.BN <= 128)) && !no_teams && !(one_each && p.BNd >= 32)) ? kGroups : 0;
+  p.teams = ((p.BNd <= 64 || (wide_teams && p.BN <= 128)) && !no_teams && !(tiling && tiling->one_each && p.BNd >= 32)) ? kGroups : 0;
   p.blk_per_group = (p.BNd / p.blk_w + kGroups - 1) / kGroups;
   p.res_tma = e.add_residual != nullptr && !p.plain_order ? 1 : 0;
   p.res_shift = p.teams ? 2 : 1;
@@ -1174,8 +1174,7 @@ GemmTcPlan* gemm_tc_plan_create(const void* A, int a_signed, const int8_t* B, in
   const bool wide_teams = Kp <= 128 && static_cast<long long>((M + kBlockM - 1) / kBlockM) >= 8LL * sms;
   static const bool no_run = [] { const char* e2 = std::getenv("B2VX_TC_RUN"); return e2 && std::strcmp(e2, "0") == 0; }();
   const int max_run = no_run ? 1 : gemm_tc_max_pieces(M, Kp, sms);
-  if (!finish_plan(plan, B, a_signed, Np, Kp, Kp, 1, ldd, e, D, status, &why, tiling, 0, 0, want_pair, wide_teams, max_run,
-                   one_tile_each((M + kBlockM - 1) / kBlockM, tiling ? tiling->n_tiles : (Np + 255) / 256, sms))) {
+  if (!finish_plan(plan, B, a_signed, Np, Kp, Kp, 1, ldd, e, D, status, &why, tiling, 0, 0, want_pair, wide_teams, max_run)) {
     delete plan;
     return fail(why);
   }
@@ -1203,6 +1202,49 @@ GemmTcPlan* gemm_tc_plan_create(const void* A, int a_signed, const int8_t* B, in
   return plan;
 }
 
+namespace {
+
+// M tile of an implicit convolution: w x h x n output pixels, at most 128; halo_w x halo_h is the input patch of the tile in halo
+// mode (see GemmParams; kHaloTileW x kHaloTileH output pixels of one image), 0 where that is not asked for.
+struct ConvTile {
+  int w, h, n, halo_w, halo_h;
+};
+constexpr int kHaloTileW = 8, kHaloTileH = 16;
+
+ConvTile conv_tile(const ConvGeom& g) {
+  ConvTile t = {1, 1, 1, 0, 0};
+  // Halo mode is asked for when the convolution has more than one tap, stride and dilation 1, and tiles of that shape waste at
+  // most 15 % of their rows on this output size.
+  if (g.kh * g.kw > 1 && g.sx == 1 && g.sy == 1 && g.dx == 1 && g.dy == 1 && g.kw <= 16 && g.kh <= 16) {
+    const double covered = static_cast<double>((g.Wo + kHaloTileW - 1) / kHaloTileW * kHaloTileW) * ((g.Ho + kHaloTileH - 1) / kHaloTileH * kHaloTileH);
+    if (static_cast<double>(g.Wo) * g.Ho >= 0.85 * covered) { t.halo_w = kHaloTileW + g.kw - 1; t.halo_h = kHaloTileH + g.kh - 1; }
+  }
+  // The shape that leaves the fewest tile rows unused.
+  double best = -1.0;
+  for (int tw = 1; tw <= g.Wo && tw <= kBlockM; ++tw) {
+    for (int th = 1; th <= g.Ho && tw * th <= kBlockM; ++th) {
+      int tn = kBlockM / (tw * th);
+      if (tn > g.N) tn = g.N;
+      if (tn < 1) continue;
+      // the box extent along a strided axis is (T-1)*stride+1 elements and may not exceed 256
+      if ((tw - 1) * g.sx + 1 > 256 || (th - 1) * g.sy + 1 > 256) continue;
+      const long long tiles = static_cast<long long>((g.Wo + tw - 1) / tw) * ((g.Ho + th - 1) / th) * ((g.N + tn - 1) / tn);
+      const double eff = static_cast<double>(g.Wo) * g.Ho * g.N / (static_cast<double>(tiles) * kBlockM);
+      // prefer wider rows at equal efficiency: longer contiguous runs per TMA box
+      if (eff > best + 1e-9 || (eff > best - 1e-9 && tw > t.w)) { best = eff; t.w = tw; t.h = th; t.n = tn; }
+    }
+  }
+  return t;
+}
+
+}  // namespace
+
+long long gemm_tc_conv_m_tiles(const ConvGeom& g) {
+  auto tiles_of = [&](int tw, int th, int tn) { return static_cast<long long>((g.Wo + tw - 1) / tw) * ((g.Ho + th - 1) / th) * ((g.N + tn - 1) / tn); };
+  const ConvTile t = conv_tile(g);
+  return std::max(tiles_of(t.w, t.h, t.n), t.halo_w ? tiles_of(kHaloTileW, kHaloTileH, 1) : 0);
+}
+
 GemmTcPlan* gemm_tc_conv_plan_create(const void* X, int x_signed, const int8_t* B, const ConvGeom& g, int Np, void* D,
                                      const ContractEpilogue& e, int* status, char* err, size_t err_len,
                                      const GemmTcTiling* tiling) {
@@ -1221,42 +1263,13 @@ GemmTcPlan* gemm_tc_conv_plan_create(const void* X, int x_signed, const int8_t* 
   std::memset(&plan->map_r, 0, sizeof(plan->map_r));
   const char* why = "";
   const int Kp = g.kh * g.kw * g.Cp;
-  // Halo mode (see GemmParams): a tile is 8 x 16 output pixels of one image.  Asked for when the convolution has more
-  // than one tap, stride and dilation 1, and tiles of that shape waste at most 15 % of their rows on this output size.
-  int halo_w = 0, halo_h = 0;
-  if (g.kh * g.kw > 1 && g.sx == 1 && g.sy == 1 && g.dx == 1 && g.dy == 1 && g.kw <= 16 && g.kh <= 16) {
-    const double covered = static_cast<double>((g.Wo + 7) / 8 * 8) * ((g.Ho + 15) / 16 * 16);
-    if (static_cast<double>(g.Wo) * g.Ho >= 0.85 * covered) { halo_w = 8 + g.kw - 1; halo_h = 16 + g.kh - 1; }
-  }
-  // M tile = TW x TH x TN output pixels, at most 128: the shape that leaves the fewest tile rows unused.
-  int bw = 1, bh = 1, bn = 1;
-  double best = -1.0;
-  for (int tw = 1; tw <= g.Wo && tw <= kBlockM; ++tw) {
-    for (int th = 1; th <= g.Ho && tw * th <= kBlockM; ++th) {
-      int tn = kBlockM / (tw * th);
-      if (tn > g.N) tn = g.N;
-      if (tn < 1) continue;
-      // the box extent along a strided axis is (T-1)*stride+1 elements and may not exceed 256
-      if ((tw - 1) * g.sx + 1 > 256 || (th - 1) * g.sy + 1 > 256) continue;
-      const long long tiles = static_cast<long long>((g.Wo + tw - 1) / tw) * ((g.Ho + th - 1) / th) * ((g.N + tn - 1) / tn);
-      const double eff = static_cast<double>(g.Wo) * g.Ho * g.N / (static_cast<double>(tiles) * kBlockM);
-      // prefer wider rows at equal efficiency: longer contiguous runs per TMA box
-      if (eff > best + 1e-9 || (eff > best - 1e-9 && tw > bw)) { best = eff; bw = tw; bh = th; bn = tn; }
-    }
-  }
-  int sms = 148;
-  {
-    int dev = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  }
-  auto tiles_of = [&](int tw, int th, int tn) { return static_cast<long long>((g.Wo + tw - 1) / tw) * ((g.Ho + th - 1) / th) * ((g.N + tn - 1) / tn); };
-  const bool one_each = one_tile_each(std::max(tiles_of(bw, bh, bn), halo_w ? tiles_of(8, 16, 1) : 0), tiling ? tiling->n_tiles : (Np + 255) / 256, sms);
-  if (!finish_plan(plan, B, x_signed, Np, Kp, g.Cp, g.kh * g.kw, g.Ocp, e, D, status, &why, tiling, halo_w, halo_h, false, false, 1, one_each)) {
+  const ConvTile t = conv_tile(g);
+  if (!finish_plan(plan, B, x_signed, Np, Kp, g.Cp, g.kh * g.kw, g.Ocp, e, D, status, &why, tiling, t.halo_w, t.halo_h)) {
     delete plan;
     return fail(why);
   }
-  if (p.halo) { bw = 8; bh = 16; bn = 1; }
+  const int halo_w = t.halo_w, halo_h = t.halo_h;
+  const int bw = p.halo ? kHaloTileW : t.w, bh = p.halo ? kHaloTileH : t.h, bn = p.halo ? 1 : t.n;
   p.conv = 1;
   p.TW = bw; p.TH = bh; p.TN = bn;
   p.tiles_w = (g.Wo + bw - 1) / bw;
@@ -1309,7 +1322,7 @@ int column_block(int data, bool teams) {
 
 }  // namespace
 
-GemmTcTiling gemm_tc_choose_tiling(long long M, int Ocp, int Kp, int with_s) {
+GemmTcTiling gemm_tc_choose_tiling(long long M, int Ocp, int Kp, int with_s, long long plan_m_tiles) {
   int dev = 0, sms = 148;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
@@ -1317,7 +1330,17 @@ GemmTcTiling gemm_tc_choose_tiling(long long M, int Ocp, int Kp, int with_s) {
   const int max_data = 256 - extra;
   const long long m_tiles = (M + kBlockM - 1) / kBlockM;
   const double rows = static_cast<double>(M < kBlockM ? M : kBlockM);
-  GemmTcTiling best = {0, 0, 0, 0};
+  GemmTcTiling best = {0, 0, 0, 0, 0};
+  // How the plan deals a tile out, and the column blocks for that: with the count of tiles that the plan has, which for an implicit
+  // convolution is more than M / 128 where its tiles do not cover the output evenly.  (Decided from M / 128 as one tile a CTA, such layers
+  // ran in teams with blocks of 16 columns: 3x3 64 -> 64 on 19 x 19 at batch 47 13.9 us for 12.3 with the blocks of 64 that teams take, with
+  // a fused Add 16.4 for 14.4, and a graph of 64 -> 32 on 75 x 75 at batch 3 14.6 for 13.3.)
+  auto with_blocks = [&](GemmTcTiling t) {
+    t.one_each = one_tile_each(plan_m_tiles > 0 ? plan_m_tiles : m_tiles, t.n_tiles, sms) ? 1 : 0;
+    // (the same tests as for teams in finish_plan and wide_teams in gemm_tc_plan_create; block widths are free to choose, a mismatch costs only time)
+    t.blk_w = column_block(t.data, (t.data <= 64 && !(t.data >= 32 && t.one_each)) || (t.rows <= 128 && Kp <= 128 && m_tiles >= 8LL * sms));
+    return t;
+  };
   double best_time = 0.0;
   const bool l2_resident = (static_cast<double>(M) + Ocp) * Kp < 48.0e6;
   // B2VX_TC_BN=<width>: force the tile width (a tuning aid; ignored when it does not fit)
@@ -1329,8 +1352,7 @@ GemmTcTiling gemm_tc_choose_tiling(long long M, int Ocp, int Kp, int with_s) {
       best.n_tiles = nt;
       best.data = data;
       best.rows = data + extra;
-      best.blk_w = column_block(data, data <= 64);
-      return best;
+      return with_blocks(best);
     }
   }
   int last_data = 0;
@@ -1376,10 +1398,7 @@ GemmTcTiling gemm_tc_choose_tiling(long long M, int Ocp, int Kp, int with_s) {
     best.data = (((Ocp + best.n_tiles - 1) / best.n_tiles) + 15) & ~15;
     best.rows = best.data + extra;
   }
-  // (the same test as wide_teams in gemm_tc_plan_create; block widths are free to choose, a mismatch costs only time)
-  best.blk_w = column_block(best.data, (best.data <= 64 && !(best.data >= 32 && one_tile_each(m_tiles, best.n_tiles, sms))) ||
-                                          (best.rows <= 128 && Kp <= 128 && m_tiles >= 8LL * sms));
-  return best;
+  return with_blocks(best);
 }
 
 int gemm_tc_row_of_channel(const GemmTcTiling& t, int c) {

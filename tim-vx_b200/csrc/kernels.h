@@ -241,14 +241,18 @@ struct GemmTcPlan;   // opaque: tensor maps + launch geometry, built once at com
 // `data` is the all-ones row (S column) and the rest is zero.
 // A tile's channels lie in its data rows in the order gemm_tc_row_of_channel gives: column blocks of blk_w (64, 32 or 16)
 // channels, within a block permuted so that an epilogue thread's accumulator columns are neighbouring channels.
+// one_each: no CTA of the launch gets a second tile, so all epilogue warps of a CTA share its only one.
 struct GemmTcTiling {
-  int n_tiles, data, rows, blk_w;
+  int n_tiles, data, rows, blk_w, one_each;
 };
 // Packed row, within its tile, of the tile's channel c.
 int gemm_tc_row_of_channel(const GemmTcTiling& t, int c);
 // Picks the tiling for M x Ocp x Kp from a small cost model (waves of tiles over the SMs, operand
 // bytes per tile, epilogue work per tile).  with_s: reserve 16 rows per tile for the ones row.
-GemmTcTiling gemm_tc_choose_tiling(long long M, int Ocp, int Kp, int with_s);
+// m_tiles: M tiles that the plan will have, gemm_tc_conv_m_tiles for an implicit convolution, 0 for a plain GEMM.
+GemmTcTiling gemm_tc_choose_tiling(long long M, int Ocp, int Kp, int with_s, long long m_tiles = 0);
+// M tiles of gemm_tc_conv_plan_create's plan (the larger count where it may still choose between two tile shapes).
+long long gemm_tc_conv_m_tiles(const ConvGeom& g);
 // The most 128-row pieces a tile of an M x Kp plain GEMM may have on a device of `sms` SMs (1 to 4).
 int gemm_tc_max_pieces(int M, int Kp, int sms);
 // tiling == null: ceil(Np / 256) equal tiles of Np / n_tiles rows in channel order, no ones row.
