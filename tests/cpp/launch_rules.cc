@@ -2,6 +2,7 @@
 //   pieces,M,Kp,sms             128-row pieces that a tile of a plain GEMM may have
 //   conv,N,W,H,k,stride,C,Oc    an implicit convolution with SAME padding, on 148 SMs: M tiles, N tiles, columns of a tile, of a
 //                               column block, whether no CTA gets a second tile
+//   im2col,N,W,H,C,kw,kh,stride,sms   output rows that a block of the first layer's im2col takes (no padding), and how many blocks there are
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
@@ -24,6 +25,15 @@ int main(int argc, char** argv) {
       const long long tiles = b2vx::gemm_tc_conv_m_tiles(g);
       const b2vx::GemmTcTiling t = b2vx::gemm_tc_choose_tiling(static_cast<long long>(g.N) * g.Wo * g.Ho, g.Ocp, g.kw * g.kh * g.Cp, 0, tiles);
       std::printf("%lld %d %d %d %d\n", tiles, t.n_tiles, t.data, t.blk_w, t.one_each);
+    } else if (what == "im2col" && v.size() == 8) {
+      b2vx::ConvGeom g = {};
+      g.N = v[0]; g.W = v[1]; g.H = v[2]; g.C = v[3]; g.kw = v[4]; g.kh = v[5]; g.sx = g.sy = v[6]; g.dx = g.dy = 1;
+      g.Wo = (g.W - g.kw) / g.sx + 1; g.Ho = (g.H - g.kh) / g.sy + 1;
+      const int padk = g.kw <= 4 ? 4 : 8;
+      int Kp = (g.kh * g.C * padk + 15) / 16 * 16;
+      if (Kp > 64) Kp = (Kp + 63) / 64 * 64;
+      const int rows = b2vx::im2col_whcn8_rows(g, Kp, padk, v[7]);
+      std::printf("%d %d\n", rows, g.N * ((g.Ho + rows - 1) / rows));
     } else return 2;
   }
   return 0;

@@ -56,3 +56,15 @@ def test_column_blocks_follow_the_tiles_of_a_convolution(ask):
         one[n, hw, oc] = one_each
     # 147 tiles by pixels, but 168 and more by 8 x 16 pieces of the images
     assert [one[n, 56, 64] for n in (4, 5, 6, 7)] == [1, 1, 0, 0] and not one[47 - 1, 19, 64] and not one[17, 33, 64] and not one[385, 7, 64] and not one[3, 75, 64]
+
+
+def test_output_rows_of_an_im2col_block_follow_the_device(ask):
+    """Several rows only where six blocks are left for every SM of the device there is."""
+    lenet, stem = (28, 28, 1, 5, 5, 1), (230, 230, 3, 7, 7, 2)
+    sizes = [(n, layer, sms) for layer in (lenet, stem) for n in (1, 13, 64, 1000) for sms in (74, 148, 296)]
+    rows = {}
+    for (n, layer, sms), (out_rows, blocks) in zip(sizes, ask([("im2col", n) + layer + (sms,) for n, layer, sms in sizes])):
+        assert out_rows >= 1 and (out_rows == 1 or blocks >= 6 * sms), (n, layer, sms)
+        rows[n, layer, sms] = out_rows
+    assert [rows[64, lenet, sms] for sms in (74, 148, 296)] == [3, 1, 1]
+    assert rows[1000, lenet, 148] > 8 and rows[1, lenet, 74] == 1 and rows[64, stem, 148] == 2

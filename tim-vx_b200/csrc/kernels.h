@@ -226,9 +226,12 @@ void launch_im2col(const void* x, int Cs, int Kp, int zx, const ConvGeom& g, voi
 void launch_im2col_whcn(const void* x, int Kp, int zx, const ConvGeom& g, void* col, cudaStream_t s);
 // The same for filters up to padk = 8 or 4 wide (dilation 1) with K index = (ky*C + c)*padk + kx: every (pixel, ky, c)
 // contributes padk consecutive input bytes, slot kx >= kw carrying a don't-care byte (zero weight).
-// Shared memory needed per block: C * kh * im2col_whcn8_pitch(g, padk) + 16 bytes.
+// Shared memory of a block of one output row: C * kh * im2col_whcn8_pitch(g, padk) + 16 bytes, and what it takes more for
+// im2col_whcn8_rows of them stays within 40 KB.
 void launch_im2col_whcn8(const void* x, int Kp, int zx, const ConvGeom& g, int padk, void* col, cudaStream_t s);
 int im2col_whcn8_pitch(const ConvGeom& g, int padk);
+// Output rows of a block on a device of `sms` SMs.
+int im2col_whcn8_rows(const ConvGeom& g, int Kp, int padk, int sms);
 
 // ---- int8 GEMM on tcgen05 tensor cores --------------------------------------
 // D[M][ldd] (u8/s8) = requant(A[M][Kp] (u8 or s8) * B[Np][Kp]^T (s8)), K-major

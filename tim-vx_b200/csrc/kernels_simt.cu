@@ -2495,24 +2495,31 @@ void launch_fc_small_m(const void* A, int a_signed, const int8_t* B, int M, int 
   else launch_fc_small_m_t<4, 16>(A, a_signed, B, M, Kp, Oc, Ocp, e, D, ldd, s);
 }
 
-void launch_im2col_whcn8(const void* x, int Kp, int zx, const ConvGeom& g, int padk, void* col, cudaStream_t s) {
-  if (g.N == 0 || g.Ho == 0 || g.Wo == 0) return;
-  const int pitch = im2col_whcn8_pitch(g, padk);
-  // Output rows of a block: eight pieces of 16 bytes for each thread where that leaves six blocks or more for every SM and the
-  // staged rows fit.  With one row a block, two barriers and the loads' latency came for as little as a third of a piece a
-  // thread: LeNet at batch 256 / 1000 host to host 88.8 -> 82.2 / 158 -> 127 us, MobileNetV2 at 64 / 1024 749 -> 743 / 8173 -> 8018,
-  // ResNet-50 at 64 1140 -> 1133.  Fewer blocks than six an SM are left alone: batch 1 keeps one row each.
+static size_t im2col_whcn8_bytes(const ConvGeom& g, int padk, int out_rows) {
+  return static_cast<size_t>(g.C) * (g.kh + (out_rows - 1) * g.sy) * im2col_whcn8_pitch(g, padk) + 16;
+}
+// Eight pieces of 16 bytes for each thread where that leaves six blocks or more for every SM and the staged rows fit.  With one
+// row a block, two barriers and the loads' latency came for as little as a third of a piece a thread: LeNet at batch 256 / 1000
+// host to host 88.8 -> 82.2 / 158 -> 127 us, MobileNetV2 at 64 / 1024 749 -> 743 / 8173 -> 8018, ResNet-50 at 64 1140 -> 1133.
+// Fewer blocks than six an SM are left alone: batch 1 keeps one row each.
+int im2col_whcn8_rows(const ConvGeom& g, int Kp, int padk, int sms) {
   const int per_row = g.Wo * (Kp / 16);
   int out_rows = (2048 + per_row - 1) / per_row;
-  const long long room = static_cast<long long>(g.N) * g.Ho / (148 * 6);
+  const long long room = static_cast<long long>(g.N) * g.Ho / (6LL * sms);
   if (out_rows > room) out_rows = static_cast<int>(room);
   if (out_rows > g.Ho) out_rows = g.Ho;
-  auto bytes = [&](int r) { return static_cast<size_t>(g.C) * (g.kh + (r - 1) * g.sy) * pitch + 16; };
-  while (out_rows > 1 && bytes(out_rows) > 40u * 1024u) --out_rows;
-  if (out_rows < 1) out_rows = 1;
+  while (out_rows > 1 && im2col_whcn8_bytes(g, padk, out_rows) > 40u * 1024u) --out_rows;
+  return out_rows < 1 ? 1 : out_rows;
+}
+void launch_im2col_whcn8(const void* x, int Kp, int zx, const ConvGeom& g, int padk, void* col, cudaStream_t s) {
+  if (g.N == 0 || g.Ho == 0 || g.Wo == 0) return;
+  int dev = 0, sms = 148;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  const int out_rows = im2col_whcn8_rows(g, Kp, padk, sms);
   const dim3 grid((g.Ho + out_rows - 1) / out_rows, g.N);
-  launch_pdl(padk == 8 ? im2col_whcn8_kernel<8> : im2col_whcn8_kernel<4>, grid, dim3(256), bytes(out_rows), s, static_cast<const uint8_t*>(x), Kp, zx, g, pitch,
-             out_rows, static_cast<uint8_t*>(col));
+  launch_pdl(padk == 8 ? im2col_whcn8_kernel<8> : im2col_whcn8_kernel<4>, grid, dim3(256), im2col_whcn8_bytes(g, padk, out_rows), s, static_cast<const uint8_t*>(x),
+             Kp, zx, g, im2col_whcn8_pitch(g, padk), out_rows, static_cast<uint8_t*>(col));
 }
 int im2col_whcn8_pitch(const ConvGeom& g, int padk) {
   // up to 3 bytes of alignment lead, the padk-byte read of the last pixel, the last word of the funnel
