@@ -41,3 +41,20 @@ def product_lib():
 def reference_cases():
     with open(os.path.join(ROOT, "tests", "golden", "reference_cases.json")) as f:
         return json.load(f)["cases"]
+
+
+@pytest.fixture(scope="session")
+def launch_rules(tmp_path_factory):
+    """Asks the CUDA library's host-side launch rules through tests/cpp/launch_rules.cc (no GPU needed): questions as tuples of a name
+    and whole numbers, answers as tuples."""
+    import pyb2vx
+    exe = str(tmp_path_factory.mktemp("rules") / "launch_rules")
+    csrc = os.path.dirname(pyb2vx.PRODUCT_LIB)
+    subprocess.check_call(["/usr/bin/g++", "-std=c++17", "-O1", "-Wall", "-Wextra", "-I" + csrc, "-I/usr/local/cuda/include",
+                           os.path.join(ROOT, "tests", "cpp", "launch_rules.cc"), pyb2vx.PRODUCT_LIB, "-Wl,-rpath," + csrc, "-o", exe])
+
+    def ask(questions):
+        out = subprocess.run([exe] + [",".join(str(f) for f in q) for q in questions], capture_output=True, text=True, timeout=60)
+        assert out.returncode == 0, out.stderr
+        return [tuple(int(f) for f in line.split()) for line in out.stdout.splitlines()]
+    return ask

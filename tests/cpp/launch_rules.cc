@@ -2,7 +2,8 @@
 //   pieces,M,Kp,sms             128-row pieces that a tile of a plain GEMM may have
 //   conv,N,W,H,k,stride,C,Oc    an implicit convolution with SAME padding, on 148 SMs: M tiles, N tiles, columns of a tile, of a
 //                               column block, whether no CTA gets a second tile
-//   im2col,N,W,H,C,kw,kh,stride,sms   output rows that a block of the first layer's im2col takes (no padding), and how many blocks there are
+//   gemm,M,K,Oc                 a plain GEMM, the same answers
+//   im2col,N,W,H,C,kw,kh,sx,sy,same,sms   output rows that a block of the first layer's im2col takes, how many blocks there are, output rows
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
@@ -25,15 +26,18 @@ int main(int argc, char** argv) {
       const long long tiles = b2vx::gemm_tc_conv_m_tiles(g);
       const b2vx::GemmTcTiling t = b2vx::gemm_tc_choose_tiling(static_cast<long long>(g.N) * g.Wo * g.Ho, g.Ocp, g.kw * g.kh * g.Cp, 0, tiles);
       std::printf("%lld %d %d %d %d\n", tiles, t.n_tiles, t.data, t.blk_w, t.one_each);
-    } else if (what == "im2col" && v.size() == 8) {
+    } else if (what == "gemm" && v.size() == 3) {
+      const b2vx::GemmTcTiling t = b2vx::gemm_tc_choose_tiling(v[0], (v[2] + 15) / 16 * 16, (v[1] + 15) / 16 * 16, 0);
+      std::printf("%d %d %d %d %d\n", (v[0] + 127) / 128, t.n_tiles, t.data, t.blk_w, t.one_each);
+    } else if (what == "im2col" && v.size() == 10) {
       b2vx::ConvGeom g = {};
-      g.N = v[0]; g.W = v[1]; g.H = v[2]; g.C = v[3]; g.kw = v[4]; g.kh = v[5]; g.sx = g.sy = v[6]; g.dx = g.dy = 1;
-      g.Wo = (g.W - g.kw) / g.sx + 1; g.Ho = (g.H - g.kh) / g.sy + 1;
+      g.N = v[0]; g.W = v[1]; g.H = v[2]; g.C = v[3]; g.kw = v[4]; g.kh = v[5]; g.sx = v[6]; g.sy = v[7]; g.dx = g.dy = 1;
+      g.Wo = (g.W - (v[8] ? 1 : g.kw)) / g.sx + 1; g.Ho = (g.H - (v[8] ? 1 : g.kh)) / g.sy + 1;
       const int padk = g.kw <= 4 ? 4 : 8;
       int Kp = (g.kh * g.C * padk + 15) / 16 * 16;
       if (Kp > 64) Kp = (Kp + 63) / 64 * 64;
-      const int rows = b2vx::im2col_whcn8_rows(g, Kp, padk, v[7]);
-      std::printf("%d %d\n", rows, g.N * ((g.Ho + rows - 1) / rows));
+      const int rows = b2vx::im2col_whcn8_rows(g, Kp, padk, v[9]);
+      std::printf("%d %d %d\n", rows, g.N * ((g.Ho + rows - 1) / rows), g.Ho);
     } else return 2;
   }
   return 0;

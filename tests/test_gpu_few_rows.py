@@ -40,10 +40,15 @@ def test_one_tile_with_fused_add(product_lib, oracle_lib, spec, batch):
 
 @pytest.mark.parametrize("channels", [32, 48, 64, 96, 150, 288])
 @pytest.mark.parametrize("form", ["1x1", "3x3", "add"])
-def test_one_narrow_tile_for_each_block(product_lib, oracle_lib, channels, form):
+def test_one_narrow_tile_for_each_block(product_lib, oracle_lib, launch_rules, channels, form):
     """Launches of about a wave with tiles of 16 to 64 columns: all epilogue warps share the only tile of a block, or, on 19 x 19 at batch
     47 and 75 x 75 at batch 3, where a convolution's spatial tiles are more than a wave and its pixels / 128 are not, teams take them."""
-    for hw, batch in ((56, 1), (19, 4), (65, 2), (19, 47), (75, 3)):
+    sizes = ((56, 1), (19, 4), (65, 2), (19, 47), (75, 3), (56, 4))
+    ks = [32, 64][form == "add"]
+    rules = launch_rules([("conv", b, hw, hw, 3, 1, ks, channels) if form == "3x3" else ("gemm", b * hw * hw, ks, channels) for hw, b in sizes])
+    narrow = [one_each for _, _, columns, _, one_each in rules if 32 <= columns <= 64]
+    assert 1 in narrow and (form != "3x3" or 0 in narrow), rules
+    for hw, batch in sizes:
         if form == "add":
             outs = []
             for lib in (oracle_lib, product_lib):
