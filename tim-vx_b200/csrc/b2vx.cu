@@ -1123,16 +1123,17 @@ b2vx_status plan_contraction(b2vx_graph* g, uint32_t node_index, const char* lab
       if (!pl) return fail(g, B2VX_UNSUPPORTED, lbl + ": " + err);
       g->gemm_plans.push_back(pl);
       *plan_holder = pl;
-      if (implicit && gemm_tc_plan_is_halo(pl)) {
-        // "gemm_i8_tc(implicit...)" -> "gemm_i8_tc(halo...)": one input patch per tile instead of one box per tap
+      // "gemm_i8_tc(implicit...)" -> "gemm_i8_tc(halo...)": one input patch per tile instead of one box per tap;
+      // "gemm_i8_tc" -> "gemm_i8_tc(x4)": tiles of four 128-row pieces
+      const int pieces = gemm_tc_plan_pieces(pl);
+      if ((implicit && gemm_tc_plan_is_halo(pl)) || pieces > 1) {
         for (Step& st : g->steps) {
           if (st.tag != plan_holder.get()) continue;
           std::string name = st.info.name;
           const size_t at = name.find("implicit");
-          if (at != std::string::npos) {
-            name.replace(at, 8, "halo");
-            std::snprintf(st.info.name, sizeof(st.info.name), "%s", name.c_str());
-          }
+          if (pieces > 1) name = (name.back() == ')' ? name.substr(0, name.size() - 1) + "," : name + "(") + "x" + std::to_string(pieces) + ")";
+          else if (at != std::string::npos) name.replace(at, 8, "halo");
+          std::snprintf(st.info.name, sizeof(st.info.name), "%s", name.c_str());
         }
       }
       return B2VX_OK;

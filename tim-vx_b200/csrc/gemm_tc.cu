@@ -1172,8 +1172,8 @@ GemmTcPlan* gemm_tc_plan_create(const void* A, int a_signed, const int8_t* B, in
   const long long tiles_256 = static_cast<long long>((M + kBlockM - 1) / kBlockM) * ((Np + 255) / 256);
   const bool want_pair = Kp >= 4096 && tiles_256 >= 2LL * sms;
   const bool wide_teams = Kp <= 128 && static_cast<long long>((M + kBlockM - 1) / kBlockM) >= 8LL * sms;
-  static const bool no_run = [] { const char* e2 = std::getenv("B2VX_TC_RUN"); return e2 && std::strcmp(e2, "0") == 0; }();
-  const int max_run = no_run ? 1 : gemm_tc_max_pieces(M, Kp, sms);
+  const char* run_env = std::getenv("B2VX_TC_RUN");   // read per plan, so that one process can build both forms
+  const int max_run = run_env && std::strcmp(run_env, "0") == 0 ? 1 : gemm_tc_max_pieces(M, Kp, sms);
   if (!finish_plan(plan, B, a_signed, Np, Kp, Kp, 1, ldd, e, D, status, &why, tiling, 0, 0, want_pair, wide_teams, max_run)) {
     delete plan;
     return fail(why);
@@ -1481,6 +1481,7 @@ GemmTcPlan* gemm_tc_plan_build_in(void* storage, size_t storage_bytes, const voi
 void gemm_tc_plan_destroy(GemmTcPlan* p) { delete p; }
 
 int gemm_tc_plan_is_halo(const GemmTcPlan* p) { return p && p->params.halo ? 1 : 0; }
+int gemm_tc_plan_pieces(const GemmTcPlan* p) { return p && p->params.run > 1 ? p->params.run : 1; }
 
 cudaError_t gemm_tc_launch(const GemmTcPlan* plan, cudaStream_t s) {
 #ifdef B2VX_TC_TRACE

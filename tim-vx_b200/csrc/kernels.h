@@ -278,6 +278,8 @@ GemmTcPlan* gemm_tc_plan_build_in(void* storage, size_t storage_bytes, const voi
 void gemm_tc_plan_destroy(GemmTcPlan* p);
 // 1 when an implicit-convolution plan loads one input patch per tile and runs the taps on shifted views of it.
 int gemm_tc_plan_is_halo(const GemmTcPlan* p);
+// 128-row pieces of a tile: 1, or 2 or 4 in run mode.
+int gemm_tc_plan_pieces(const GemmTcPlan* p);
 cudaError_t gemm_tc_launch(const GemmTcPlan* p, cudaStream_t s);
 // 1 when this build and device can run the tensor-core path.
 int gemm_tc_available(void);
