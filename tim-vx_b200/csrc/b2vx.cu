@@ -2271,8 +2271,8 @@ b2vx_status b2vx_graph_compile(b2vx_graph* g) {
     s.fn = [=](cudaStream_t st2) { launch_cl_to_whcn(src, g->tensors[i].d_io, N, C, H, W, Cp, el, st2); return cudaGetLastError(); };
     g->steps.push_back(std::move(s));
   }
-  // up to four of them in one launch: a launch costs more than the rows (LeNet, whose two outputs took one each: batch 1 40.0 -> 38.6 us
-  // host to host, 256 81.2 -> 78.2, with the softmax's programmatic dependent launch)
+  // up to four of them in one launch: a launch costs more than the rows (LeNet, whose two outputs took one each: batch 1 38.7 -> 38.0 us
+  // host to host, 256 79.3 -> 78.6, 1000 125.7 -> 124.6)
   for (size_t first = 0; first < row_outputs.size(); first += 4) {
     const std::vector<size_t> ids(row_outputs.begin() + first, row_outputs.begin() + std::min(first + 4, row_outputs.size()));
     PackRows pack;

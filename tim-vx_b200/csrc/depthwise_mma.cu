@@ -327,7 +327,9 @@ DwMmaPlan* dw_mma_plan_create(const void* x, int x_signed, const int8_t* w, cons
   // Channel groups of a slab: all of them up to nine, else whole sectors (an even number), the split that leaves the
   // fewest groups idle; among equals the one that fills a block with eight warps (8 groups, or 4 of two strips) before the one
   // that makes six: two blocks of either share an SM.  Batch 256: 28 x 28 x 192 57.1 us with 6 groups, 43.0 with 4; 14 x 14 x 576
-  // 46.1 and 34.5; 7 x 7 x 960 25.1 and 22.5.
+  // 46.1 and 34.5; 7 x 7 x 960 25.1 and 22.5.  (Fewest idle groups first is not always fastest: at 288, 480 and 672 channels 6
+  // groups leave none idle, and eight warps with some idle take less: 28 x 28 x 288 at batch 256 65.8 us with 6 groups and 58.3 with 4,
+  // 14 x 14 x 480 34.5 and 29.1 with 8, 14 x 14 x 672 41.4 and 34.6 with 4.  Below one wave of tiles the widths are within 0.5 us.)
   p.groups = all;
   if (all > kMaxWarps) {
     int best_idle = 1 << 30;

@@ -169,6 +169,8 @@ struct GemmParams {
   // two of up to 64, which is what TMEM holds for four teams.  MobileNetV2 at batch 1024: stem GEMM (K = 48, 32 channels) 418 -> 200 us,
   // 32 -> 16 at 112 x 112 382 -> 131 us (617 MB: 0.72 of HBM), 96 -> 24 at 56 x 56 118 -> 74, 144 -> 32 at 28 x 28 42 -> 38.  With two pieces
   // the epilogue is nearly level with the overhead: ResNet-50's stem GEMM (K = 192, 64 channels) at batch 64 35.9 -> 33.3.
+  // Only where every team of a CTA gets two tiles or more, a margin that was chosen, not measured; and tiles of up to 32 columns with
+  // rows for two or three pieces a tile by that rule, but not for four, stay at one piece (two were not measured there).
   int run;
   // Columns are dealt to the epilogue warps in blocks of blk_w (64, 32 or 16), blk_per_group consecutive blocks to a
   // warp group (all of them in team mode).  plain_order: the weight rows are not permuted (blk_w is 16 then).
@@ -1182,8 +1184,9 @@ GemmTcPlan* gemm_tc_plan_create(const void* A, int a_signed, const int8_t* B, in
   p.num_kb = (Kp + p.BK - 1) / p.BK;
   p.m_tiles = (M + p.run * kBlockM - 1) / (p.run * kBlockM);
   // Rows past the end are left out of the box: filled with zeros they cost the TMA unit time (host to host, eight layers of
-  // 4096 x 4096: 17 rows 150 -> 101 us, 24 rows 149 -> 105; twelve of 2048 x 2048, 49 rows: 120 -> 104; from 64 rows on level).
-  // What lies in the tile's other rows is multiplied into accumulators that nobody reads.
+  // 4096 x 4096: 17 rows 150 -> 101 us, 24 rows 149 -> 105, 32 and 50 rows level; twelve of 2048 x 2048, 49 rows: 120 -> 104; from 64
+  // rows on level).  The accumulators of the tile's other rows hold products of what lay in shared memory: the epilogue requantizes them
+  // (and looks the fused Add up with leftovers of the residual buffer), but stores only rows below M.
   p.box_rows = M < kBlockM ? M : p.run > 1 ? 2 * kBlockM : kBlockM;   // run mode: two pieces a box
   p.a_tx_bytes = static_cast<uint32_t>(p.run > 1 ? p.run * kBlockM : p.box_rows) * p.BK;
   const uint64_t adims[2] = {static_cast<uint64_t>(Kp), static_cast<uint64_t>(M)};
@@ -1440,8 +1443,9 @@ double gemm_tc_measure_int8_peak(int reps, int* sm_count, int* status) {
 
 size_t gemm_tc_plan_bytes(void) { return sizeof(GemmTcPlan); }
 
-// Same plan as gemm_tc_plan_create, but built inside caller-provided storage (no heap allocation);
-// the caller must not pass it to gemm_tc_plan_destroy.
+// A plain-GEMM plan built inside caller-provided storage (no heap allocation); the caller must not pass it to
+// gemm_tc_plan_destroy.  Simpler than gemm_tc_plan_create's: channels in order, full 128-row boxes, one 128-row tile at a time in
+// teams or by column blocks of 16, no pair or run mode.
 GemmTcPlan* gemm_tc_plan_build_in(void* storage, size_t storage_bytes, const void* A, int a_signed, const int8_t* B, int M,
                                   int Np, int Kp, void* D, int ldd, const ContractEpilogue& e, int* status, char* err,
                                   size_t err_len) {

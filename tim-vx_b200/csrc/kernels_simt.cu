@@ -1548,7 +1548,8 @@ __device__ __forceinline__ float load_real(const void* x, int kind, long long i,
   return __fmul_rn(__fsub_rn(__int2float_rn(v), __int2float_rn(z)), s);
 }
 
-// One thread per slice; slices are short (class scores).
+// One thread per slice; slices are short (class scores).  Programmatic dependent launch: LeNet at batch 1 / 256 / 1000 host to host
+// 38.3 -> 38.0 / 79.0 -> 78.6 / 125.3 -> 124.6 us.
 __global__ void softmax_kernel(const void* __restrict__ x, int x_kind, float sx, int zx, void* __restrict__ y, int y_kind,
                                OutQuant out, float beta, SoftmaxGeom g) {
   pdl_trigger();
